@@ -1146,6 +1146,13 @@ cudaError_t lu_eliminate(const PanelConfig& pc, const BatchLayout& lay, int batc
         if (err != cudaSuccess) return err;
         continue;
       }
+    } else if (w.tc_images && kb <= kTc64Depth) {
+      // at every size: one 64 x 64 x 32 tile takes 130 us on the FP64 pipe of its SM, more than the whole launch here
+      tc64_update(lay, batch, k + kb, n, k + kb, col_end, k, kb, M, w.tc_images, w.tc_alpha,
+                  w.tc_image_batch, w.tc_wait_polls, s);
+      err = cudaGetLastError();
+      if (err != cudaSuccess) return err;
+      continue;
     }
     gemm_any<T>(pc.nb, lay, batch, k + kb, n, k + kb, col_end, k, kb, M, nullptr, s);
     err = cudaGetLastError();
@@ -1167,7 +1174,7 @@ void lu_forward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cp
 
 template <typename T>
 void lu_backward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cplx<T>* M, const int* skip,
-                     cudaStream_t s) {
+                     cudaStream_t s, const LuWork* w) {
   const int n = lay.n, col_end = lay.n + lay.m;
   const int last = ((n - 1) / pc.nb) * pc.nb;
   dim3 grid(unsigned((lay.m + 7) / 8), unsigned(batch));
@@ -1181,6 +1188,13 @@ void lu_backward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, c
       default:
         if constexpr (sizeof(T) == 8) rhs_upper_kernel<T, 8><<<grid, 256, 0, s>>>(lay, k, M, skip);
         break;
+    }
+    if constexpr (sizeof(T) == 8) {
+      if (w && w->tc_images && kb <= kTc64Depth && !skip) {
+        tc64_update(lay, batch, 0, k, n, col_end, k, kb, M, w->tc_images, w->tc_alpha, w->tc_image_batch,
+                    w->tc_wait_polls, s);
+        continue;
+      }
     }
     gemm_any<T>(pc.nb, lay, batch, 0, k, n, col_end, k, kb, M, skip, s);
   }
@@ -1291,9 +1305,10 @@ template void lu_forward_rhs<double>(const PanelConfig&, const BatchLayout&, int
                                      cudaStream_t);
 template void lu_forward_rhs<float>(const PanelConfig&, const BatchLayout&, int, float2*, const LuWork&, const int*,
                                     cudaStream_t);
-template void lu_backward_rhs<double>(const PanelConfig&, const BatchLayout&, int, double2*, const int*,
-                                      cudaStream_t);
-template void lu_backward_rhs<float>(const PanelConfig&, const BatchLayout&, int, float2*, const int*, cudaStream_t);
+template void lu_backward_rhs<double>(const PanelConfig&, const BatchLayout&, int, double2*, const int*, cudaStream_t,
+                                      const LuWork*);
+template void lu_backward_rhs<float>(const PanelConfig&, const BatchLayout&, int, float2*, const int*, cudaStream_t,
+                                     const LuWork*);
 template void launch_absorber_solve<double>(const BatchLayout&, int, const double2*, double2*, const int*,
                                             cudaStream_t);
 template void launch_absorber_solve<float>(const BatchLayout&, int, const float2*, double2*, const int*,

@@ -55,8 +55,21 @@ constexpr long long kTcWaitPolls = 1LL << 26;
 void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int col_end, float2* M, uint8_t* images,
                         int* err_flag, const int* skip, long long wait_polls, KernelSpans* spans, cudaStream_t s);
 
+// C[r_begin:r_end, c_begin:c_end] -= M[rows, ka:ka+kb] M[ka:ka+kb, cols] in FP64 accuracy, kb <= 32, on the tensor
+// cores from exact 8-bit digit products (tc_update64.cu).  images: tc64_image_bytes of image_batch systems; a larger
+// batch runs as several launches over them.  alpha: 32 ints per imaged system, zero before the first call and left zero
+// by each.  wait_polls bounds the waits of
+// the kernel's roles on each other; a CTA whose waits run out finishes its tiles in FP64 multiply-adds, so the update
+// is complete whatever the budget.
+constexpr int kTc64Depth = 32;
+size_t tc64_image_bytes(int n, int m, int batch);
+void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int c_begin, int c_end, int ka, int kb,
+                 double2* M, uint8_t* images, int* alpha, int image_batch, long long wait_polls, cudaStream_t s);
+
 struct LuWork {
-  uint8_t* tc_images = nullptr;  // operand images for the tensor-core update (FP32 only); null = CUDA cores
+  uint8_t* tc_images = nullptr;  // operand images for the tensor-core updates (FP32 or FP64); null = CUDA cores
+  int tc_image_batch = 0;        // systems the FP64 update's images hold
+  int* tc_alpha = nullptr;       // the FP64 update's column scales (tc64_update)
   int* tc_err = nullptr;         // set when a tensor-core wait timed out
   long long tc_wait_polls = kTcWaitPolls;  // poll budget of the role waits in the tensor-core update
   KernelSpans* tc_spans = nullptr;         // events around the tensor-core update launches (profiling)
@@ -97,10 +110,11 @@ template <typename T>
 void lu_forward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cplx<T>* M, const LuWork& w,
                     const int* skip, cudaStream_t s);
 
-// Backward sweep on the RHS columns: X = U^-1 Y (in place).
+// Backward sweep on the RHS columns: X = U^-1 Y (in place).  w (FP64, nullable): block updates on the tensor cores
+// where it holds operand images.
 template <typename T>
 void lu_backward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cplx<T>* M, const int* skip,
-                     cudaStream_t s);
+                     cudaStream_t s, const LuWork* w = nullptr);
 
 // gg from the eliminated [U | Y]: solve U[n-m:, n-m:] X = Y[n-m:, :] (m x m,
 // upper triangular) and write X (FP64, column-major m x m) per matrix.

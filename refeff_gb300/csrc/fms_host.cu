@@ -433,6 +433,10 @@ struct Workspace {
   bool use_tc = false;               // FP32 trailing update on the tensor cores
   DevBuf<uint8_t> tc_images;         // operand images of the tensor-core update (and the residual's X digits)
   size_t tc_image_size = 0;
+  bool use_tc64 = false;             // FP64 block updates on the tensor cores
+  int tc64_batch = 0;                // systems their operand images hold
+  DevBuf<int> tc64_alpha;            // their column scales, zero between updates
+  DevBuf<uint8_t> tc64_images;       // their operand images; a refined workspace lends its tc_images instead
   int residual_pref = 1;             // refinement residual on the tensor cores (baked into graphs)
   DevBuf<int> tc_err;                // set by a tensor-core wait that timed out
   long long tc_wait_polls = kTcWaitPolls;  // poll budget of the tensor-core update's role waits (baked into graphs)
@@ -919,6 +923,7 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
   RF_CUDA(ctx, ws.status.alloc(size_t(B)));
   RF_CUDA(ctx, ws.info.alloc(size_t(B)));
   ws.use_tc = ws.fp32 && ctx->use_tensor_cores != 0;
+  ws.use_tc64 = ctx->use_tensor_cores != 0;
   if (ws.use_tc) {
     ws.tc_image_size = tc_image_bytes(n, m, B);
     RF_CUDA(ctx, ws.tc_images.alloc(ws.tc_image_size));
@@ -932,9 +937,27 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
 // A workspace whose (re)configuration failed part-way (an allocation) is left
 // unconfigured, so that the next call configures it again instead of running
 // on buffers sized for another shape.
+// `lu64`: the FP64 elimination runs in it (not only the refined form or the iterative ones), so it needs operand
+// images for the FP64 tensor-core updates where the refined form's do not serve.
 int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int batch, bool fp32,
-                     const TunePrefs* tune = nullptr) {
-  const int rc = ensure_workspace_impl(ctx, ws, n, m, batch, fp32, tune);
+                     const TunePrefs* tune = nullptr, bool lu64 = true) {
+  int rc = ensure_workspace_impl(ctx, ws, n, m, batch, fp32, tune);
+  if (!rc && lu64 && ws.use_tc64) {
+    // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); without room
+    // for them the updates stay on the CUDA cores
+    const size_t one = tc64_image_bytes(n, m, 1);
+    ws.tc64_batch = ws.use_tc ? ws.batch
+                              : int(std::min<size_t>(size_t(ws.batch), std::max<size_t>(1, (size_t(1) << 30) / one)));
+    const size_t bytes = ws.use_tc ? 0 : tc64_image_bytes(n, m, ws.tc64_batch), na = size_t(ws.tc64_batch) * 32;
+    if (ws.tc64_images.n < bytes || ws.tc64_alpha.n < na) {
+      ws.drop_graphs();
+      if ((bytes && ws.tc64_images.alloc(bytes) != cudaSuccess) || ws.tc64_alpha.alloc(na) != cudaSuccess ||
+          cudaMemset(ws.tc64_alpha.p, 0, na * sizeof(int)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+        cudaGetLastError();
+        ws.use_tc64 = false;
+      }
+    }
+  }
   if (rc) {
     ws.drop_graphs();
     ws.batch = 0;
@@ -943,7 +966,9 @@ int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int b
   return rc;
 }
 
-LuWork lu_work(Workspace& ws, const PanelConfig& pc) {
+// `polls`: the FP64 updates take the caller's poll budget too (dense solves; elsewhere the FP64 LU is itself what a
+// timed-out call falls back on).
+LuWork lu_work(Workspace& ws, const PanelConfig& pc, bool polls = false) {
   LuWork w;
   w.ipiv = ws.ipiv.p;
   w.perm = ws.perm.p;
@@ -958,6 +983,12 @@ LuWork lu_work(Workspace& ws, const PanelConfig& pc) {
     w.nperm_in = ws.nperm_in.p;
     w.linv = ws.linv.p;
     w.pair128 = pc.pair128;
+  }
+  if (&pc == &ws.pc64 && ws.use_tc64 && ws.tc64_alpha.p) {
+    w.tc_images = ws.use_tc ? ws.tc_images.p : ws.tc64_images.p;
+    w.tc_image_batch = ws.tc64_batch;
+    w.tc_alpha = ws.tc64_alpha.p;
+    if (polls) w.tc_wait_polls = ws.tc_wait_polls;
   }
   if (&pc == &ws.pc32 && ws.use_tc) {
     w.tc_images = ws.tc_images.p;
@@ -1218,7 +1249,8 @@ cudaError_t run_fms_batch(refeff_fms_plan& p, Workspace& ws, int batch, refeff_f
         // the absorber alone: its block is the trailing m x m triangle solve
         launch_absorber_solve<double>(lay, batch, ws.M64.p, ws.gg_stage.p, ws.status.p, s);
       } else {
-        lu_backward_rhs<double>(ws.pc64, lay, batch, ws.M64.p, nullptr, s);
+        const LuWork w64 = lu_work(ws, ws.pc64);
+        lu_backward_rhs<double>(ws.pc64, lay, batch, ws.M64.p, nullptr, s, &w64);
         launch_copy_rhs64(lay, batch, ws.M64.p, ws.X64.p, s);
         launch_extract_blocks(lay, batch, ws.X64.p, p.d_blocks.p, int(p.blocks.size()), p.gg_per, ws.gg_stage.p,
                               ws.status.p, s);
@@ -1385,7 +1417,7 @@ int solve_device_energies_enqueue(refeff_fms_plan& p, int E, const double2* d_k,
   }
   if (bicg) RF_CUDA(ctx, p.d_bicg_iters_all.alloc(size_t(E)));
   auto prepare = [&](Workspace& ws) -> int {
-  int rc = ensure_workspace(ctx, ws, p.n, p.m, B, fp32, &p.tune);
+  int rc = ensure_workspace(ctx, ws, p.n, p.m, B, fp32, &p.tune, p.minv == 0);
   if (rc) return rc;
   RF_CUDA(ctx, ws.k_stage.alloc(size_t(ws.batch) * p.nsp));
   RF_CUDA(ctx, ws.x_stage.alloc(size_t(ws.batch) * xph));
@@ -2165,8 +2197,9 @@ int inverse_columns(refeff_fms_plan* plan, const refeff_fms_energy_points* point
     launch_build_system(p.P, nb, ws.k_stage.p, ws.x_stage.p, lay, ws.M64.p, nullptr, ws.status.p, s);
     count_launch();
     unit_rhs_kernel<<<dim3(64, unsigned(nb)), 256, 0, s>>>(lay, ws.M64.p, s0, cnt);
-    RF_CUDA(ctx, lu_eliminate<double>(ws.pc64, lay, nb, ws.M64.p, lu_work(ws, ws.pc64), s));
-    lu_backward_rhs<double>(ws.pc64, lay, nb, ws.M64.p, nullptr, s);
+    const LuWork w64 = lu_work(ws, ws.pc64);
+    RF_CUDA(ctx, lu_eliminate<double>(ws.pc64, lay, nb, ws.M64.p, w64, s));
+    lu_backward_rhs<double>(ws.pc64, lay, nb, ws.M64.p, nullptr, s, &w64);
     count_launch();
     if (whole_block)
       inverse_block_kernel<<<unsigned(nb), 256, 0, s>>>(lay, ws.M64.p, s0, cnt, dout.p);
@@ -2221,9 +2254,10 @@ int dense_solve_device(refeff_fms_context* ctx, Workspace& ws, int batch, bool f
   RF_CUDA(ctx, cudaMemsetAsync(ws.status.p, 0, size_t(batch) * sizeof(int), s));
   RF_CUDA(ctx, cudaMemsetAsync(ws.info.p, 0, size_t(batch) * sizeof(int), s));
   if (!fp32) {
-    cudaError_t e = lu_eliminate<double>(ws.pc64, lay, batch, ws.M64.p, lu_work(ws, ws.pc64), s);
+    const LuWork w64 = lu_work(ws, ws.pc64, true);
+    cudaError_t e = lu_eliminate<double>(ws.pc64, lay, batch, ws.M64.p, w64, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "lu_eliminate<double>");
-    lu_backward_rhs<double>(ws.pc64, lay, batch, ws.M64.p, nullptr, s);
+    lu_backward_rhs<double>(ws.pc64, lay, batch, ws.M64.p, nullptr, s, &w64);
     RF_CUDA(ctx, ws.X64.alloc(size_t(ws.batch) * lay.lda * lay.m));
     launch_copy_rhs64(lay, batch, ws.M64.p, ws.X64.p, s);
   } else {

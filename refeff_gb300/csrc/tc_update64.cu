@@ -1,0 +1,629 @@
+// Tensor-core (tcgen05, sm_103a) block update of the FP64 elimination and of
+// the FP64 triangular sweeps over many right-hand sides:
+//     C[r, c] -= sum_k A[r, k] B[k, c]      (complex FP64, K <= 32)
+// with C, A and B blocks of one matrix.
+//
+// The FP64 pipe of GB300 runs 2 multiply-adds per SM and cycle (1.15 TFLOP/s
+// measured in this update); the bf16 tensor path runs about 1600 times that.
+// The products are therefore formed exactly on the tensor path from signed
+// 8-bit digits, an error-free splitting after Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication by using fast routines
+// of matrix multiplication and its applications", Numer. Algorithms 59 (2012):
+//
+//   * column k of A is multiplied by 2^g_k and row k of B by 2^-g_k so that no
+//     column of A is small in every row (graded systems: without it a system
+//     whose columns span 24 orders of magnitude loses every digit in the back
+//     substitution); row r of A is then scaled by a power of two 2^-e_r so that
+//     its real and imaginary parts lie in (-1, 1), column c of B by 2^-f_c;
+//   * each scaled value is rounded to a 62-bit fixed-point number and cut into
+//     eight signed digits of weights 2^-6, 2^-14, ..., 2^-62 (|t| <= 128, exact
+//     in bf16);
+//   * tcgen05.mma kind::f16 with FP32 accumulation sums the digit products of
+//     one level s = i + j (2 .. 9, 36 pairs) without rounding: at most 8 pairs
+//     x 2 real products x 32 columns x 2^14 = 2^23 < 2^24;
+//   * the epilogue adds the eight exact level sums in 64-bit integers, converts
+//     the total to FP64 (one rounding) and subtracts it from C (one rounding).
+//
+// Dropped and cut parts weigh about 2^-62 of 2^(e_r + f_c) per product, less
+// than what the FMA chain it replaces rounds away in its 32 steps: on FMS
+// systems of n = 117 .. 304 the error of the solution is 0.3 .. 1.0 of the
+// chain's (seven digits, 28 pairs, measured up to twice the chain's error), and
+// on random systems with rows, columns or both graded over 24 orders the
+// componentwise backward error stays below the chain's.
+//
+// Layout of the work: a CTA owns a 128-row tile of A, whose digits for all 32
+// columns (128 KB) stay in shared memory while it walks 16-column tiles of B
+// and C.  One MMA multiplies one digit plane of A by the adjacent digit slots
+// of B (N = 32 (9 - i)) into the adjacent level accumulators, so the 36 x 4
+// real products of a K step take 16 instructions.  Two sets of 256 TMEM columns
+// alternate, and sixteen epilogue warps finish one tile while the next is
+// multiplied.  The tensor work per tile (2304 cycles), its C traffic (64 KB)
+// and its 4096 FP64 subtractions (2048 cycles) are of the same size, so neither
+// a deeper K nor a wider tile would win much.
+//
+// Every wait on an mbarrier is bounded.  A CTA whose waits ran out drains its
+// copies and MMAs, and its epilogue warps finish their remaining tiles with
+// FP64 multiply-adds from the matrix, so the update is complete in any case;
+// rows and columns that hold an infinity or NaN take the same path.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include "cplx.cuh"
+#include "batched_lu.cuh"
+
+namespace rfx {
+
+namespace {
+
+constexpr int kRows = 128;                       // rows per tile (MMA M)
+constexpr int kCols = 16;                        // columns per tile
+constexpr int kDig = 8;                          // digits per value
+constexpr int kPlane = kRows * 32;               // one digit plane of A, one K step (16 columns): 4 KB
+constexpr int kAHalf = 2 * kDig * kPlane;        // re and im digits of one K step: 64 KB
+constexpr int kATile = 2 * kAHalf;               // 128 KB
+constexpr int kBSide = kDig * 2 * kCols * 32;    // eight slots of 32 rows of 16 bf16: 8 KB
+constexpr int kBHalf = 2 * kBSide;               // P = [Br | Bi] and Q = [-Bi | Br], one K step: 16 KB
+constexpr int kBTile = 2 * kBHalf;               // 32 KB
+constexpr int kBStages = 3;
+constexpr int kEpiWarps = 16;
+constexpr int kThreads = 32 * (2 + kEpiWarps);
+constexpr uint32_t kTmemCols = 512;              // two accumulator sets of 8 levels x [re | im] x 16 columns
+constexpr int kBarOff = kATile + kBStages * kBTile;
+constexpr int kSmem = kBarOff + 256 + 1024;      // + alignment of the base to 1 KB
+static_assert(kSmem <= 227 * 1024, "dynamic shared memory per CTA");
+constexpr int kNonfinite = 1 << 28;              // exponent of a row or column with an infinity or NaN
+
+// barriers: A halves full / empty, B stages full / empty, accumulators full / empty, drain
+enum : int { kAFull = 0, kAEmpty = 2, kBFull = 4, kBEmpty = 4 + kBStages, kAccFull = 4 + 2 * kBStages,
+             kAccEmpty = 6 + 2 * kBStages, kDrain = 8 + 2 * kBStages, kBars = 9 + 2 * kBStages };
+static_assert(kBars * 8 <= 128, "barrier area");
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// Byte offset of 16-byte chunk `chunk` of row `row` in a K-major tile of 32-byte rows with the 32-byte swizzle.
+__device__ __forceinline__ int sw32(int row, int chunk) { return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4); }
+// start >> 4, LBO 1 (unused when swizzled), SBO = 8 rows x 32 B, version 1, 32-byte swizzle (layout 6)
+__device__ __forceinline__ uint64_t desc_sw32(uint32_t saddr) {
+  return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(1) << 16) | (uint64_t(256 >> 4) << 32) | (uint64_t(1) << 46) |
+         (uint64_t(6) << 61);
+}
+// kind::f16, D = F32, A = B = BF16, both K-major, M = 128, N columns
+__device__ __forceinline__ uint32_t idesc_bf16(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(kRows >> 4) << 24);
+}
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Bounded wait of one role on another (poll budget, or 1 s); gives up early once the CTA's abort flag is up,
+// and raises that flag when it runs out.
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long polls) {
+  const uint64_t t0 = global_ns();
+  for (long long it = 0; it < polls; ++it) {
+    if (mbar_try(bar, parity)) return true;
+    if ((it & 255) == 255) {
+      if (*abort_flag) return false;
+      if (global_ns() - t0 > 1000000000ull) break;
+    }
+  }
+  *abort_flag = 1;
+  return false;
+}
+// Drain wait for work this thread issued itself (the full default budget, no abort exit).
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {
+  const uint64_t t0 = global_ns();
+  for (long long it = 0; it < kTcWaitPolls; ++it)
+    if (mbar_try(bar, parity) || ((it & 1023) == 1023 && global_ns() - t0 > 1000000000ull)) return;
+}
+
+__device__ __forceinline__ int field_of(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+// larger exponent field of the two parts; -1 for zero
+__device__ __forceinline__ int field_of(double2 v) {
+  return v.x == 0.0 && v.y == 0.0 ? -1 : max(field_of(v.x), field_of(v.y));
+}
+constexpr int kNoEntry = -(1 << 20);  // exponent of a row or column of zeros
+// v 2^(62 - e) rounded to an integer (|v| < 2^e), biased by 128 in every byte: byte j holds digit 8 - j plus 128.
+__device__ __forceinline__ uint2 biased_digits(double v, int e) {
+  const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
+  const int field = int(bits >> 52) & 0x7ff;
+  unsigned long long x = bits & 0xfffffffffffffull;
+  if (field) x |= 1ull << 52;
+  const int sh = max(field, 1) - 1075 + 62 - e;  // <= 9
+  if (sh >= 0) x <<= sh;
+  else x = sh < -54 ? 0ull : (x + (1ull << (-sh - 1))) >> -sh;
+  if (bits >> 63) x = 0ull - x;
+  x += 0x8080808080808080ull;
+  return make_uint2(uint32_t(x), uint32_t(x >> 32));
+}
+// digit d (0 .. 7, most significant first) as a float
+__device__ __forceinline__ float digit_of(uint2 y, int d) {
+  const int j = 7 - d;
+  const uint32_t w = j >= 4 ? y.y : y.x;
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | (j & 3))) - 8388736.0f;  // 2^23 + 128
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+
+// sum_k A[row, k] B[k, col] in FP64 multiply-adds: the path of rows and columns that the digits cannot hold, and
+// of tiles whose waits ran out.
+__device__ __noinline__ double2 direct_sum(const double2* __restrict__ arow, const double2* __restrict__ bcol, int lda,
+                                           int kb) {
+  double2 acc = make_double2(0.0, 0.0);
+  for (int k = 0; k < kb; ++k) cfma(acc, arow[size_t(lda) * k], bcol[k]);
+  return acc;
+}
+
+// The eight exact level sums of one real output (levels 2 .. 9, weights 2^-12 .. 2^-68 of 2^e) as an FP64 number.
+__device__ __forceinline__ double join_levels(const float (&s)[kDig], int e) {
+  const int p = __float2int_rn(s[0]) * 256 + __float2int_rn(s[1]);
+  const int q = __float2int_rn(s[2]) * 256 + __float2int_rn(s[3]);
+  const int r = __float2int_rn(s[4]) * 256 + __float2int_rn(s[5]);
+  const int l = __float2int_rn(s[6]) * 256 + __float2int_rn(s[7]);
+  // h = the levels 2 .. 7 in units of 2^-52: |h| < 2^59; l holds levels 8 and 9, 16 bits further down
+  const long long h = (static_cast<long long>(p) * 4294967296LL) + static_cast<long long>(q) * 65536 + r;
+  const bool small = ((h + (1ll << 45)) >> 46) == 0;
+  const long long v = small ? h * 65536 + l : h + ((l + 32768) >> 16);
+  const int ex = e - (small ? 68 : 52);
+  double d = __ll2double_rn(v);
+  if (ex > -900 && ex < 900) {  // 1 <= |d| < 2^63 when it is not zero: its exponent takes ex without leaving the range
+    int hi = __double2hiint(d);
+    if (v != 0) hi += ex * (1 << 20);
+    return __hiloint2double(hi, __double2loint(d));
+  }
+  return scalbn(d, ex);
+}
+
+}  // namespace
+
+// alpha[b][k] = 2048 + max over the rows of (exponent of A[row, k] - exponent of the row's largest entry), 0 where column k
+// is zero: g_k = 2048 - alpha.  The table is zero before and is cleared again by the update kernel.
+__global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int r_begin, int r_end, int ka, int kb,
+                                                           const double2* __restrict__ M, int* __restrict__ alpha) {
+  __shared__ int cmax[32];
+  const int b = blockIdx.y, lane = threadIdx.x & 31, row = r_begin + blockIdx.x * kRows + int(threadIdx.x);
+  if (threadIdx.x < 32) cmax[threadIdx.x] = 0;
+  const double2* A = M + size_t(b) * lay.stride + size_t(row) + size_t(lay.lda) * ka;
+  int f[32], top = 0;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) f[k] = row < r_end && k < kb ? field_of(A[size_t(lay.lda) * k]) : -1;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) top = max(top, f[k]);
+  int mine = 0;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    const int v = __reduce_max_sync(0xffffffffu, f[k] > 0 && top < 0x7ff ? f[k] - top + 2048 : 0);
+    if (lane == k) mine = v;
+  }
+  __syncthreads();
+  atomicMax(&cmax[lane], mine);
+  __syncthreads();
+  if (threadIdx.x < 32 && cmax[lane] > 0) atomicMax(alpha + b * 32 + lane, cmax[lane]);
+}
+
+// Digits of both operands.  Blocks x < nbm: a row tile of A, image[b][bm][K step][re 1..8, im 1..8][128 rows of 16 bf16]
+// and the row exponents, two threads per row, 16 columns each.  The others: a column tile of B,
+// image[b][bn][K step][P, Q][digit 1..8][32 rows of 16 bf16] with P = [Br | Bi], Q = [-Bi | Br] (16 columns each) and the
+// column exponents, one warp per column, one lane per row.
+__global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end,
+                                                         int ka, int kb, const double2* __restrict__ M,
+                                                         const int* __restrict__ alpha, uint8_t* __restrict__ aimg,
+                                                         uint8_t* __restrict__ bimg, int* __restrict__ rexp,
+                                                         int* __restrict__ cexp, int nbm, int nbm_all, int nbn_all) {
+  __shared__ __align__(16) uint8_t sm[kBTile];
+  __shared__ int gk[32];
+  const int b = blockIdx.y;
+  if (threadIdx.x < 32) {
+    const int a = alpha[b * 32 + int(threadIdx.x)];
+    gk[threadIdx.x] = a > 0 ? 2048 - a : 0;
+  }
+  __syncthreads();
+  const double2* Mb = M + size_t(b) * lay.stride;
+  if (int(blockIdx.x) < nbm) {
+    int* rowmax = reinterpret_cast<int*>(sm);
+    const int bm = blockIdx.x, r = threadIdx.x & (kRows - 1), h = threadIdx.x >> 7;
+    const int row = r_begin + bm * kRows + r;
+    const double2* A = Mb + size_t(row) + size_t(lay.lda) * (ka + 16 * h);
+    double2 v[16];
+    int e = kNoEntry;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = row < r_end && 16 * h + i < kb ? A[size_t(lay.lda) * i] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int f = field_of(v[i]);
+      if (f >= 0) e = max(e, f == 0x7ff ? kNonfinite : f - 1022 + gk[16 * h + i]);
+    }
+    if (h == 0) rowmax[r] = e;
+    __syncthreads();
+    if (h == 1) rowmax[r] = max(rowmax[r], e);
+    __syncthreads();
+    e = rowmax[r];
+    if (e == kNoEntry) e = 0;
+    if (h == 0) rexp[(size_t(b) * nbm_all + bm) * kRows + r] = e;
+    if (h * 16 >= kb) return;  // a K step that is not multiplied
+    uint8_t* out = aimg + (size_t(b) * nbm_all + bm) * kATile + size_t(h) * kAHalf;
+#pragma unroll
+    for (int ch = 0; ch < 2; ++ch)
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint2 y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double x = part ? v[8 * ch + i].y : v[8 * ch + i].x;
+          y[i] = biased_digits(e == kNonfinite ? 0.0 : x, e - gk[16 * h + 8 * ch + i]);
+        }
+#pragma unroll
+        for (int d = 0; d < kDig; ++d) {
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w[i] = pack_bf16(digit_of(y[2 * i], d), digit_of(y[2 * i + 1], d));
+          *reinterpret_cast<uint4*>(out + (part * kDig + d) * kPlane + sw32(r, ch)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+      }
+    return;
+  }
+  const int bn = int(blockIdx.x) - nbm, k = threadIdx.x & 31;
+  uint8_t* const p = sm + (k >> 4) * kBHalf;
+  uint8_t* const q = p + kBSide;
+  const int ch = (k >> 3) & 1, kk = (k & 7) * 2;
+  for (int c = threadIdx.x >> 5; c < kCols; c += 8) {
+    const int col = c_begin + bn * kCols + c;
+    double2 v = make_double2(0.0, 0.0);
+    if (col < c_end && k < kb) v = Mb[size_t(ka + k) + size_t(lay.lda) * col];
+    const int f = field_of(v);
+    int e = __reduce_max_sync(0xffffffffu, f < 0 ? kNoEntry : f == 0x7ff ? kNonfinite : f - 1022 - gk[k]);
+    if (e == kNoEntry) e = 0;
+    if (k == 0) cexp[(size_t(b) * nbn_all + bn) * kCols + c] = e;
+    if (e == kNonfinite) v = make_double2(0.0, 0.0);
+    const uint2 yr = biased_digits(v.x, e + gk[k]), yi = biased_digits(v.y, e + gk[k]);
+#pragma unroll
+    for (int d = 0; d < kDig; ++d) {
+      const float re = digit_of(yr, d), im = digit_of(yi, d);
+      auto put = [&](uint8_t* base, int row, float x) {
+        *reinterpret_cast<uint16_t*>(base + sw32(row, ch) + kk) = uint16_t(__float_as_uint(x) >> 16);
+      };
+      put(p, d * 32 + c, re);
+      put(p, d * 32 + 16 + c, im);
+      put(q, d * 32 + c, -im);
+      put(q, d * 32 + 16 + c, re);
+    }
+  }
+  __syncthreads();
+  uint4* out = reinterpret_cast<uint4*>(bimg + (size_t(b) * nbn_all + bn) * kBTile);
+  const int bytes = kb > 16 ? kBTile : kBHalf;
+  for (int i = threadIdx.x; i < bytes / 16; i += 256) out[i] = reinterpret_cast<const uint4*>(sm)[i];
+}
+
+// The walk of a CTA: units (matrix, row tile, segment of `chunk` column tiles), every gridDim.x-th, and the column
+// tiles inside each.
+struct Tc64Work {
+  int nbm, nbn, nseg, chunk, units;
+};
+struct Tc64Tile {
+  int u, bn, bn_end, b, bm;
+  __device__ __forceinline__ void unit(const Tc64Work& w) {
+    const int seg = u % w.nseg, rest = u / w.nseg;
+    bm = rest % w.nbm;
+    b = rest / w.nbm;
+    bn = seg * w.chunk;
+    bn_end = min(bn + w.chunk, w.nbn);
+  }
+  __device__ __forceinline__ bool start(const Tc64Work& w) {
+    u = blockIdx.x;
+    if (u >= w.units) return false;
+    unit(w);
+    return true;
+  }
+  __device__ __forceinline__ bool next(const Tc64Work& w) {
+    if (++bn < bn_end) return true;
+    u += gridDim.x;
+    if (u >= w.units) return false;
+    unit(w);
+    return true;
+  }
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+    tc64_update_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end, int ka, int kb,
+                       double2* __restrict__ M, const uint8_t* __restrict__ aimg, const uint8_t* __restrict__ bimg,
+                       const int* __restrict__ rexp, const int* __restrict__ cexp, int nbm_all, int nbn_all,
+                       Tc64Work w, int* __restrict__ alpha, int alpha_n, long long polls) {
+  extern __shared__ uint8_t smraw[];
+  const uint32_t raw = smem_u32(smraw);
+  const uint32_t sbase = (raw + 1023u) & ~1023u;
+  uint8_t* const meta = smraw + (sbase - raw) + kBarOff;
+  auto bar = [&](int i) { return smem_u32(meta) + 8u * uint32_t(i); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + 128);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + 132);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nk = kb > 16 ? 2 : 1;  // K steps
+  if (blockIdx.x == 0)
+    for (int i = tid; i < alpha_n; i += kThreads) alpha[i] = 0;  // read by the split kernel before; for the next update
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 32) {
+    for (int i = 0; i < kBars; ++i)
+      mbar_init(bar(i), i == kAccEmpty || i == kAccEmpty + 1 ? uint32_t(kEpiWarps) : 1u);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    // ---- producer: the digits of A once per unit, those of B per tile ----
+    if (lane == 0) {
+      uint32_t units = 0, tiles = 0;
+      Tc64Tile t;
+      bool more = t.start(w), ok = true;
+      uint32_t a_issued[2] = {0, 0};
+      while (more && ok && !*abort_flag) {
+        const uint8_t* ab = aimg + (size_t(t.b) * nbm_all + t.bm) * kATile;
+        for (int h = 0; h < nk && ok; ++h) {
+          ok = role_wait(bar(kAEmpty + h), (units & 1) ^ 1, abort_flag, polls);
+          if (!ok) break;
+          mbar_expect_tx(bar(kAFull + h), kAHalf);
+          for (int i = 0; i < 4; ++i)
+            bulk_copy(sbase + h * kAHalf + i * (kAHalf / 4), ab + h * kAHalf + i * (kAHalf / 4), kAHalf / 4, bar(kAFull + h));
+          ++a_issued[h];
+        }
+        const int u = t.u;
+        while (more && t.u == u && ok) {
+          const int st = int(tiles % kBStages);
+          ok = role_wait(bar(kBEmpty + st), ((tiles / kBStages) & 1) ^ 1, abort_flag, polls);
+          if (!ok) break;
+          mbar_expect_tx(bar(kBFull + st), uint32_t(nk * kBHalf));
+          bulk_copy(sbase + kATile + st * kBTile, bimg + (size_t(t.b) * nbn_all + t.bn) * kBTile, uint32_t(nk * kBHalf),
+                    bar(kBFull + st));
+          ++tiles;
+          more = t.next(w);
+        }
+        ++units;
+      }
+      // every copy has landed before the CTA ends
+      for (int h = 0; h < nk; ++h)
+        if (a_issued[h]) drain_wait(bar(kAFull + h), (a_issued[h] - 1) & 1);
+      for (uint32_t q = tiles > uint32_t(kBStages) ? tiles - kBStages : 0; q < tiles; ++q)
+        drain_wait(bar(kBFull + int(q % kBStages)), (q / kBStages) & 1);
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer ----
+    if (lane == 0) {
+      uint32_t units = 0, tiles = 0;
+      bool issued = false, ok = true;
+      Tc64Tile t;
+      bool more = t.start(w), first = true;
+      while (more && ok && !*abort_flag) {
+        const uint32_t buf = tiles & 1;
+        const int st = int(tiles % kBStages);
+        ok = role_wait(bar(kAccEmpty + int(buf)), ((tiles >> 1) & 1) ^ 1, abort_flag, polls) &&
+             role_wait(bar(kBFull + st), (tiles / kBStages) & 1, abort_flag, polls);
+        if (!ok) break;
+        Tc64Tile nx = t;
+        const bool nmore = nx.next(w);
+        const bool last = !nmore || nx.u != t.u;  // of the unit
+        for (int h = 0; h < nk; ++h) {
+          if (first && !(ok = role_wait(bar(kAFull + h), units & 1, abort_flag, polls))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sA = sbase + h * kAHalf, sP = sbase + kATile + st * kBTile + h * kBHalf;
+          const uint64_t dp = desc_sw32(sP), dq = desc_sw32(sP + kBSide);
+#pragma unroll 1
+          for (int i = 0; i < kDig; ++i) {
+            // digit i + 1 of A against digits 1 .. 8 - i of B: levels i + 2 .. 9
+            const uint32_t d = tmem + buf * 256 + uint32_t(32 * i), id = idesc_bf16(32 * (kDig - i));
+            mma_bf16(d, desc_sw32(sA + i * kPlane), dp, id, h || i ? 1u : 0u);
+            mma_bf16(d, desc_sw32(sA + (kDig + i) * kPlane), dq, id, 1u);
+          }
+          issued = true;
+          if (last) mma_commit(bar(kAEmpty + h));
+        }
+        if (!ok) break;
+        mma_commit(bar(kBEmpty + st));
+        mma_commit(bar(kAccFull + int(buf)));
+        ++tiles;
+        first = last;
+        if (last) ++units;
+        t = nx;
+        more = nmore;
+      }
+      if (issued) {  // every MMA has completed before the tensor memory is freed
+        mma_commit(bar(kDrain));
+        drain_wait(bar(kDrain), 0);
+      }
+    }
+  } else {
+    // ---- epilogue: warp (quarter, g) finishes rows [32 quarter, + 32), columns [4 g, + 4) of every tile ----
+    const int g = (warp - 2) >> 2, quarter = warp & 3;
+    const uint32_t lane_off = uint32_t(quarter * 32) << 16;
+    const int lda = lay.lda;
+    uint32_t tiles = 0;
+    bool direct = false;  // the waits ran out: the remaining tiles in FP64 multiply-adds
+    Tc64Tile t;
+    bool more = t.start(w);
+    // C of this thread's four entries, each loaded again for the next tile once it has been used
+    double2 cn[4];
+    auto c_ptr = [&](const Tc64Tile& q) {
+      return M + size_t(q.b) * lay.stride + size_t(r_begin + q.bm * kRows + quarter * 32 + lane) +
+             size_t(lda) * size_t(c_begin + q.bn * kCols + 4 * g);
+    };
+    // columns of the tile that this thread has: 0 where its row lies outside the block
+    auto c_count = [&](const Tc64Tile& q) {
+      return r_begin + q.bm * kRows + quarter * 32 + lane < r_end ? c_end - (c_begin + q.bn * kCols + 4 * g) : 0;
+    };
+    double2* cur = M;
+    int have = 0;
+    if (more) {
+      cur = c_ptr(t);
+      have = c_count(t);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cn[j] = j < have ? cur[size_t(lda) * j] : make_double2(0.0, 0.0);
+    }
+    while (more) {
+      const int er = rexp[(size_t(t.b) * nbm_all + t.bm) * kRows + quarter * 32 + lane];
+      const int4 ec4 = *reinterpret_cast<const int4*>(cexp + (size_t(t.b) * nbn_all + t.bn) * kCols + 4 * g);
+      const int ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w};
+      const int tb = t.b, tcol = c_begin + t.bn * kCols + 4 * g, trow = r_begin + t.bm * kRows + quarter * 32 + lane;
+      more = t.next(w);
+      double2* const nxt = more ? c_ptr(t) : M;
+      const int nhave = more ? c_count(t) : 0;
+      const uint32_t buf = tiles & 1;
+      if (!direct) {
+        const bool ready = role_wait(bar(kAccFull + int(buf)), (tiles >> 1) & 1, abort_flag, polls);
+        direct = !__all_sync(0xffffffffu, ready);
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t lv[2][kDig][2];
+        __syncwarp();
+        if (!direct) {
+          const uint32_t ta = tmem + buf * 256 + lane_off + uint32_t(4 * g + 2 * half);
+#pragma unroll
+          for (int part = 0; part < 2; ++part)
+#pragma unroll
+            for (int s = 0; s < kDig; ++s)
+              asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
+                           : "=r"(lv[part][s][0]), "=r"(lv[part][s][1])
+                           : "r"(ta + uint32_t(32 * s + 16 * part)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (half == 1) {  // the accumulators are in registers: they may be overwritten
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            if (lane == 0) mbar_arrive(bar(kAccEmpty + int(buf)));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int c = 2 * half + j;
+          if (c < have) {
+            double2 v = cn[c];
+            double2 p;
+            if (direct || er == kNonfinite || ec[c] == kNonfinite) {
+              const double2* Mb = M + size_t(tb) * lay.stride;
+              p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
+            } else {
+              float sr[kDig], si[kDig];
+#pragma unroll
+              for (int s = 0; s < kDig; ++s) {
+                sr[s] = __uint_as_float(lv[0][s][j]);
+                si[s] = __uint_as_float(lv[1][s][j]);
+              }
+              p = make_double2(join_levels(sr, er + ec[c]), join_levels(si, er + ec[c]));
+            }
+            v.x -= p.x;
+            v.y -= p.y;
+            cur[size_t(lda) * c] = v;
+          }
+          cn[c] = c < nhave ? nxt[size_t(lda) * c] : make_double2(0.0, 0.0);
+        }
+      }
+      ++tiles;
+      cur = nxt;
+      have = nhave;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+namespace {
+struct Tc64Images {
+  int nbm, nbn;
+  size_t a, b, r, c, total;  // byte offsets of the A and B images, the row and column exponents
+};
+Tc64Images tc64_images(int n, int m, int batch) {
+  Tc64Images v;
+  v.nbm = (n + kRows - 1) / kRows;
+  v.nbn = (n + m + kCols - 1) / kCols;
+  v.a = 0;
+  v.b = v.a + size_t(batch) * v.nbm * kATile;
+  v.r = v.b + size_t(batch) * v.nbn * kBTile;
+  v.c = v.r + size_t(batch) * v.nbm * kRows * sizeof(int);
+  v.total = v.c + size_t(batch) * v.nbn * kCols * sizeof(int);
+  return v;
+}
+}  // namespace
+
+size_t tc64_image_bytes(int n, int m, int batch) { return tc64_images(n, m, batch).total; }
+
+void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int c_begin, int c_end, int ka, int kb,
+                 double2* M, uint8_t* images, int* alpha, int image_batch, long long wait_polls, cudaStream_t s) {
+  const int rows = r_end - r_begin, cols = c_end - c_begin;
+  if (rows <= 0 || cols <= 0 || kb <= 0 || image_batch <= 0) return;
+  const Tc64Images im = tc64_images(lay.n, lay.m, image_batch);
+  int* rexp = reinterpret_cast<int*>(images + im.r);
+  int* cexp = reinterpret_cast<int*>(images + im.c);
+  const int sms = current_sm_count();
+  ensure_smem_limit(reinterpret_cast<const void*>(tc64_update_kernel), size_t(kSmem));
+  for (int b0 = 0; b0 < batch; b0 += image_batch) {
+    const int nb = std::min(image_batch, batch - b0);
+    double2* Mb = M + size_t(b0) * lay.stride;
+    Tc64Work w;
+    w.nbm = (rows + kRows - 1) / kRows;
+    w.nbn = (cols + kCols - 1) / kCols;
+    // Column tiles per unit: a unit loads the 128 KB of A digits once (about one tile's time), so up to 24 tiles
+    // share them; fewer where that would leave SMs without a unit.
+    const long long tiles = (long long)nb * w.nbm * w.nbn;
+    const int want = int(std::max<long long>(1, std::min<long long>(24, (tiles + sms - 1) / sms)));
+    w.nseg = (w.nbn + want - 1) / want;
+    w.chunk = (w.nbn + w.nseg - 1) / w.nseg;
+    w.units = nb * w.nbm * w.nseg;
+    count_launch();
+    tc64_scale_kernel<<<dim3(unsigned(w.nbm), unsigned(nb)), kRows, 0, s>>>(lay, r_begin, r_end, ka, kb, Mb, alpha);
+    count_launch();
+    tc64_split_kernel<<<dim3(unsigned(w.nbm + w.nbn), unsigned(nb)), 256, 0, s>>>(
+        lay, r_begin, r_end, c_begin, c_end, ka, kb, Mb, alpha, images + im.a, images + im.b, rexp, cexp, w.nbm, im.nbm,
+        im.nbn);
+    count_launch();
+    tc64_update_kernel<<<unsigned(std::min(w.units, sms)), kThreads, kSmem, s>>>(
+        lay, r_begin, r_end, c_begin, c_end, ka, kb, Mb, images + im.a, images + im.b, rexp, cexp, im.nbm, im.nbn, w,
+        alpha, nb * 32, wait_polls > 0 ? wait_polls : kTcWaitPolls);
+  }
+}
+
+}  // namespace rfx
