@@ -51,6 +51,7 @@
 #include <cstdint>
 #include "cplx.cuh"
 #include "batched_lu.cuh"
+#include "digits64.cuh"
 
 namespace rfx {
 
@@ -58,7 +59,6 @@ namespace {
 
 constexpr int kRows = 128;                       // rows per tile (MMA M)
 constexpr int kCols = 16;                        // columns per tile
-constexpr int kDig = 8;                          // digits per value
 constexpr int kPlane = kRows * 32;               // one digit plane of A, one K step (16 columns): 4 KB
 constexpr int kAHalf = 2 * kDig * kPlane;        // re and im digits of one K step: 64 KB
 constexpr int kATile = 2 * kAHalf;               // 128 KB
@@ -72,7 +72,6 @@ constexpr uint32_t kTmemCols = 512;              // two accumulator sets of 8 le
 constexpr int kBarOff = kATile + kBStages * kBTile;
 constexpr int kSmem = kBarOff + 256 + 1024;      // + alignment of the base to 1 KB
 static_assert(kSmem <= 227 * 1024, "dynamic shared memory per CTA");
-constexpr int kNonfinite = 1 << 28;              // exponent of a row or column with an infinity or NaN
 
 // barriers: A halves full / empty, B stages full / empty, accumulators full / empty, drain
 enum : int { kAFull = 0, kAEmpty = 2, kBFull = 4, kBEmpty = 4 + kBStages, kAccFull = 4 + 2 * kBStages,
@@ -134,12 +133,14 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // Bounded wait of one role on another (poll budget, or 1 s); gives up early once the CTA's abort flag is up,
 // and raises that flag when it runs out.
 __device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long polls) {
-  const uint64_t t0 = global_ns();
+  uint64_t t0 = 0;  // the clock is read after 256 polls: its read takes longer than most waits
   for (long long it = 0; it < polls; ++it) {
     if (mbar_try(bar, parity)) return true;
     if ((it & 255) == 255) {
       if (*abort_flag) return false;
-      if (global_ns() - t0 > 1000000000ull) break;
+      const uint64_t t = global_ns();
+      if (t0 == 0) t0 = t;
+      else if (t - t0 > 1000000000ull) break;
     }
   }
   *abort_flag = 1;
@@ -147,67 +148,19 @@ __device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, volatil
 }
 // Drain wait for work this thread issued itself (the full default budget, no abort exit).
 __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return;
   const uint64_t t0 = global_ns();
   for (long long it = 0; it < kTcWaitPolls; ++it)
     if (mbar_try(bar, parity) || ((it & 1023) == 1023 && global_ns() - t0 > 1000000000ull)) return;
 }
 
-__device__ __forceinline__ int field_of(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-// larger exponent field of the two parts; -1 for zero
-__device__ __forceinline__ int field_of(double2 v) {
-  return v.x == 0.0 && v.y == 0.0 ? -1 : max(field_of(v.x), field_of(v.y));
-}
-constexpr int kNoEntry = -(1 << 20);  // exponent of a row or column of zeros
-// v 2^(62 - e) rounded to an integer (|v| < 2^e), biased by 128 in every byte: byte j holds digit 8 - j plus 128.
-__device__ __forceinline__ uint2 biased_digits(double v, int e) {
-  const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
-  const int field = int(bits >> 52) & 0x7ff;
-  unsigned long long x = bits & 0xfffffffffffffull;
-  if (field) x |= 1ull << 52;
-  const int sh = max(field, 1) - 1075 + 62 - e;  // <= 9
-  if (sh >= 0) x <<= sh;
-  else x = sh < -54 ? 0ull : (x + (1ull << (-sh - 1))) >> -sh;
-  if (bits >> 63) x = 0ull - x;
-  x += 0x8080808080808080ull;
-  return make_uint2(uint32_t(x), uint32_t(x >> 32));
-}
-// digit d (0 .. 7, most significant first) as a float
-__device__ __forceinline__ float digit_of(uint2 y, int d) {
-  const int j = 7 - d;
-  const uint32_t w = j >= 4 ? y.y : y.x;
-  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | (j & 3))) - 8388736.0f;  // 2^23 + 128
-}
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-}
-
 // sum_k A[row, k] B[k, col] in FP64 multiply-adds: the path of rows and columns that the digits cannot hold, and
 // of tiles whose waits ran out.
-__device__ __noinline__ double2 direct_sum(const double2* __restrict__ arow, const double2* __restrict__ bcol, int lda,
-                                           int kb) {
+__device__ __forceinline__ double2 direct_sum(const double2* arow, const double2* bcol, int lda, int kb) {
   double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 1
   for (int k = 0; k < kb; ++k) cfma(acc, arow[size_t(lda) * k], bcol[k]);
   return acc;
-}
-
-// The eight exact level sums of one real output (levels 2 .. 9, weights 2^-12 .. 2^-68 of 2^e) as an FP64 number.
-__device__ __forceinline__ double join_levels(const float (&s)[kDig], int e) {
-  const int p = __float2int_rn(s[0]) * 256 + __float2int_rn(s[1]);
-  const int q = __float2int_rn(s[2]) * 256 + __float2int_rn(s[3]);
-  const int r = __float2int_rn(s[4]) * 256 + __float2int_rn(s[5]);
-  const int l = __float2int_rn(s[6]) * 256 + __float2int_rn(s[7]);
-  // h = the levels 2 .. 7 in units of 2^-52: |h| < 2^59; l holds levels 8 and 9, 16 bits further down
-  const long long h = (static_cast<long long>(p) * 4294967296LL) + static_cast<long long>(q) * 65536 + r;
-  const bool small = ((h + (1ll << 45)) >> 46) == 0;
-  const long long v = small ? h * 65536 + l : h + ((l + 32768) >> 16);
-  const int ex = e - (small ? 68 : 52);
-  double d = __ll2double_rn(v);
-  if (ex > -900 && ex < 900) {  // 1 <= |d| < 2^63 when it is not zero: its exponent takes ex without leaving the range
-    int hi = __double2hiint(d);
-    if (v != 0) hi += ex * (1 << 20);
-    return __hiloint2double(hi, __double2loint(d));
-  }
-  return scalbn(d, ex);
 }
 
 }  // namespace
@@ -514,49 +467,42 @@ __global__ void __launch_bounds__(kThreads, 1)
         direct = !__all_sync(0xffffffffu, ready);
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // one column at a time: the level sums of more would not fit in registers beside C, and C spilled to local
+      // memory stalls on its own loads (4 us a tile)
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t lv[2][kDig][2];
+      for (int c = 0; c < 4; ++c) {
+        uint32_t lv[2 * kDig];
         __syncwarp();
         if (!direct) {
-          const uint32_t ta = tmem + buf * 256 + lane_off + uint32_t(4 * g + 2 * half);
+          const uint32_t ta = tmem + buf * 256 + lane_off + uint32_t(4 * g + c);
 #pragma unroll
-          for (int part = 0; part < 2; ++part)
-#pragma unroll
-            for (int s = 0; s < kDig; ++s)
-              asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];"
-                           : "=r"(lv[part][s][0]), "=r"(lv[part][s][1])
-                           : "r"(ta + uint32_t(32 * s + 16 * part)));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (half == 1) {  // the accumulators are in registers: they may be overwritten
+          for (int s = 0; s < kDig; ++s) {
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(lv[s]) : "r"(ta + uint32_t(32 * s)));
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];"
+                         : "=r"(lv[kDig + s])
+                         : "r"(ta + uint32_t(32 * s + 16)));
+          }
+          // the loaded registers pass through the wait, so that nothing reads them before it
+          asm volatile("tcgen05.wait::ld.sync.aligned;"
+                       : "+r"(lv[0]), "+r"(lv[1]), "+r"(lv[2]), "+r"(lv[3]), "+r"(lv[4]), "+r"(lv[5]), "+r"(lv[6]),
+                         "+r"(lv[7]), "+r"(lv[8]), "+r"(lv[9]), "+r"(lv[10]), "+r"(lv[11]), "+r"(lv[12]),
+                         "+r"(lv[13]), "+r"(lv[14]), "+r"(lv[15])::"memory");
+          if (c == 3) {  // the accumulators are in registers: they may be overwritten
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             if (lane == 0) mbar_arrive(bar(kAccEmpty + int(buf)));
           }
         }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int c = 2 * half + j;
-          if (c < have) {
-            double2 v = cn[c];
-            double2 p;
-            if (direct || er == kNonfinite || ec[c] == kNonfinite) {
-              const double2* Mb = M + size_t(tb) * lay.stride;
-              p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
-            } else {
-              float sr[kDig], si[kDig];
-#pragma unroll
-              for (int s = 0; s < kDig; ++s) {
-                sr[s] = __uint_as_float(lv[0][s][j]);
-                si[s] = __uint_as_float(lv[1][s][j]);
-              }
-              p = make_double2(join_levels(sr, er + ec[c]), join_levels(si, er + ec[c]));
-            }
-            v.x -= p.x;
-            v.y -= p.y;
-            cur[size_t(lda) * c] = v;
+        if (c < have) {
+          double2 p;
+          if (direct || er == kNonfinite || ec[c] == kNonfinite) {
+            const double2* Mb = M + size_t(tb) * lay.stride;
+            p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
+          } else {
+            p = make_double2(join_levels(lv, er + ec[c]), join_levels(lv + kDig, er + ec[c]));
           }
-          cn[c] = c < nhave ? nxt[size_t(lda) * c] : make_double2(0.0, 0.0);
+          cur[size_t(lda) * c] = make_double2(cn[c].x - p.x, cn[c].y - p.y);
         }
+        cn[c] = c < nhave ? nxt[size_t(lda) * c] : make_double2(0.0, 0.0);
       }
       ++tiles;
       cur = nxt;
