@@ -836,11 +836,10 @@ static bool fit_panel(int elem, int nb, int n, int& cluster, int& rpc, int& smem
       for (int cl = 1; cl <= (pass == 0 ? 8 : 16); cl *= 2) {
         const size_t budget = size_t(pass == 0 ? 100 : 200) * 1024;
         const int r = (n + cl - 1) / cl;
-        const size_t bsz = panel_smem_any(elem, nb, r, n, g == 1);
-        if (bsz <= budget) {
+        if (panel_smem_any(elem, nb, r, n, g == 1) <= budget) {
           cluster = cl;
-          rpc = r;
-          smem = int(bsz);
+          rpc = elem == 16 ? (r + 15) / 16 * 16 : r;  // the FP64 panel works in whole 16-row tiles
+          smem = int(panel_smem_any(elem, nb, rpc, n, g == 1));
           pos_global = g;
           return true;
         }
@@ -1020,12 +1019,13 @@ static void rhs_lower_any(int nb, const BatchLayout& lay, int batch, int k, int 
 template <typename T>
 static cudaError_t panel_any(const PanelConfig& pc, int nb, const BatchLayout& lay, int batch, int k, cplx<T>* M,
                              const LuWork& w, cudaStream_t s) {
-  if (nb == 32) return launch_panel<T, 32>(pc, lay, batch, k, M, w, s);
-  if (nb == 16) return launch_panel<T, 16>(pc, lay, batch, k, M, w, s);
   if constexpr (sizeof(T) == 8) {
-    if (nb == 8) return launch_panel<T, 8>(pc, lay, batch, k, M, w, s);
+    return launch_panel64(pc, nb, lay, batch, k, M, w, s);
+  } else {
+    if (nb == 32) return launch_panel<T, 32>(pc, lay, batch, k, M, w, s);
+    if (nb == 16) return launch_panel<T, 16>(pc, lay, batch, k, M, w, s);
+    return cudaErrorInvalidValue;
   }
-  return cudaErrorInvalidValue;
 }
 
 // FP32 elimination with two-level blocking: each 64-column outer block is

@@ -97,6 +97,10 @@ struct LuWork {
   int pair128 = 0;
 };
 
+// The FP64 cluster panel of columns [k, k + nb) (panel64.cu), nb 32, 16 or 8.
+cudaError_t launch_panel64(const PanelConfig& pc, int nb, const BatchLayout& lay, int batch, int k, double2* M,
+                           const LuWork& w, cudaStream_t s);
+
 // Elimination of the whole augmented system: after it, columns [0, n) hold
 // L\U and columns [n, n+m) hold Y = L^-1 P B.
 template <typename T>
