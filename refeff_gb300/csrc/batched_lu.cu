@@ -834,7 +834,8 @@ static bool fit_panel(int elem, int nb, int n, int& cluster, int& rpc, int& smem
   for (int pass = 0; pass < 2; ++pass)
     for (int g = global_first ? 1 : 0; g < (pass == 0 && !global_first ? 1 : 2); ++g)  // bookkeeping in global memory only as the last resort
       for (int cl = 1; cl <= (pass == 0 ? 8 : 16); cl *= 2) {
-        const size_t budget = size_t(pass == 0 ? 100 : 200) * 1024;
+        // (the 32-column FP64 panel has 25 KB of static shared memory beside these)
+        const size_t budget = size_t(pass == 0 ? 100 : elem == 16 && nb == 32 ? 195 : 200) * 1024;
         const int r = (n + cl - 1) / cl;
         if (panel_smem_any(elem, nb, r, n, g == 1) <= budget) {
           cluster = cl;

@@ -46,38 +46,58 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
+// v 2^ex rounded to FP64 in integer operations: the conversion instruction runs on the FP64 pipe, where a warp's
+// instruction takes 64 cycles of its quarter of the SM.
+__device__ __forceinline__ double scaled_double(long long v, int ex) {
+  if (v == 0) return 0.0;
+  const uint32_t sign = uint32_t(static_cast<unsigned long long>(v) >> 32) & 0x80000000u;
+  const unsigned long long a = static_cast<unsigned long long>(v < 0 ? -v : v);
+  const int lz = __clzll(static_cast<long long>(a));
+  const unsigned long long m = a << lz;  // leading one at bit 63
+  const int field = 1023 + 63 - lz + ex;
+  if (field > 0 && field < 2046) {
+    // 53 bits, rounded half up; a carry out of the mantissa moves into the exponent as it should
+    const unsigned long long bits = (m >> 11) + ((m >> 10) & 1) + (static_cast<unsigned long long>(field - 1) << 52);
+    return __hiloint2double(int(uint32_t(bits >> 32) | sign), int(uint32_t(bits)));
+  }
+  return scalbn(__ll2double_rn(v), ex);
+}
+
 // The eight exact level sums of one real output (levels 2 .. 9, weights 2^-12 .. 2^-68 of 2^e, bit patterns of
-// integer-valued floats) as an FP64 number.
+// integer-valued floats) as an FP64 number.  Integers up to 2^22 are read off the mantissa after adding 1.5 x 2^23;
+// kWide (more than 16 products per pair, K > 8): levels 7 and 8 can exceed that and are converted, level 9 may then be
+// off by one unit of 2^-68.
+template <bool kWide>
 __device__ __forceinline__ double join_levels(const uint32_t* s, int e) {
-  auto sum = [&](int i) { return __float2int_rn(__uint_as_float(s[i])); };
-  const int p = sum(0) * 256 + sum(1), q = sum(2) * 256 + sum(3);
-  const int r = sum(4) * 256 + sum(5), l = sum(6) * 256 + sum(7);
+  constexpr int kBase = 0x4B400000;  // the pattern of 1.5 x 2^23
+  auto pat = [&](int i) { return __float_as_int(__uint_as_float(s[i]) + 12582912.0f); };
+  auto sum = [&](int i) { return kWide ? __float2int_rn(__uint_as_float(s[i])) : pat(i) - kBase; };
+  const int p = pat(0) * 256 + pat(1) - int(257u * uint32_t(kBase));
+  const int q = pat(2) * 256 + pat(3) - int(257u * uint32_t(kBase));
+  const int r = (pat(4) - kBase) * 256 + sum(5);
+  const int l = sum(6) * 256 + (pat(7) - kBase);
   // h = the levels 2 .. 7 in units of 2^-52: |h| < 2^59; l holds levels 8 and 9, 16 bits further down
   const long long h = (static_cast<long long>(p) * 4294967296LL) + static_cast<long long>(q) * 65536 + r;
   const bool small = ((h + (1ll << 45)) >> 46) == 0;
   const long long v = small ? h * 65536 + l : h + ((l + 32768) >> 16);
-  const int ex = e - (small ? 68 : 52);
-  double d = __ll2double_rn(v);
-  if (ex > -900 && ex < 900) {  // 1 <= |d| < 2^63 when it is not zero: its exponent takes ex without leaving the range
-    int hi = __double2hiint(d);
-    if (v != 0) hi += ex * (1 << 20);
-    return __hiloint2double(hi, __double2loint(d));
-  }
-  return scalbn(d, ex);
+  return scaled_double(v, e - (small ? 68 : 52));
 }
 
 // ---------------------------------------------------------------------------
-// Warp-level form: C (16 x 8 complex) -= A (16 x 8) B (8 x 8) by mma.sync m16n8k8
-// on the digits, for updates inside kernels that hold their operands in shared
-// memory (too shallow, K = 8, to be worth a trip through tensor memory).
+// Warp-level form: C (16 x 8 complex) -= A (16 x 8) B (8 x 8) by mma.sync on the
+// digits, for updates inside kernels that hold their operands in shared memory
+// (too shallow, K = 8, to be worth a trip through tensor memory).  One
+// m16n8k16 takes the real and imaginary parts of A side by side:
+// Cr = [Ar Ai] [Br; -Bi], Ci = [Ar Ai] [Bi; Br].
 // Lane (g = lane / 4, t = lane % 4) holds A[g or g + 8][2t, 2t + 1], B[2t, 2t + 1][g]
 // and C[g or g + 8][2t, 2t + 1].
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void mma_k8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+__device__ __forceinline__ void mma_k16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                        uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(b));
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 struct DigitTileA {
@@ -156,10 +176,8 @@ __device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t
     const uint32_t br = words[(2 * j) * 32 + lane], bi = words[(2 * j + 1) * 32 + lane], nbi = bi ^ 0x80008000u;
 #pragma unroll
     for (int i = 0; i + j < kDig; ++i) {
-      mma_k8(cr[i + j], a.re[i][0], a.re[i][1], br);
-      mma_k8(ci[i + j], a.re[i][0], a.re[i][1], bi);
-      mma_k8(cr[i + j], a.im[i][0], a.im[i][1], nbi);
-      mma_k8(ci[i + j], a.im[i][0], a.im[i][1], br);
+      mma_k16(cr[i + j], a.re[i][0], a.re[i][1], a.im[i][0], a.im[i][1], br, nbi);
+      mma_k16(ci[i + j], a.re[i][0], a.re[i][1], a.im[i][0], a.im[i][1], bi, br);
     }
   }
 #pragma unroll
@@ -173,7 +191,7 @@ __device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t
         li[s] = __float_as_uint(ci[s][2 * h + q]);
       }
       const int e = a.e[h] + ecol[2 * t + q];
-      p[h][q] = make_double2(join_levels(lr, e), join_levels(li, e));
+      p[h][q] = make_double2(join_levels<false>(lr, e), join_levels<false>(li, e));
     }
 }
 

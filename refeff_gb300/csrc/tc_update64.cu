@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const double2* Mb = M + size_t(tb) * lay.stride;
             p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
           } else {
-            p = make_double2(join_levels(lv, er + ec[c]), join_levels(lv + kDig, er + ec[c]));
+            p = make_double2(join_levels<true>(lv, er + ec[c]), join_levels<true>(lv + kDig, er + ec[c]));
           }
           cur[size_t(lda) * c] = make_double2(cn[c].x - p.x, cn[c].y - p.y);
         }
