@@ -1006,13 +1006,15 @@ static void gemm_any(int nb, const BatchLayout& lay, int batch, int r_begin, int
 template <typename T, bool kSolve = true>
 static void rhs_lower_any(int nb, const BatchLayout& lay, int batch, int k, int c_begin, int c_end, cplx<T>* M,
                           const LuWork& w, const int* skip, cudaStream_t s) {
-  switch (nb) {
-    case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
-    case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
-    case 16: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
-    default:
-      if constexpr (sizeof(T) == 8) launch_rhs_lower<T, 8, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s);
-      break;
+  if constexpr (sizeof(T) == 8) {
+    static_assert(kSolve, "the FP64 panels have no inner panels whose moves go to earlier columns");
+    launch_trsm64(false, lay, batch, k, min(nb, lay.n - k), c_begin, c_end, M, w, skip, s);
+  } else {
+    switch (nb) {
+      case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+      case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+      default: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+    }
   }
 }
 
@@ -1181,16 +1183,15 @@ void lu_backward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, c
   dim3 grid(unsigned((lay.m + 7) / 8), unsigned(batch));
   for (int k = last; k >= 0; k -= pc.nb) {
     const int kb = min(pc.nb, n - k);
-    count_launch();
-    switch (pc.nb) {
-      case 64: rhs_upper_kernel<T, 64><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
-      case 32: rhs_upper_kernel<T, 32><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
-      case 16: rhs_upper_kernel<T, 16><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
-      default:
-        if constexpr (sizeof(T) == 8) rhs_upper_kernel<T, 8><<<grid, 256, 0, s>>>(lay, k, M, skip);
-        break;
-    }
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (sizeof(T) == 4) {
+      count_launch();
+      switch (pc.nb) {
+        case 64: rhs_upper_kernel<T, 64><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
+        case 32: rhs_upper_kernel<T, 32><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
+        default: rhs_upper_kernel<T, 16><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
+      }
+    } else {
+      launch_trsm64(true, lay, batch, k, kb, n, col_end, M, LuWork(), skip, s);
       if (w && w->tc_images && kb <= kTc64Depth && !skip) {
         tc64_update(lay, batch, 0, k, n, col_end, k, kb, M, w->tc_images, w->tc_alpha, w->tc_image_batch,
                     w->tc_wait_polls, s);

@@ -101,6 +101,11 @@ struct LuWork {
 cudaError_t launch_panel64(const PanelConfig& pc, int nb, const BatchLayout& lay, int batch, int k, double2* M,
                            const LuWork& w, cudaStream_t s);
 
+// FP64 solves with the triangle in rows and columns [k, k + kb) (trsm64.cu), kb <= 32: upper, X = U11^-1 Y on the
+// columns; else the moves of the panel at k, then U12 = L11^-1 (P A12).
+void launch_trsm64(bool upper, const BatchLayout& lay, int batch, int k, int kb, int c_begin, int c_end, double2* M,
+                   const LuWork& w, const int* skip, cudaStream_t s);
+
 // Elimination of the whole augmented system: after it, columns [0, n) hold
 // L\U and columns [n, n+m) hold Y = L^-1 P B.
 template <typename T>

@@ -104,9 +104,9 @@ struct DigitTileA {
   uint32_t re[kDig][2], im[kDig][2];  // rows g and g + 8
   int e[2];                           // their exponents
 };
-// Columns of A that are small in all 16 rows lose as many bits: a tile with one more than this many below its
-// rows' largest entries is left to the FP64 pipe, as is one with an infinity or NaN.
-constexpr int kTileSlack = 6;
+// A column of A that lies 2^-s below the rows' largest entries in all 16 rows keeps 62 - s bits: a tile with one beyond
+// this s (fewer than FP64's 53) is left to the FP64 pipe, as is one with an infinity or NaN.
+constexpr int kTileSlack = 9;
 
 // v[h][q] = A[g + 8 h][2t + q].  False (whole warp): the tile does not fit the digits.
 __device__ __forceinline__ bool cut_tile_a(const double2 (&v)[2][2], DigitTileA& a) {
