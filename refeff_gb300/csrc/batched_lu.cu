@@ -19,6 +19,7 @@
 // applies each panel's moves to the new right-hand side just before that
 // panel's L columns, which is the same permutation order the elimination saw.
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <climits>
 #include "cplx.cuh"
 #include "batched_lu.cuh"
@@ -1025,6 +1026,9 @@ static cudaError_t panel_any(const PanelConfig& pc, int nb, const BatchLayout& l
   if constexpr (sizeof(T) == 8) {
     return launch_panel64(pc, nb, lay, batch, k, M, w, s);
   } else {
+    bool served = false;
+    const cudaError_t err = launch_panel32(nb, std::max(pc.cluster, 8), lay, batch, k, M, w, s, served);
+    if (served || err != cudaSuccess) return err;
     if (nb == 32) return launch_panel<T, 32>(pc, lay, batch, k, M, w, s);
     if (nb == 16) return launch_panel<T, 16>(pc, lay, batch, k, M, w, s);
     return cudaErrorInvalidValue;

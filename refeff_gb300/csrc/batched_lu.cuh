@@ -101,6 +101,10 @@ struct LuWork {
 cudaError_t launch_panel64(const PanelConfig& pc, int nb, const BatchLayout& lay, int batch, int k, double2* M,
                            const LuWork& w, cudaStream_t s);
 
+// The FP32 panel of columns [k, k + nb) in registers (panel32.cu), nb 16 or 32; served = false (nothing launched) when
+// its rows do not fit a cluster of max_cluster CTAs.
+cudaError_t launch_panel32(int nb, int max_cluster, const BatchLayout& lay, int batch, int k, float2* M,
+                           const LuWork& w, cudaStream_t s, bool& served);
 // FP64 solves with the triangle in rows and columns [k, k + kb) (trsm64.cu), kb <= 32: upper, X = U11^-1 Y on the
 // columns; else the moves of the panel at k, then U12 = L11^-1 (P A12).
 void launch_trsm64(bool upper, const BatchLayout& lay, int batch, int k, int kb, int c_begin, int c_end, double2* M,
