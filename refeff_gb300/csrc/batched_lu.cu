@@ -1105,8 +1105,8 @@ static cudaError_t lu_eliminate_two_level(const PanelConfig& pc, const BatchLayo
     }
   };
   auto update = [&](int k, int kb, int c_end) {
-    if (w.tc_images) tc_trailing_update(lay, batch, k, kb, c_end, M, w.tc_images, w.tc_err, nullptr, w.tc_wait_polls,
-                                        w.tc_spans, s);
+    if (w.tc_images) tc_trailing_update(lay, batch, k, kb, c_end, M, w.tc_images, w.tc_alpha, w.tc_err, nullptr,
+                                        w.tc_wait_polls, w.tc_spans, s);
     else gemm_any<float>(64, lay, batch, k + kb, n, k + kb, c_end, k, kb, M, nullptr, s);
   };
   for (int k = 0; k < n; k += pair ? 128 : 64) {
@@ -1148,7 +1148,8 @@ cudaError_t lu_eliminate(const PanelConfig& pc, const BatchLayout& lay, int batc
     rhs_lower_any<T>(pc.nb, lay, batch, k, k + kb, col_end, M, wl, nullptr, s);
     if constexpr (sizeof(T) == 4) {
       if (w.tc_images) {
-        tc_trailing_update(lay, batch, k, kb, col_end, M, w.tc_images, w.tc_err, nullptr, w.tc_wait_polls, w.tc_spans, s);
+        tc_trailing_update(lay, batch, k, kb, col_end, M, w.tc_images, w.tc_alpha, w.tc_err, nullptr, w.tc_wait_polls,
+                           w.tc_spans, s);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
         continue;

@@ -47,13 +47,14 @@ struct KernelSpans {
 // Default poll budget of each mbarrier wait in the tensor-core update (the
 // waits also give up after one second of %globaltimer).
 constexpr long long kTcWaitPolls = 1LL << 26;
-// C -= L21 U12 for elimination step k with tcgen05 MMAs (split TF32, FP32 accumulation).
+// C -= L21 U12 for elimination step k with tcgen05 MMAs (two FP16 terms per value, FP32 accumulation).
+// alpha: kTcKMax ints per system, zero before the first call and left zero by each.
 // wait_polls bounds the waits of the producer, MMA and epilogue roles on each
 // other; the final waits for copies and MMAs still in flight keep the default
 // budget, so nothing is outstanding when a CTA exits.  spans (nullable)
 // records CUDA events around the kernel while spans->on.
 void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int col_end, float2* M, uint8_t* images,
-                        int* err_flag, const int* skip, long long wait_polls, KernelSpans* spans, cudaStream_t s);
+                        int* alpha, int* err_flag, const int* skip, long long wait_polls, KernelSpans* spans, cudaStream_t s);
 
 // C[r_begin:r_end, c_begin:c_end] -= M[rows, ka:ka+kb] M[ka:ka+kb, cols] in FP64 accuracy, kb <= 32, on the tensor
 // cores from exact 8-bit digit products (tc_update64.cu).  images: tc64_image_bytes of image_batch systems; a larger
@@ -69,7 +70,7 @@ void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int 
 struct LuWork {
   uint8_t* tc_images = nullptr;  // operand images for the tensor-core updates (FP32 or FP64); null = CUDA cores
   int tc_image_batch = 0;        // systems the FP64 update's images hold
-  int* tc_alpha = nullptr;       // the FP64 update's column scales (tc64_update)
+  int* tc_alpha = nullptr;       // the updates' column scales (tc_trailing_update, tc64_update), zero between updates
   int* tc_err = nullptr;         // set when a tensor-core wait timed out
   long long tc_wait_polls = kTcWaitPolls;  // poll budget of the role waits in the tensor-core update
   KernelSpans* tc_spans = nullptr;         // events around the tensor-core update launches (profiling)

@@ -435,7 +435,7 @@ struct Workspace {
   size_t tc_image_size = 0;
   bool use_tc64 = false;             // FP64 block updates on the tensor cores
   int tc64_batch = 0;                // systems their operand images hold
-  DevBuf<int> tc64_alpha;            // their column scales, zero between updates
+  DevBuf<int> tc_alpha;              // column scales of the tensor-core updates, zero between them
   DevBuf<uint8_t> tc64_images;       // their operand images; a refined workspace lends its tc_images instead
   int residual_pref = 1;             // refinement residual on the tensor cores (baked into graphs)
   DevBuf<int> tc_err;                // set by a tensor-core wait that timed out
@@ -464,6 +464,11 @@ struct Workspace {
   DevBuf<int> hflag;
   std::map<int, cudaGraphExec_t> graphs;  // key: form * 65536 + energies in the batch
   std::map<int, unsigned long long> graph_launches;  // kernel launches per replay
+  cudaError_t alloc_alpha(size_t count) {
+    cudaError_t e = tc_alpha.alloc(count);
+    if (e == cudaSuccess) e = cudaMemset(tc_alpha.p, 0, tc_alpha.n * sizeof(int));
+    return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
+  }
   void drop_graphs() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
@@ -925,7 +930,8 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
   ws.use_tc = ws.fp32 && ctx->use_tensor_cores != 0;
   ws.use_tc64 = ctx->use_tensor_cores != 0;
   if (ws.use_tc) {
-    ws.tc_image_size = tc_image_bytes(n, m, B);
+    ws.tc_image_size = std::max(tc_image_bytes(n, m, B), tc64_image_bytes(n, m, 1));
+    RF_CUDA(ctx, ws.alloc_alpha(size_t(B) * kTcKMax));
     RF_CUDA(ctx, ws.tc_images.alloc(ws.tc_image_size));
     RF_CUDA(ctx, ws.tc_err.alloc(1));
     RF_CUDA(ctx, cudaMemset(ws.tc_err.p, 0, sizeof(int)));
@@ -945,14 +951,13 @@ int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int b
   if (!rc && lu64 && ws.use_tc64) {
     // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); without room
     // for them the updates stay on the CUDA cores
-    const size_t one = tc64_image_bytes(n, m, 1);
-    ws.tc64_batch = ws.use_tc ? ws.batch
-                              : int(std::min<size_t>(size_t(ws.batch), std::max<size_t>(1, (size_t(1) << 30) / one)));
+    const size_t one = tc64_image_bytes(n, m, 1), room = ws.use_tc ? ws.tc_image_size : size_t(1) << 30;
+    ws.tc64_batch = int(std::min<size_t>(size_t(ws.batch), std::max<size_t>(1, room / one)));
+    while (ws.use_tc && ws.tc64_batch > 1 && tc64_image_bytes(n, m, ws.tc64_batch) > room) --ws.tc64_batch;
     const size_t bytes = ws.use_tc ? 0 : tc64_image_bytes(n, m, ws.tc64_batch), na = size_t(ws.tc64_batch) * 32;
-    if (ws.tc64_images.n < bytes || ws.tc64_alpha.n < na) {
+    if (ws.tc64_images.n < bytes || ws.tc_alpha.n < na) {
       ws.drop_graphs();
-      if ((bytes && ws.tc64_images.alloc(bytes) != cudaSuccess) || ws.tc64_alpha.alloc(na) != cudaSuccess ||
-          cudaMemset(ws.tc64_alpha.p, 0, na * sizeof(int)) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+      if ((bytes && ws.tc64_images.alloc(bytes) != cudaSuccess) || ws.alloc_alpha(na) != cudaSuccess) {
         cudaGetLastError();
         ws.use_tc64 = false;
       }
@@ -984,14 +989,15 @@ LuWork lu_work(Workspace& ws, const PanelConfig& pc, bool polls = false) {
     w.linv = ws.linv.p;
     w.pair128 = pc.pair128;
   }
-  if (&pc == &ws.pc64 && ws.use_tc64 && ws.tc64_alpha.p) {
+  if (&pc == &ws.pc64 && ws.use_tc64 && ws.tc_alpha.p) {
     w.tc_images = ws.use_tc ? ws.tc_images.p : ws.tc64_images.p;
     w.tc_image_batch = ws.tc64_batch;
-    w.tc_alpha = ws.tc64_alpha.p;
+    w.tc_alpha = ws.tc_alpha.p;
     if (polls) w.tc_wait_polls = ws.tc_wait_polls;
   }
   if (&pc == &ws.pc32 && ws.use_tc) {
     w.tc_images = ws.tc_images.p;
+    w.tc_alpha = ws.tc_alpha.p;
     w.tc_err = ws.tc_err.p;
     w.tc_wait_polls = ws.tc_wait_polls;
     w.tc_spans = &ws.tc_spans;

@@ -3,19 +3,27 @@
 // with A = L21 (rows below the block) and B = U12 (block rows, trailing
 // columns); K is one 64-column block, or two when the elimination pairs them.
 //
-// Each complex product is formed from real TF32 MMAs with FP32 accumulation in
-// tensor memory, using a two-term split x = hi + lo (hi = tf32(x), lo =
-// tf32(x - hi)) and the three products hi*hi + hi*lo + lo*hi, which keeps the
+// Each complex product is formed from real FP16 MMAs with FP32 accumulation in
+// tensor memory, using a two-term split x = hi + lo (hi = fp16(x), lo =
+// fp16(x - hi)) and the three products hi*hi + hi*lo + lo*hi, which keeps the
 // update at about FP32 accuracy:
 //     Cr += Ar Br + Ai (-Bi)        Ci += Ar Bi + Ai Br
-// The operands are first written by tc_split_* into tile images that are
-// already in the UMMA shared-memory layout (K-major, 128-byte rows, 128-byte
+// FP16 carries the same 11 significant bits as TF32 at twice the rate and half
+// the operand bytes; what it lacks is exponent range, which power-of-two scales
+// give back: column k of A and row k of B are balanced by 2^g_k (so that no
+// column of A is small in every row), each row of A and each column of B is
+// scaled to a largest entry in [2^13, 2^14), and the epilogue takes the scales
+// out again.  Entries more than 2^16 below their row's largest lose relative,
+// not absolute, accuracy.
+// The operands are first written by tc_split_kernel into tile images that are
+// already in the UMMA shared-memory layout (K-major, 64-byte rows, 64-byte
 // swizzle), so the update kernel moves them with plain cp.async.bulk copies
 // completed on mbarriers.  The update runs as one persistent, warp-specialised
 // CTA per SM over 128 x 64 complex tiles (tc_update_persistent_kernel below).
 // Every wait on an mbarrier is bounded; on timeout the kernel records an error
 // flag, ends every role, waits for its copies and MMAs in flight, frees its
 // tensor memory and returns.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "cplx.cuh"
@@ -27,42 +35,39 @@ namespace {
 
 constexpr int BM = kTcBM;         // 128 rows per tile (MMA M)
 constexpr int BN = kTcBN;         // 64 columns per tile (MMA N)
-// Operand rows of kRowBytes bytes with the matching swizzle (128 or 64): with
-// 64-byte rows a K chunk holds KC = 16 TF32 values per row (56 KB of planes),
-// and four chunks are in flight; 128-byte rows (112 KB chunks, two in flight)
-// measured 2% slower with the paired-N MMAs (and faster before them).
+// Operand rows of 64 bytes with the 64-byte swizzle: a K chunk holds KC = 32
+// FP16 values per row (56 KB of planes), and four chunks are in flight.
 constexpr int kRowBytes = 64;
-constexpr int KC = kRowBytes / 4;          // K elements per chunk
-constexpr int A_PLANE = BM * kRowBytes;    // bytes per A plane per chunk (16 KB)
-constexpr int B_PLANE = BN * kRowBytes;    // bytes per B plane per chunk (8 KB)
+constexpr int KC = kRowBytes / 2;          // K elements per chunk
+constexpr int A_PLANE = BM * kRowBytes;    // bytes per A plane per chunk (8 KB)
+constexpr int B_PLANE = BN * kRowBytes;    // bytes per B plane per chunk (4 KB)
 constexpr int A_PLANES = 4;       // re_hi, re_lo, im_hi, im_lo
 // B slots -im_hi, re_hi, im_hi, -im_lo, re_lo, im_lo: each adjacent pair is one 2 BN-row B operand
 constexpr int B_PLANES = 6;
-constexpr int SMEM_OPS = A_PLANES * A_PLANE + B_PLANES * B_PLANE;  // 112 KB
+constexpr int SMEM_OPS = A_PLANES * A_PLANE + B_PLANES * B_PLANE;  // 56 KB
 constexpr long long kWaitLimit = kTcWaitPolls;  // drains of copies and MMAs in flight
 constexpr int kChunks = kTcKMax / KC;  // K chunks per tile image (K up to 128)
 
-__device__ __forceinline__ uint32_t tf32_bits(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
-}
-
-// Byte offset of element (row, k) (k < KC, 4 bytes) in a K-major tile of
-// kRowBytes-byte rows with the matching swizzle: the 16-byte chunk index is
-// XORed with address bits [7, 10) shifted down (row % 8 for 128-byte rows,
-// (row / 2) % 4 for 64-byte rows), the canonical UMMA layouts.
+// Byte offset of element (row, k) (k < KC, 2 bytes) in a K-major tile of 64-byte rows with the 64-byte swizzle: the
+// 16-byte chunk index XOR (row / 2) % 4.
 __device__ __forceinline__ int sw_offset(int row, int k) {
-  if constexpr (kRowBytes == 128) return row * 128 + ((((k >> 2) ^ (row & 7))) << 4) + ((k & 3) << 2);
-  return row * 64 + ((((k >> 2) ^ ((row >> 1) & 3))) << 4) + ((k & 3) << 2);
+  return row * 64 + ((((k >> 3) ^ ((row >> 1) & 3))) << 4) + ((k & 7) << 1);
 }
 
-__device__ __forceinline__ void split4(float2 v, uint32_t out[4]) {
-  const uint32_t rh = tf32_bits(v.x), ih = tf32_bits(v.y);
-  out[0] = rh;
-  out[1] = tf32_bits(v.x - __uint_as_float(rh));
-  out[2] = ih;
-  out[3] = tf32_bits(v.y - __uint_as_float(ih));
+// 2^e, e clamped to the normal range
+__device__ __forceinline__ float pow2(int e) { return __int_as_float(min(max(e + 127, 1), 254) << 23); }
+// v 2^x for |x| beyond what one factor holds
+__device__ __forceinline__ float scaled(float v, int x) { return v * pow2(x >> 1) * pow2(x - (x >> 1)); }
+// the shift that brings values below 2^e below 2^14, within what the epilogue's factor 2^-shift can undo
+__device__ __forceinline__ int shift_of(int e) { return min(max(14 - e, -112), 112); }
+// larger exponent field of the two parts (0: zero or denormal)
+__device__ __forceinline__ int field_of(float2 v) {
+  return int(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu) >> 23);
+}
+// the FP16 terms of a scaled value
+__device__ __forceinline__ void split2(float x, __half& hi, __half& lo) {
+  hi = __float2half_rn(x);
+  lo = __float2half_rn(x - __half2float(hi));
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -71,21 +76,19 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint64_t umma_desc_sw(uint32_t saddr) {
   // start address >> 4 (14 bits), LBO = 1 (unused for swizzled K-major), SBO = 8 rows (the 8-row groups),
-  // descriptor version 1, base offset 0, layout type 2 = 128-byte swizzle / 4 = 64-byte swizzle.
-  constexpr uint64_t kLayout = kRowBytes == 128 ? 2 : 4;
+  // descriptor version 1, base offset 0, layout type 4 = 64-byte swizzle.
   return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(1) << 16) | (uint64_t((8 * kRowBytes) >> 4) << 32) |
-         (uint64_t(1) << 46) | (kLayout << 61);
+         (uint64_t(1) << 46) | (uint64_t(4) << 61);
 }
 
-// kind::tf32, D = F32, A = B = TF32, both K-major, M = BM, N = 2 BN: one A plane against two adjacent B
+// kind::f16, D = F32, A = B = F16, both K-major, M = BM, N = 2 BN: one A plane against two adjacent B
 // slots, into the adjacent accumulators [Cr | Ci].
-constexpr uint32_t kIdesc =
-    (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t((2 * BN) >> 3) << 17) | (uint32_t(BM >> 4) << 24);
+constexpr uint32_t kIdesc = (1u << 4) | (uint32_t((2 * BN) >> 3) << 17) | (uint32_t(BM >> 4) << 24);
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate));
 }
 
@@ -112,68 +115,184 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// operand images: A[b][bm][chunk][plane] (8 KB), B[b][bn][chunk][plane] (4 KB), chunks of KC = 16
+// scales and operand images: A[b][bm][chunk][plane] (8 KB), B[b][bn][chunk][plane] (4 KB), chunks of KC = 32
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) tc_split_a_kernel(BatchLayout lay, int k, int kb, const float2* __restrict__ M,
-                                                         uint8_t* __restrict__ img, int nbm) {
-  // The tile is read down the columns (coalesced in the column-major matrix),
-  // turned around in shared memory, and written as 16-byte chunks of the
-  // swizzled K-major rows, so that every warp stores 512 contiguous bytes.
-  constexpr int TS = BM + 1;  // padded row of the transposed tile
-  __shared__ float2 T[KC * TS];
-  const int nch = (kb + KC - 1) / KC;  // the grid holds nch chunks per row tile
-  const int bm = blockIdx.x / nch, chunk = blockIdx.x % nch, b = blockIdx.y;
-  const int n = lay.n;
-  const int r0 = k + kb + bm * BM;
-  const float2* Mb = M + size_t(b) * lay.stride;
-  for (int e = threadIdx.x; e < BM * KC; e += blockDim.x) {
-    const int r = e % BM, kk = e / BM;
-    const int kcol = chunk * KC + kk;
-    T[kk * TS + r] = (r0 + r < n && kcol < kb) ? Mb[size_t(r0 + r) + size_t(lay.lda) * (k + kcol)] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  uint8_t* base = img + ((size_t(b) * nbm + bm) * kChunks + chunk) * size_t(A_PLANES) * A_PLANE;
-  for (int e = threadIdx.x; e < BM * (KC / 4); e += blockDim.x) {
-    const int k4 = e % (KC / 4), r = e / (KC / 4);
-    uint32_t q[4][4];
+// alpha[b][k] = 256 + max over the rows of (exponent of A[row, k] - exponent of the row's largest entry), 0 where column k
+// is zero: g_k = 256 - alpha.  The table is zero before and is cleared again by the update kernel.
+template <int kK>  // kb <= kK, a multiple of 32
+__global__ void __launch_bounds__(BM) tc_scale_kernel(BatchLayout lay, int k, int kb, const float2* __restrict__ M,
+                                                      int* __restrict__ alpha) {
+  __shared__ int cmax[kTcKMax];
+  const int b = blockIdx.y, lane = threadIdx.x & 31, row = k + kb + blockIdx.x * BM + int(threadIdx.x);
+  cmax[threadIdx.x] = 0;
+  const float2* A = M + size_t(b) * lay.stride + size_t(row) + size_t(lay.lda) * k;
+  uint32_t f[kK / 4];  // exponent fields, four to a word
+  int top = 0;
+#pragma unroll
+  for (int q = 0; q < kK / 4; ++q) {
+    f[q] = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      uint32_t sv[4];
-      split4(T[(4 * k4 + i) * TS + r], sv);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) q[p][i] = sv[p];
+      const int kk = 4 * q + i, v = row < lay.n && kk < kb ? field_of(A[size_t(lay.lda) * kk]) : 0;
+      f[q] |= uint32_t(v) << (8 * i);
+      top = max(top, v);
     }
-    const int off = sw_offset(r, 4 * k4);
+  }
+  __syncthreads();
 #pragma unroll
-    for (int p = 0; p < 4; ++p)
-      *reinterpret_cast<uint4*>(base + size_t(p) * A_PLANE + off) = make_uint4(q[p][0], q[p][1], q[p][2], q[p][3]);
+  for (int q = 0; q < kK / 32; ++q) {
+    int mine = 0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int v = int(f[8 * q + i / 4] >> (8 * (i % 4))) & 255;
+      const int m = __reduce_max_sync(0xffffffffu, v > 0 && top < 255 ? v - top + 256 : 0);
+      if (lane == i) mine = m;
+    }
+    if (mine > 0) atomicMax(&cmax[32 * q + lane], mine);
+  }
+  __syncthreads();
+  if (cmax[threadIdx.x] > 0) atomicMax(alpha + b * kTcKMax + threadIdx.x, cmax[threadIdx.x]);
+}
+static_assert(BM == kTcKMax, "one thread a column of the table");
+
+__device__ __forceinline__ void load_balance(const int* alpha, int* gk) {
+  if (threadIdx.x < kTcKMax) {
+    const int a = alpha[threadIdx.x];
+    gk[threadIdx.x] = a > 0 ? 256 - a : 0;
+  }
+  __syncthreads();
+}
+
+// Operand images: blocks x < nbm take a row tile of A, the others a column tile of B.
+__device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int kb, const float2* __restrict__ M,
+                                             const int* gk, uint8_t* __restrict__ img, float* __restrict__ rscale,
+                                             int nbm, uint8_t* smem) {
+  // The tile is read down the columns (coalesced in the column-major matrix),
+  // turned around in shared memory, and written as 16-byte chunks of the
+  // swizzled K-major rows.
+  constexpr int TS = BM + 1;  // padded row of the transposed tile
+  float2* T = reinterpret_cast<float2*>(smem);
+  int(*rowe)[BM] = reinterpret_cast<int(*)[BM]>(smem + KC * TS * sizeof(float2));
+  const int nch = (kb + KC - 1) / KC;
+  const int bm = blockIdx.x, b = blockIdx.y;
+  const int n = lay.n, r0 = k + kb + bm * BM;
+  const float2* Mb = M + size_t(b) * lay.stride + size_t(lay.lda) * k;
+  {
+    const int r = threadIdx.x & (BM - 1), h = threadIdx.x / BM;
+    int e = -(1 << 20);
+    if (r0 + r < n)
+#pragma unroll 8
+      for (int kk = h; kk < kb; kk += 2) {
+        const int f = field_of(Mb[size_t(r0 + r) + size_t(lay.lda) * kk]);
+        if (f > 0) e = max(e, f - 126 + gk[kk]);
+      }
+    rowe[h][r] = e;
+    __syncthreads();
+    if (h == 0) {
+      e = max(e, rowe[1][r]);
+      if (e == -(1 << 20)) e = 0;
+      e = shift_of(e);  // |A| 2^g < 2^e along the row
+      rowe[0][r] = e;
+      rscale[(size_t(b) * nbm + bm) * BM + r] = pow2(-e);
+    }
+    __syncthreads();
+  }
+  for (int chunk = 0; chunk < nch; ++chunk) {
+    for (int e = threadIdx.x; e < BM * KC; e += 256) {
+      const int r = e % BM, kk = e / BM, kcol = chunk * KC + kk;
+      float2 v = make_float2(0.f, 0.f);
+      if (r0 + r < n && kcol < kb) {
+        v = Mb[size_t(r0 + r) + size_t(lay.lda) * kcol];
+        const int x = rowe[0][r] + gk[kcol];
+        v = make_float2(scaled(v.x, x), scaled(v.y, x));
+      }
+      T[kk * TS + r] = v;
+    }
+    __syncthreads();
+    uint8_t* base = img + ((size_t(b) * nbm + bm) * kChunks + chunk) * size_t(A_PLANES) * A_PLANE;
+    for (int e = threadIdx.x; e < BM * (KC / 8); e += 256) {
+      const int k8 = e % (KC / 8), r = e / (KC / 8);
+      __align__(16) __half q[A_PLANES][8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 v = T[(8 * k8 + i) * TS + r];
+        split2(v.x, q[0][i], q[1][i]);
+        split2(v.y, q[2][i], q[3][i]);
+      }
+      const int off = sw_offset(r, 8 * k8);
+#pragma unroll
+      for (int p = 0; p < A_PLANES; ++p)
+        *reinterpret_cast<uint4*>(base + size_t(p) * A_PLANE + off) = *reinterpret_cast<const uint4*>(q[p]);
+    }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(256) tc_split_b_kernel(BatchLayout lay, int k, int kb, int col_end,
-                                                         const float2* __restrict__ M, uint8_t* __restrict__ img,
-                                                         int nbn) {
-  const int nch = (kb + KC - 1) / KC;  // the grid holds nch chunks per column tile
-  const int bn = blockIdx.x / nch, chunk = blockIdx.x % nch, b = blockIdx.y;
-  const int c0 = k + kb + bn * BN;
-  const float2* Mb = M + size_t(b) * lay.stride;
-  uint8_t* base = img + ((size_t(b) * nbn + bn) * kChunks + chunk) * size_t(B_PLANES) * B_PLANE;
-  for (int e = threadIdx.x; e < BN * KC; e += blockDim.x) {
-    const int kk = e % KC, c = e / KC;
-    const int krow = chunk * KC + kk;
-    float2 v = make_float2(0.f, 0.f);
-    if (c0 + c < col_end && krow < kb) v = Mb[size_t(k + krow) + size_t(lay.lda) * (c0 + c)];
-    uint32_t s[4];
-    split4(v, s);
-    const int off = sw_offset(c, kk);
-    auto put = [&](int slot, uint32_t x) { *reinterpret_cast<uint32_t*>(base + size_t(slot) * B_PLANE + off) = x; };
-    put(0, s[2] ^ 0x80000000u);  // -im_hi
-    put(1, s[0]);                // re_hi
-    put(2, s[2]);                // im_hi
-    put(3, s[3] ^ 0x80000000u);  // -im_lo
-    put(4, s[1]);                // re_lo
-    put(5, s[3]);                // im_lo
+__device__ __forceinline__ void split_b_tile(const BatchLayout& lay, int bn, int k, int kb, int col_end,
+                                             const float2* __restrict__ M, const int* gk, uint8_t* __restrict__ img,
+                                             float* __restrict__ cscale, int nbn, uint8_t* smem) {
+  int* cole = reinterpret_cast<int*>(smem);
+  const int b = blockIdx.y, c0 = k + kb + bn * BN;
+  const float2* Mb = M + size_t(b) * lay.stride + size_t(k);
+  // column exponents: one warp a column, lanes down its rows
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int c = wid; c < BN; c += 8) {
+    int e = -(1 << 20);
+    if (c0 + c < col_end)
+      for (int kk = lane; kk < kb; kk += 32) {
+        const int f = field_of(Mb[size_t(kk) + size_t(lay.lda) * (c0 + c)]);
+        if (f > 0) e = max(e, f - 126 - gk[kk]);
+      }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (e == -(1 << 20)) e = 0;
+    if (lane == 0) {
+      e = shift_of(e);  // |B| 2^-g < 2^e along the column
+      cole[c] = e;
+      cscale[(size_t(b) * nbn + bn) * BN + c] = pow2(-e);
+    }
   }
+  __syncthreads();
+  const int nch = (kb + KC - 1) / KC;
+  // a thread takes eight consecutive rows of a column: one 16-byte chunk of each slot
+  for (int e = threadIdx.x; e < BN * nch * (KC / 8); e += 256) {
+    const int k8 = e % (nch * (KC / 8)), c = e / (nch * (KC / 8)), chunk = k8 / (KC / 8), kin = 8 * (k8 % (KC / 8));
+    __align__(16) __half q[B_PLANES][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int krow = 8 * k8 + i;
+      float2 v = make_float2(0.f, 0.f);
+      if (c0 + c < col_end && krow < kb) {
+        v = Mb[size_t(krow) + size_t(lay.lda) * (c0 + c)];
+        const int x = cole[c] - gk[krow];
+        v = make_float2(scaled(v.x, x), scaled(v.y, x));
+      }
+      __half rh, rl, ih, il;
+      split2(v.x, rh, rl);
+      split2(v.y, ih, il);
+      q[0][i] = __hneg(ih);
+      q[1][i] = rh;
+      q[2][i] = ih;
+      q[3][i] = __hneg(il);
+      q[4][i] = rl;
+      q[5][i] = il;
+    }
+    uint8_t* base = img + ((size_t(b) * nbn + bn) * kChunks + chunk) * size_t(B_PLANES) * B_PLANE + sw_offset(c, kin);
+#pragma unroll
+    for (int p = 0; p < B_PLANES; ++p)
+      *reinterpret_cast<uint4*>(base + size_t(p) * B_PLANE) = *reinterpret_cast<const uint4*>(q[p]);
+  }
+}
+
+__global__ void __launch_bounds__(256) tc_split_kernel(BatchLayout lay, int k, int kb, int col_end,
+                                                       const float2* __restrict__ M, const int* __restrict__ alpha,
+                                                       uint8_t* __restrict__ aimg, uint8_t* __restrict__ bimg,
+                                                       float* __restrict__ rscale, float* __restrict__ cscale, int nbm,
+                                                       int nbm_all, int nbn_all) {
+  __shared__ __align__(16) uint8_t smem[KC * (BM + 1) * sizeof(float2) + 2 * BM * sizeof(int)];
+  __shared__ int gk[kTcKMax];
+  load_balance(alpha + blockIdx.y * kTcKMax, gk);
+  if (int(blockIdx.x) < nbm) split_a_tile(lay, k, kb, M, gk, aimg, rscale, nbm_all, smem);
+  else split_b_tile(lay, int(blockIdx.x) - nbm, k, kb, col_end, M, gk, bimg, cscale, nbn_all, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -237,8 +356,9 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 
 __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
     BatchLayout lay, int k, int kb, int col_end, float2* __restrict__ M, const uint8_t* __restrict__ aimg,
-    const uint8_t* __restrict__ bimg, int nbm_all, int nbn_all, int nbm, int nbn, int batch, int* __restrict__ err_flag,
-    const int* skip, long long polls) {
+    const uint8_t* __restrict__ bimg, const float* __restrict__ rscale, const float* __restrict__ cscale, int nbm_all,
+    int nbn_all, int nbm, int nbn, int batch, int* __restrict__ alpha, int* __restrict__ err_flag, const int* skip,
+    long long polls) {
   extern __shared__ uint8_t smraw[];
   const uint32_t raw = smem_u32(smraw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -254,6 +374,8 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
   const int per_matrix = nbm * nbn;
   const int total = per_matrix * batch;  // the host keeps this below 2^31
   const int nchunks = (kb + KC - 1) / KC;  // 1 .. kChunks
+  // the balance table, read by the split kernels before: zero again for the next update
+  for (int i = blockIdx.x * kPThreads + tid; i < batch * kTcKMax; i += gridDim.x * kPThreads) alpha[i] = 0;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -347,7 +469,7 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
           *(volatile int*)consumed = int(c + 1);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t sA = sbase + uint32_t(st) * SMEM_OPS, sB = sA + A_PLANES * A_PLANE;
-          for (int ks = 0; ks < KC / 8; ++ks) {
+          for (int ks = 0; ks < KC / 16; ++ks) {
             const uint32_t koff = uint32_t(ks * 32);
             auto ad = [&](int p) { return umma_desc_sw(sA + p * A_PLANE + koff); };
             auto bd = [&](int p) { return umma_desc_sw(sB + p * B_PLANE + koff); };
@@ -356,12 +478,12 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
             //            + Ai hi [-Bi hi | Br hi] + Ai hi [-Bi lo | Br lo] + Ai lo [-Bi hi | Br hi],
             // i.e. Cr += Ar Br + Ai (-Bi), Ci += Ar Bi + Ai Br, each hi*hi + hi*lo + lo*hi
             (void)tmem_i;
-            mma_tf32(tmem_r, ad(0), bd(1), acc0);
-            mma_tf32(tmem_r, ad(0), bd(4), 1u);
-            mma_tf32(tmem_r, ad(1), bd(1), 1u);
-            mma_tf32(tmem_r, ad(2), bd(0), 1u);
-            mma_tf32(tmem_r, ad(2), bd(3), 1u);
-            mma_tf32(tmem_r, ad(3), bd(0), 1u);
+            mma_f16(tmem_r, ad(0), bd(1), acc0);
+            mma_f16(tmem_r, ad(0), bd(4), 1u);
+            mma_f16(tmem_r, ad(1), bd(1), 1u);
+            mma_f16(tmem_r, ad(2), bd(0), 1u);
+            mma_f16(tmem_r, ad(2), bd(3), 1u);
+            mma_f16(tmem_r, ad(3), bd(0), 1u);
           }
           issued = true;
           umma_commit(bar(kBarEmpty + st));  // the stage is free once these MMAs have read it
@@ -403,8 +525,10 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
       const int row = r0 + quarter * 32 + lane;
       const bool row_ok = row < n;
       const int ld = lay.lda;  // column offsets within a tile stay far below 2^31 elements
+      const float rs = rscale[(size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane];
+      const float* cs = cscale + (size_t(b) * nbn_all + bn) * BN;
       float2* crow = M + size_t(b) * lay.stride + size_t(row) + size_t(lay.lda) * size_t(c0);
-      // C of 16 columns at a time, the next part loaded while this one is stored
+      // C of 16 columns at a time, an entry of the next part loaded as soon as this one's is used
       float2 cn[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j)
@@ -415,16 +539,6 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
       const uint32_t tmem_r = tmem + uint32_t(g * 128) + lane_off, tmem_i = tmem_r + 64;
 #pragma unroll 1
       for (int part = 0; part < BN / 16; ++part) {
-        float2 cc[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) cc[j] = cn[j];
-        if (part + 1 < BN / 16) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int col = c0 + (part + 1) * 16 + j;
-            cn[j] = (row_ok && col < col_end) ? crow[((part + 1) * 16 + j) * ld] : make_float2(0.f, 0.f);
-          }
-        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t cr[8], ci[8];
@@ -437,17 +551,18 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
                          "=r"(ci[7])
                        : "r"(tmem_i + uint32_t(part * 16 + h * 8)));
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (row_ok) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = c0 + part * 16 + h * 8 + j;
-              if (col < col_end) {
-                float2 v = cc[h * 8 + j];
-                v.x -= __uint_as_float(cr[j]);
-                v.y -= __uint_as_float(ci[j]);
-                crow[(part * 16 + h * 8 + j) * ld] = v;
-              }
+          for (int j = 0; j < 8; ++j) {
+            const int i = h * 8 + j, off = part * 16 + i;
+            if (row_ok && c0 + off < col_end) {
+              float2 v = cn[i];
+              const float sc = rs * cs[off];
+              v.x = fmaf(-__uint_as_float(cr[j]), sc, v.x);
+              v.y = fmaf(-__uint_as_float(ci[j]), sc, v.y);
+              crow[off * ld] = v;
             }
+            if (part + 1 < BN / 16)
+              cn[i] = (row_ok && c0 + off + 16 < col_end) ? crow[(off + 16) * ld] : make_float2(0.f, 0.f);
           }
         }
       }
@@ -463,24 +578,44 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-size_t tc_image_bytes(int n, int m, int batch) {
-  const int nbm = (n + BM - 1) / BM, nbn = (n + m + BN - 1) / BN;
-  return size_t(batch) * kChunks * (size_t(nbm) * A_PLANES * A_PLANE + size_t(nbn) * B_PLANES * B_PLANE);
+namespace {
+struct TcImages {
+  int nbm, nbn;
+  size_t a, b, r, c, total;  // byte offsets of the A and B images, the row and column scales
+};
+TcImages tc_images(int n, int m, int batch) {
+  TcImages v;
+  v.nbm = (n + BM - 1) / BM;
+  v.nbn = (n + m + BN - 1) / BN;
+  v.a = 0;
+  v.b = v.a + size_t(batch) * v.nbm * kChunks * A_PLANES * A_PLANE;
+  v.r = v.b + size_t(batch) * v.nbn * kChunks * B_PLANES * B_PLANE;
+  v.c = v.r + size_t(batch) * v.nbm * BM * sizeof(float);
+  v.total = v.c + size_t(batch) * v.nbn * BN * sizeof(float);
+  return v;
 }
+}  // namespace
+
+size_t tc_image_bytes(int n, int m, int batch) { return tc_images(n, m, batch).total; }
 
 void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int col_end, float2* M, uint8_t* images,
-                        int* err_flag, const int* skip, long long wait_polls, KernelSpans* spans, cudaStream_t s) {
+                        int* alpha, int* err_flag, const int* skip, long long wait_polls, KernelSpans* spans,
+                        cudaStream_t s) {
   const int rows = lay.n - (k + kb), cols = col_end - (k + kb);
   if (rows <= 0 || cols <= 0 || kb <= 0) return;
-  const int nbm_all = (lay.n + BM - 1) / BM, nbn_all = (lay.n + lay.m + BN - 1) / BN;
-  uint8_t* aimg = images;
-  uint8_t* bimg = images + size_t(batch) * kChunks * size_t(nbm_all) * A_PLANES * A_PLANE;
+  const TcImages im = tc_images(lay.n, lay.m, batch);
+  uint8_t *aimg = images + im.a, *bimg = images + im.b;
+  float *rscale = reinterpret_cast<float*>(images + im.r), *cscale = reinterpret_cast<float*>(images + im.c);
+  const int nbm_all = im.nbm, nbn_all = im.nbn;
   const int nbm = (rows + BM - 1) / BM, nbn = (cols + BN - 1) / BN;
+  const dim3 sgrid{unsigned(nbm), unsigned(batch)};
   count_launch();
-  const int nch = (kb + KC - 1) / KC;
-  tc_split_a_kernel<<<dim3(unsigned(nch * nbm), unsigned(batch)), 256, 0, s>>>(lay, k, kb, M, aimg, nbm_all);
+  if (kb <= 32) tc_scale_kernel<32><<<sgrid, BM, 0, s>>>(lay, k, kb, M, alpha);
+  else if (kb <= 64) tc_scale_kernel<64><<<sgrid, BM, 0, s>>>(lay, k, kb, M, alpha);
+  else tc_scale_kernel<kTcKMax><<<sgrid, BM, 0, s>>>(lay, k, kb, M, alpha);
   count_launch();
-  tc_split_b_kernel<<<dim3(unsigned(nch * nbn), unsigned(batch)), 256, 0, s>>>(lay, k, kb, col_end, M, bimg, nbn_all);
+  tc_split_kernel<<<dim3(unsigned(nbm + nbn), unsigned(batch)), 256, 0, s>>>(lay, k, kb, col_end, M, alpha, aimg, bimg,
+                                                                            rscale, cscale, nbm, nbm_all, nbn_all);
   const int sms = current_sm_count();
   ensure_smem_limit(reinterpret_cast<const void*>(tc_update_persistent_kernel), size_t(kPSmem));
   const long long tiles = (long long)nbm * nbn * batch;
@@ -497,8 +632,8 @@ void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int co
     cudaEventRecord(e0, s);
   }
   count_launch();
-  tc_update_persistent_kernel<<<grid, kPThreads, kPSmem, s>>>(lay, k, kb, col_end, M, aimg, bimg, nbm_all, nbn_all,
-                                                              nbm, nbn, batch, err_flag, skip,
+  tc_update_persistent_kernel<<<grid, kPThreads, kPSmem, s>>>(lay, k, kb, col_end, M, aimg, bimg, rscale, cscale, nbm_all,
+                                                              nbn_all, nbm, nbn, batch, alpha, err_flag, skip,
                                                               wait_polls > 0 ? wait_polls : kTcWaitPolls);
   if (prof) {
     cudaEventRecord(e1, s);
