@@ -202,9 +202,16 @@ __device__ __forceinline__ float4 dfc_sub(float4 a, float4 b) {
 // ---------------------------------------------------------------------------
 // Build kernel: CTA = (column atom j, chunk of kBuildRowAtoms row atoms, energy).
 // ---------------------------------------------------------------------------
+// The parity form (below) serves one spin channel without a spin selector up to this L; beyond it its table would not
+// leave room for the small-d tables.
+constexpr int kParityMaxL = 5;
+
+// its entries (l2, m2 - m1), |m2 - m1| <= L + l2, of one pair: entry l2 (2L + l2) + (m2 - m1) + L + l2
+__host__ __device__ constexpr int ept_per_pair(int L) { return (L + 1) * (3 * L + 1); }
+
 struct BuildSmem {
   // offsets in doubles from the dynamic smem base
-  int tcol0, tcol1, colinfo, rowinfo, pref, eph, g, dsm, clm, flag;
+  int tcol0, tcol1, colinfo, rowinfo, pref, eph, g, dsm, clm, flag, ept;
   int total_bytes;
 };
 
@@ -219,11 +226,16 @@ __host__ __device__ inline BuildSmem build_smem_layout(int L, int nsp, int ds) {
   b.colinfo = o; o += 2 * ncol_max;            // int4 per column (as 2 doubles)
   b.rowinfo = o; o += 2 * RA * ncol_max;       // int4 per row
   b.pref = o; o += 2 * RA * nsp;
-  b.eph = o; o += 2 * RA * (4 * L + 1);
   b.g = o; o += 2 * RA * nsp * L1 * L1 * L1;
   b.dsm = o; o += RA * ds;
-  b.clm = o; o += 2 * RA * nsp * (L + 2) * L1;
   b.flag = o; o += RA;                          // one int per pair (stored in a double slot)
+  b.clm = o;
+  b.eph = o + 2 * RA * nsp * (L + 2) * L1;
+  // the phases times -t of the parity form take the place of both (the Hankel tables are spent by then, and it reads the
+  // phases from the plan)
+  b.ept = o;
+  const int both = 2 * RA * nsp * (L + 2) * L1 + 2 * RA * (4 * L + 1), ept = nsp == 1 && L <= kParityMaxL ? 2 * RA * ept_per_pair(L) : 0;
+  o += both > ept ? both : ept;
   b.total_bytes = o * int(sizeof(double));
   return b;
 }
@@ -468,7 +480,8 @@ __global__ void __launch_bounds__(256) build_system_kernel(PlanDev P, const doub
     else dsm[t] = P.pair_dsmall[src];
   }
   // ---- per pair: azimuth phases e^{i m (phi - pi)}, m in [-2L, 2L] (resident, from the plan) ----
-  for (int t = tid; t < RA * (4 * L + 1); t += nthr) {
+  const bool parity = nsp == 1 && P.ispin == 0 && L <= kParityMaxL;
+  for (int t = parity ? RA * (4 * L + 1) : tid; t < RA * (4 * L + 1); t += nthr) {
     const int p = t / (4 * L + 1), q = t % (4 * L + 1);
     const size_t src = (size_t(j) + size_t(N) * (i0 + p)) * (4 * L + 1) + q;
     if constexpr (kMode == 1) reinterpret_cast<float4*>(eph)[t] = P.pair_eph_df[src];
@@ -606,6 +619,103 @@ __global__ void __launch_bounds__(256) build_system_kernel(PlanDev P, const doub
     }
     return dfc_mul(eph4[p * (4 * L + 1) + (m2 - m1 + 2 * L)], make_float4(sx.hi, sy.hi, sx.lo, sy.lo));
   };
+  if (parity) {
+    // Parity form (t depends on l alone): with d_{-m,-m'} = (-1)^{m - m'} d_{m,m'} of the small-d tables, the mu sum S of
+    // element (l1 m1, l2 m2) is (-1)^{m1 + m2} that of (l1 -m1, l2 -m2), so one sum serves the columns m2 and -m2; and
+    // e^{i (m2 - m1)(phi - pi)} (-t_l2) is formed once per (pair, m2 - m1, l2).  Per element 82 + 44 FP32 operations of
+    // double-float arithmetic (8 + 4 FP64 ones) at L = 3 instead of 132 + 88 (13 + 8).
+    double2* ept = reinterpret_cast<double2*>(sm + lay_s.ept);
+    float4* ept4 = reinterpret_cast<float4*>(ept);
+    auto phase_at = [&](int p, int dm) { return (size_t(j) + size_t(N) * (i0 + p)) * (4 * L + 1) + (dm + 2 * L); };
+    const int nl = P.atom_lmax[j] + 1;  // l2 of the columns
+    const int eps = ept_per_pair(L);
+    for (int t = tid; t < RA * eps; t += nthr) {
+      const int p = t / eps;
+      int l2 = 0, dm = t - p * eps;
+      while (dm > 2 * (L + l2)) dm -= 2 * (L + l2++) + 1;
+      dm -= L + l2;
+      if (l2 >= nl) continue;
+      if constexpr (kMode == 1) {
+        ept4[t] = dfc_neg(dfc_mul(P.pair_eph_df[phase_at(p, dm)], reinterpret_cast<const float4*>(tcol0)[l2 * l2]));
+      } else if constexpr (kMode == 0) {
+        ept[t] = cneg(cmul(P.pair_eph[phase_at(p, dm)], tcol0[l2 * l2]));
+      } else {
+        ept[t] = P.pair_eph[phase_at(p, dm)];
+      }
+    }
+    __syncthreads();
+    const int ncolh = nl * (nl + 1) / 2, total = nrow * ncolh;  // columns (l2, m2 >= 0)
+    auto advance = [&](int& v, int& cc) {
+      v += nthr;
+      while (v >= nrow) {
+        v -= nrow;
+        ++cc;
+      }
+    };
+    for (int idx = tid, v = tid % nrow, ch = tid / nrow; idx < total; idx += nthr, advance(v, ch)) {
+      const int4 ri = rowinfo[v];
+      int l2 = 0, m2 = ch;
+      while (m2 > l2) m2 -= ++l2;  // ch = l2 (l2 + 1) / 2 + m2
+      const int rp = ri.x >> 2, l1 = ri.y, m1 = ri.z;
+      const int r = r0 + ri.w, c = cj0 + l2 * l2 + l2 + m2;
+      const bool same = i0 + rp == j, on = !same && flag[rp];
+      const int w1 = 2 * l1 + 1, w2 = 2 * l2 + 1, mn = min(l1, l2);
+      const int tbo = rp * P.ds + dpd + lblock_offset(l1) + (m1 + l1), tfo = rp * P.ds + lblock_offset(l2) + (m2 + l2) * w2 + l2;
+      const int go = rp * gsz + l1 + L1 * l2;
+      // both signs of m2
+      auto put = [&](int rr, int cc, int dm, auto sum) {
+        const size_t ai = base + size_t(rr) + size_t(lay.lda) * cc;
+        const int bc = cc - cj0;
+        if constexpr (kMode == 1) {
+          float4 x = on ? dfc_mul(ept4[rp * eps + l2 * (2 * L + l2) + dm + L + l2], sum) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (rr == cc) df_add(x.x, x.z, 1.f, 0.f);
+          reinterpret_cast<float4*>(M64)[ai] = x;
+          M32[ai] = make_float2(x.x, x.y);
+          if (absorber_col) {
+            const float4 gcol = on ? dfc_mul(P.pair_eph_df[phase_at(rp, dm)], sum) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const size_t bi = base + size_t(rr) + size_t(lay.lda) * (size_t(lay.n) + bcol_j + bc);
+            reinterpret_cast<float4*>(M64)[bi] = gcol;
+            M32[bi] = make_float2(gcol.x, gcol.y);
+          }
+        } else {
+          double2 x = on ? cmul(ept[rp * eps + l2 * (2 * L + l2) + dm + L + l2], sum) : make_double2(0.0, 0.0);
+          if (kMode == 0 && rr == cc) x.x += 1.0;
+          M64[ai] = x;
+          if (kMode == 0 && absorber_col)
+            M64[base + size_t(rr) + size_t(lay.lda) * (size_t(lay.n) + bcol_j + bc)] =
+                on ? cmul(P.pair_eph[phase_at(rp, dm)], sum) : make_double2(0.0, 0.0);
+        }
+      };
+      const bool flip = (m1 + m2) & 1;
+      if constexpr (kMode == 1) {
+        df sx{0.f, 0.f}, sy{0.f, 0.f};
+        if (on)
+          for (int mu = -mn; mu <= mn; ++mu) {
+            const float2 b = dsm2[tbo + (mu + l1) * w1], f = dsm2[tfo + mu];
+            float dh, dl;
+            df_prod(b.x, b.y, f.x, f.y, dh, dl);
+            const float4 gv = gtab4[go + L1 * L1 * (mu < 0 ? -mu : mu)];
+            df_mac(sx, dh, dl, gv.x, gv.z);
+            df_mac(sy, dh, dl, gv.y, gv.w);
+          }
+        const float4 sum = make_float4(sx.hi, sy.hi, sx.lo, sy.lo);
+        put(r, c, m2 - m1, sum);
+        if (m2 > 0) put(r - 2 * m1, c - 2 * m2, m1 - m2, flip ? dfc_neg(sum) : sum);
+      } else {
+        double2 sum = make_double2(0.0, 0.0);
+        if (on)
+          for (int mu = -mn; mu <= mn; ++mu) {
+            const double dd = dsm[tbo + (mu + l1) * w1] * dsm[tfo + mu];
+            const double2 gv = gtab[go + L1 * L1 * (mu < 0 ? -mu : mu)];
+            sum.x = fma(dd, gv.x, sum.x);
+            sum.y = fma(dd, gv.y, sum.y);
+          }
+        put(r, c, m2 - m1, sum);
+        if (m2 > 0) put(r - 2 * m1, c - 2 * m2, m1 - m2, flip ? cneg(sum) : sum);
+      }
+    }
+    return;
+  }
   const int total = nrow * ncol;
   // element idx is (row v, column cc) with idx = v + nrow cc; (v, cc) follow idx without a division
   auto advance = [&](int& v, int& cc) {
