@@ -360,7 +360,7 @@ int refeff_fms_autotune_multi(refeff_fms_context* ctx, int n_plans, refeff_fms_p
                               const refeff_fms_energy_points* points, refeff_fms_form form, int sample_energies,
                               const char* cache_path, refeff_fms_tuning* out);
 /* Per-plan choices of the FP32 elimination: inner_width 0 (by size: two-level
- * from n = 512 with 16-column inner panels first), 16 or 32 (two-level with
+ * from n = 512, with inner panels of 32 columns up to n = 4608 and of 16 beyond), 16 or 32 (two-level with
  * that inner panel width first, from n = 128) or 1 (single-level panels);
  * paired_blocks -1 (the context's REFEFF_FMS_OPT_PAIRED_BLOCKS), 0 or 1.
  * Applies from the plan's next solve. */

@@ -855,13 +855,13 @@ PanelConfig choose_panel(int n, int inner_pref) {
   pc.cluster = 0;
   const bool forced = inner_pref == 16 || inner_pref == 32;
   if (sizeof(T) == 4 && ((inner_pref == 0 && n >= 512) || (forced && n >= 128))) {
-    // two-level: 64-column blocks of 16- or 32-column cluster panels.  16 columns
-    // halve the shared memory of a panel, and with the row bookkeeping in global
-    // scratch a 4-CTA panel takes 72 KB per CTA, three CTAs per SM: about three
-    // times as many panels (energies) are factored at once as with 32 columns
-    // and the bookkeeping in shared memory.  The panel's column chain, not its
-    // arithmetic, bounds it (measured at n = 2256: elimination 103.8 -> 90.8 ms).
-    const int order[2] = {inner_pref == 32 ? 32 : 16, inner_pref == 32 ? 16 : 32};
+    // two-level: 64-column blocks of 16- or 32-column cluster panels.  A 32-column panel of the register kernel takes a
+    // row a thread, so it serves 512 rows a CTA, and halves the launches between the panels (their row solves, moves and
+    // in-block updates); 16 columns serve 1024 rows a CTA.  Measured, 16 against 32 columns: n = 688 x 60 5.83 / 5.37 ms,
+    // n = 1392 x 60 14.1 / 13.2 ms, n = 2256 x 10 18.0 / 16.7 ms, n = 2256 x 100 58.7 / 58.6 ms, n = 4112 x 24
+    // 64.6 / 62.2 ms (whole calls).  Where more than the first rows of 32 columns do not fit, 16.
+    const bool wide = inner_pref ? inner_pref == 32 : n <= 4608;
+    const int order[2] = {wide ? 32 : 16, wide ? 16 : 32};
     for (int iw : order)
       if (fit_panel(8, iw, n, pc.inner_cluster, pc.inner_rpc, pc.inner_smem, pc.inner_pos_global, iw == 16)) {
         pc.nb = 64;

@@ -26,8 +26,8 @@ struct PanelConfig {
   int pair128 = 0;
 };
 
-// inner_pref (FP32): 0 picks by n (two-level from n = 512, 16-column inner
-// panels first); 16 or 32 asks for two-level with that inner width first
+// inner_pref (FP32): 0 picks by n (two-level from n = 512, with 32-column inner
+// panels up to n = 4608 and 16-column ones beyond); 16 or 32 asks for two-level with that inner width first
 // (from n = 128); 1 asks for single-level panels.
 template <typename T> PanelConfig choose_panel(int n, int inner_pref = 0);
 

@@ -251,6 +251,8 @@ cudaError_t launch_panel32(int nb, int max_cluster, const BatchLayout& lay, int 
   while (cl < max_cluster && (R + cl - 1) / cl > cap) cl *= 2;
   while (cl < 8 && R > 256 * cl && (long long)batch * cl * 2 <= sms) cl *= 2;
   const int rows = (R + cl - 1) / cl;
+  // two smaller CTAs per SM (96 registers) where there are more CTAs than SMs
+  if (nb == 32 && rows <= 320 && (long long)batch * cl > sms) return launch_shape<32, 1, 320, 2>(cl, rows, lay, batch, k, M, w, s);
   if (nb == 32) return launch_shape<32, 1, 512, 1>(cl, rows, lay, batch, k, M, w, s);
   if (rows <= 512) return launch_shape<16, 1, 512, 2>(cl, rows, lay, batch, k, M, w, s);
   return launch_shape<16, 2, 512, 1>(cl, rows, lay, batch, k, M, w, s);
