@@ -95,7 +95,12 @@ extern "C" unsigned long long refeff_fms_kernel_launches(void) { return g_launch
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
+struct DenseCache;  // the kept workspace of the context's dense solves (below)
+
 struct refeff_fms_context {
+  refeff_fms_context();
+  ~refeff_fms_context();
+  std::unique_ptr<DenseCache> dense;
   int device = 0;
   cudaStream_t stream = nullptr;
   std::string last_error;
@@ -261,6 +266,7 @@ void rfx::context_release(refeff_fms_context* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
   }
+  ctx->dense.reset();
   for (cudaStream_t q : ctx->pool) {
     cudaStreamSynchronize(q);
     cudaStreamDestroy(q);
@@ -2252,6 +2258,141 @@ extern "C" int refeff_fms_gg_section(const refeff_fms_plan* plan, const refeff_c
 // ---------------------------------------------------------------------------
 namespace {
 
+}  // namespace
+
+// The workspace and staging buffer of a context's dense solves, kept between calls (allocating and freeing them took
+// longer than a batch of small solves) unless they hold more than kDenseKeep bytes.
+struct DenseCache {
+  Workspace ws;
+  DevBuf<double2> stage;
+  int tensor_cores = 0;  // the option they were set up under
+  size_t bytes() const {
+    return (ws.M64.n + ws.X64.n + ws.R.n + stage.n) * sizeof(double2) + ws.M32.n * sizeof(float2) +
+           ws.Xsplit.n * sizeof(float4) + ws.tc_images.n + ws.tc64_images.n;
+  }
+};
+constexpr size_t kDenseKeep = size_t(512) << 20;
+refeff_fms_context::refeff_fms_context() = default;
+refeff_fms_context::~refeff_fms_context() = default;
+
+namespace {
+
+// The context's dense workspace, configured for the call.
+int dense_workspace(refeff_fms_context* ctx, int n, int m, int batch, bool fp32, DenseCache*& out) {
+  for (int attempt = 0;; ++attempt) {
+    const bool fresh = !ctx->dense || ctx->dense->tensor_cores != ctx->use_tensor_cores || attempt;
+    if (fresh) {
+      ctx->dense = std::make_unique<DenseCache>();
+      ctx->dense->tensor_cores = ctx->use_tensor_cores;
+    }
+    out = ctx->dense.get();
+    const int rc = ensure_workspace(ctx, out->ws, n, m, batch, fp32);
+    if (rc != REFEFF_FMS_ERR_OUT_OF_MEMORY || fresh) return rc;
+    cudaGetLastError();  // buffers kept from other shapes may be in the way: once more from nothing
+  }
+}
+// Gives a large workspace back at the end of a call.
+struct DenseTrim {
+  refeff_fms_context* ctx;
+  ~DenseTrim() {
+    if (ctx->dense && ctx->dense->bytes() > kDenseKeep) ctx->dense.reset();
+  }
+};
+
+// Packed systems (A: count x n x n, may be null; B: count x n x m; column-major) into [A | B] of the layout, the rows
+// beyond n zero; *nonfinite (nullable) is set when an entry is an infinity or NaN.
+__global__ void pack_systems_kernel(BatchLayout lay, const double2* __restrict__ A, const double2* __restrict__ B,
+                                    double2* __restrict__ M, int* nonfinite) {
+  const int b = blockIdx.z, c = blockIdx.y, n = lay.n;
+  const double2* src = c < n ? (A ? A + (size_t(b) * n + c) * n : nullptr) : B + (size_t(b) * lay.m + (c - n)) * n;
+  double2* dst = M + size_t(b) * lay.stride + size_t(lay.lda) * c;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < lay.lda; r += gridDim.x * blockDim.x) {
+    const double2 v = src && r < n ? src[r] : make_double2(0.0, 0.0);
+    dst[r] = v;
+    if (nonfinite && !cfinite(v)) *nonfinite = 1;
+  }
+}
+__global__ void check_finite_kernel(BatchLayout lay, const double2* __restrict__ M, int* nonfinite) {
+  const double2* col = M + size_t(blockIdx.z) * lay.stride + size_t(lay.lda) * (lay.n + blockIdx.y);
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < lay.n; r += gridDim.x * blockDim.x)
+    if (!cfinite(col[r])) *nonfinite = 1;
+}
+__global__ void unpack_solutions_kernel(BatchLayout lay, const double2* __restrict__ X, double2* __restrict__ out) {
+  const int b = blockIdx.z, c = blockIdx.y;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < lay.n; r += gridDim.x * blockDim.x)
+    out[(size_t(b) * lay.m + c) * lay.n + r] = X[(size_t(b) * lay.m + c) * lay.lda + r];
+}
+
+// Systems of more than this many entries are copied row by row of the layout; smaller ones through the staging buffer,
+// as many at a time as kStage holds, in one copy and one kernel.
+constexpr size_t kStage = size_t(4) << 20;  // entries (64 MB)
+
+// Host systems -> [A | B] of the first `count` matrices.  A may be null (its columns are zeroed).  nonfinite (nullable,
+// device): set when an entry of B is not finite.
+int upload_systems(refeff_fms_context* ctx, DenseCache& d, int count, const refeff_complex128* A,
+                   const refeff_complex128* B, cudaStream_t s, int* nonfinite = nullptr) {
+  const BatchLayout& lay = d.ws.lay;
+  const size_t n = size_t(lay.n), m = size_t(lay.m), na = A ? n * n : 0, one = na + n * m;
+  if (one > kStage) {
+    RF_CUDA(ctx, cudaMemsetAsync(d.ws.M64.p, 0, size_t(count) * lay.stride * sizeof(double2), s));
+    for (int b = 0; b < count; ++b) {
+      double2* Mb = d.ws.M64.p + size_t(b) * lay.stride;
+      if (A)
+        RF_CUDA(ctx, cudaMemcpy2DAsync(Mb, size_t(lay.lda) * sizeof(double2), A + size_t(b) * na, n * sizeof(double2),
+                                       n * sizeof(double2), n, cudaMemcpyHostToDevice, s));
+      RF_CUDA(ctx, cudaMemcpy2DAsync(Mb + size_t(lay.lda) * n, size_t(lay.lda) * sizeof(double2), B + size_t(b) * n * m,
+                                     n * sizeof(double2), n * sizeof(double2), m, cudaMemcpyHostToDevice, s));
+      if (nonfinite) {  // of the right-hand sides
+        count_launch();
+        check_finite_kernel<<<dim3(8, unsigned(m), 1), 128, 0, s>>>(lay, Mb, nonfinite);
+      }
+    }
+    return REFEFF_FMS_OK;
+  }
+  const int per = int(std::min<size_t>(size_t(count), kStage / one));
+  RF_CUDA(ctx, d.stage.alloc(size_t(per) * one));
+  for (int b0 = 0; b0 < count; b0 += per) {
+    const size_t nb = size_t(std::min(per, count - b0));
+    if (A) RF_CUDA(ctx, cudaMemcpyAsync(d.stage.p, A + size_t(b0) * na, nb * na * sizeof(double2), cudaMemcpyHostToDevice, s));
+    RF_CUDA(ctx, cudaMemcpyAsync(d.stage.p + nb * na, B + size_t(b0) * n * m, nb * n * m * sizeof(double2),
+                                 cudaMemcpyHostToDevice, s));
+    const unsigned gx = unsigned(std::min<size_t>(8, (size_t(lay.lda) + 127) / 128));
+    for (size_t z = 0; z < nb; z += 65535) {  // grid limit of the third dimension
+      const size_t nz = std::min<size_t>(65535, nb - z);
+      count_launch();
+      pack_systems_kernel<<<dim3(gx, unsigned(n + m), unsigned(nz)), 128, 0, s>>>(
+          lay, A ? d.stage.p + z * na : nullptr, d.stage.p + nb * na + z * n * m,
+          d.ws.M64.p + (size_t(b0) + z) * lay.stride, nonfinite);
+    }
+    RF_CUDA(ctx, cudaGetLastError());
+  }
+  return REFEFF_FMS_OK;
+}
+
+// X64 of the first `count` matrices -> packed host solutions.
+int download_solutions(refeff_fms_context* ctx, DenseCache& d, int count, refeff_complex128* X, cudaStream_t s) {
+  const BatchLayout& lay = d.ws.lay;
+  const size_t n = size_t(lay.n), m = size_t(lay.m), one = n * m;
+  if (one > kStage) {
+    for (int b = 0; b < count; ++b)
+      RF_CUDA(ctx, cudaMemcpy2DAsync(X + size_t(b) * one, n * sizeof(double2), d.ws.X64.p + size_t(b) * lay.lda * m,
+                                     size_t(lay.lda) * sizeof(double2), n * sizeof(double2), m, cudaMemcpyDeviceToHost, s));
+    return REFEFF_FMS_OK;
+  }
+  const int per = int(std::min<size_t>(std::min<size_t>(size_t(count), 65535), kStage / one));
+  RF_CUDA(ctx, d.stage.alloc(size_t(per) * one));
+  for (int b0 = 0; b0 < count; b0 += per) {
+    const int nb = std::min(per, count - b0);
+    count_launch();
+    unpack_solutions_kernel<<<dim3(unsigned(std::min<size_t>(8, (n + 127) / 128)), unsigned(m), unsigned(nb)), 128, 0, s>>>(
+        lay, d.ws.X64.p + size_t(b0) * lay.lda * m, d.stage.p);
+    RF_CUDA(ctx, cudaGetLastError());
+    RF_CUDA(ctx, cudaMemcpyAsync(X + size_t(b0) * one, d.stage.p, size_t(nb) * one * sizeof(double2),
+                                 cudaMemcpyDeviceToHost, s));
+  }
+  return REFEFF_FMS_OK;
+}
+
 // [A | B] already in M64 (every system of the batch): solve and leave X in
 // ws.X64 (n x m per system, leading dimension lay.lda), statuses in ws.status
 // and first zero pivots in ws.info.  Asynchronous on stream s.
@@ -2259,6 +2400,7 @@ int dense_solve_device(refeff_fms_context* ctx, Workspace& ws, int batch, bool f
   const BatchLayout& lay = ws.lay;
   RF_CUDA(ctx, cudaMemsetAsync(ws.status.p, 0, size_t(batch) * sizeof(int), s));
   RF_CUDA(ctx, cudaMemsetAsync(ws.info.p, 0, size_t(batch) * sizeof(int), s));
+  if (ws.use_tc) RF_CUDA(ctx, cudaMemsetAsync(ws.tc_err.p, 0, sizeof(int), s));  // the workspace outlives a timed-out call
   if (!fp32) {
     const LuWork w64 = lu_work(ws, ws.pc64, true);
     cudaError_t e = lu_eliminate<double>(ws.pc64, lay, batch, ws.M64.p, w64, s);
@@ -2341,9 +2483,6 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   }
   if (!std::isfinite(total) || !(total > 0.0))
     return fail(ctx, REFEFF_FMS_ERR_INVALID_ARGUMENT, "reciprocal FMS total k-point weight must be positive and finite");
-  for (size_t i = 0; i < nn * size_t(n_kpoints); ++i)
-    if (!std::isfinite(structure_factors[i].re) || !std::isfinite(structure_factors[i].im))
-      return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite structure factor");
   // the lattice T by columns, non-zero entries only (FmsReciprocalPlan::new, reciprocal.rs:80-97)
   std::vector<int> ptr(static_cast<size_t>(order) + 1, 0), rows;
   std::vector<double2> vals;
@@ -2364,18 +2503,24 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   }
   RF_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  Workspace ws;
   const BatchLayout lay0 = make_layout(order, order);
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
+  if (ctx->dense) free_b += ctx->dense->bytes();  // kept for calls like this one
   const size_t per = bytes_per_system(lay0, fp32) + size_t(lay0.lda) * order * sizeof(double2);
-  const int B = int(std::max<size_t>(1, std::min<size_t>(size_t(n_kpoints), std::min<size_t>(256, free_b / 2 / per))));
-  int rc = ensure_workspace(ctx, ws, order, order, B, fp32);
+  const int B = int(std::max<size_t>(1, std::min<size_t>(size_t(n_kpoints), std::min<size_t>(1024, free_b / 2 / per))));
+  DenseCache* dense = nullptr;
+  DenseTrim trim{ctx};
+  int rc = dense_workspace(ctx, order, order, B, fp32, dense);
   if (rc) return rc;
+  Workspace& ws = dense->ws;
   const BatchLayout& lay = ws.lay;
   DevBuf<int> d_ptr, d_rows;
   DevBuf<double2> d_vals, d_acc;
   DevBuf<double> d_w;
+  DevBuf<int> d_nonfinite;
+  RF_CUDA(ctx, d_nonfinite.alloc(1));
+  RF_CUDA(ctx, cudaMemsetAsync(d_nonfinite.p, 0, sizeof(int), s));
   RF_CUDA(ctx, d_ptr.upload(ptr.data(), ptr.size(), s));
   RF_CUDA(ctx, d_rows.upload(rows.data(), rows.size(), s));
   RF_CUDA(ctx, d_vals.upload(vals.data(), vals.size(), s));
@@ -2385,12 +2530,8 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   std::vector<int> st(static_cast<size_t>(n_kpoints));
   for (int k0 = 0; k0 < n_kpoints; k0 += B) {
     const int nb = std::min(B, n_kpoints - k0);
-    RF_CUDA(ctx, cudaMemsetAsync(ws.M64.p, 0, size_t(nb) * lay.stride * sizeof(double2), s));
-    for (int b = 0; b < nb; ++b)
-      RF_CUDA(ctx, cudaMemcpy2DAsync(ws.M64.p + size_t(b) * lay.stride + size_t(lay.lda) * order,
-                                     size_t(lay.lda) * sizeof(double2), structure_factors + size_t(k0 + b) * nn,
-                                     size_t(order) * sizeof(double2), size_t(order) * sizeof(double2), size_t(order),
-                                     cudaMemcpyHostToDevice, s));
+    rc = upload_systems(ctx, *dense, nb, nullptr, structure_factors + size_t(k0) * nn, s, d_nonfinite.p);
+    if (rc) return rc;
     count_launch();
     kkr_system_kernel<<<dim3(unsigned((order + 127) / 128), unsigned(order), unsigned(nb)), 128, 0, s>>>(
         lay, ws.M64.p, d_ptr.p, d_rows.p, d_vals.p);
@@ -2403,9 +2544,11 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   }
   std::vector<double2> acc(nn);
   RF_CUDA(ctx, cudaMemcpyAsync(acc.data(), d_acc.p, nn * sizeof(double2), cudaMemcpyDeviceToHost, s));
-  int tc_timeout = 0;
+  int tc_timeout = 0, nonfinite = 0;
   if (ws.use_tc) RF_CUDA(ctx, cudaMemcpyAsync(&tc_timeout, ws.tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  RF_CUDA(ctx, cudaMemcpyAsync(&nonfinite, d_nonfinite.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   RF_CUDA(ctx, cudaStreamSynchronize(s));
+  if (nonfinite) return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite structure factor");
   if (tc_timeout) return fail(ctx, REFEFF_FMS_ERR_CUDA, "tensor-core update timed out");
   int first_bad = -1;
   for (int q = 0; q < n_kpoints; ++q) {
@@ -2515,25 +2658,17 @@ extern "C" int refeff_complex_lu_solve_batched(refeff_fms_context* ctx, int n, i
   RF_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
   const bool fp32 = form == REFEFF_FMS_FORM_FP32_REFINED;
-  Workspace ws;
-  int rc = ensure_workspace(ctx, ws, n, m, batch, fp32);
+  DenseCache* dense = nullptr;
+  DenseTrim trim{ctx};
+  int rc = dense_workspace(ctx, n, m, batch, fp32, dense);
   if (rc) return rc;
-  const BatchLayout& lay = ws.lay;
-  RF_CUDA(ctx, cudaMemsetAsync(ws.M64.p, 0, size_t(batch) * lay.stride * sizeof(double2), s));
-  for (int b = 0; b < batch; ++b) {
-    RF_CUDA(ctx, cudaMemcpy2DAsync(ws.M64.p + size_t(b) * lay.stride, size_t(lay.lda) * sizeof(double2),
-                                   A + size_t(b) * n * n, size_t(n) * sizeof(double2), size_t(n) * sizeof(double2), size_t(n),
-                                   cudaMemcpyHostToDevice, s));
-    RF_CUDA(ctx, cudaMemcpy2DAsync(ws.M64.p + size_t(b) * lay.stride + size_t(lay.lda) * n,
-                                   size_t(lay.lda) * sizeof(double2), B + size_t(b) * n * m, size_t(n) * sizeof(double2),
-                                   size_t(n) * sizeof(double2), size_t(m), cudaMemcpyHostToDevice, s));
-  }
+  Workspace& ws = dense->ws;
+  rc = upload_systems(ctx, *dense, batch, A, B, s);
+  if (rc) return rc;
   rc = dense_solve_device(ctx, ws, batch, fp32, s);
   if (rc) return rc;
-  for (int b = 0; b < batch; ++b)
-    RF_CUDA(ctx, cudaMemcpy2DAsync(X + size_t(b) * n * m, size_t(n) * sizeof(double2), ws.X64.p + size_t(b) * lay.lda * m,
-                                   size_t(lay.lda) * sizeof(double2), size_t(n) * sizeof(double2), size_t(m),
-                                   cudaMemcpyDeviceToHost, s));
+  rc = download_solutions(ctx, *dense, batch, X, s);
+  if (rc) return rc;
   std::vector<int> st(static_cast<size_t>(batch)), info(static_cast<size_t>(batch));
   RF_CUDA(ctx, cudaMemcpyAsync(st.data(), ws.status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
   RF_CUDA(ctx, cudaMemcpyAsync(info.data(), ws.info.p, info.size() * sizeof(int), cudaMemcpyDeviceToHost, s));

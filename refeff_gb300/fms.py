@@ -578,14 +578,14 @@ def complex_lu_solve_batched(ctx: Context, A, B, form=FORM_FP64_LU):
         B = B[None]
     batch, n, _ = A.shape
     m = B.shape[2]
-    a = np.ascontiguousarray(np.stack([A[i].reshape(-1, order="F") for i in range(batch)]))
-    b = np.ascontiguousarray(np.stack([B[i].reshape(-1, order="F") for i in range(batch)]))
-    x = np.zeros_like(b)
+    a = np.ascontiguousarray(A.transpose(0, 2, 1))  # column-major systems
+    b = np.ascontiguousarray(B.transpose(0, 2, 1))
+    x = np.zeros((batch, m, n), np.complex128)
     st = np.zeros(batch, np.int32)
     piv = np.zeros(batch, np.int32)
     rc = ctx._lib.refeff_complex_lu_solve_batched(ctx.handle, n, m, batch, _ptr(a), _ptr(b), _ptr(x), int(form),
                                                   _ptr(st), _ptr(piv))
-    X = np.stack([x[i].reshape((n, m), order="F") for i in range(batch)])
+    X = np.ascontiguousarray(x.transpose(0, 2, 1))
     if rc and rc not in (9, 10):
         raise FmsError(rc, ctx.last_error())
     return X, st, piv
