@@ -148,7 +148,7 @@ unsigned long long refeff_fms_kernel_launches(void);
  *     option or plan setting changes; 0 keeps one launch sequence per plan. */
 #define REFEFF_FMS_OPT_MULTI_GRAPH 7
 /*   REFEFF_FMS_OPT_BICG_TENSOR: 1 (default) runs the BICGSTAB form's
- *     matrix-vector products on the tensor cores (split TF32, four real
+ *     matrix-vector products on the tensor cores (two FP16 terms a value, four real
  *     products, up to 32 right-hand sides); 2 the three-product (3M) form of
  *     the same; 0 on the FP32 CUDA cores.  A product whose bounded wait gives
  *     up hands its matrices to the refined LU. */

@@ -15,6 +15,7 @@
 //   v = A p^;  alpha = rho_new / (r~, v);   s = r - alpha v;  s^ = D s
 //   t = A s^;  omega = (t, s) / (t, t);     x += alpha p^ + omega s^;  r = s - omega t
 //   rho_new = (r~, r);  stop when |r| <= tol |b|.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -43,6 +44,13 @@ struct View {
   int* done;
   float2* part;    // partial products of slices 1..nsplit-1 of the last split product
   int nsplit = 1;  // column slices of that product (1: not split)
+  // tensor-core product (image NULL without it): the exponents of A's rows, of X's columns per vector block, and X as
+  // the product's operand
+  unsigned* amax = nullptr;
+  int* xexp = nullptr;
+  uint8_t* image = nullptr;
+  int xblocks = 0;           // vector blocks of a column
+  int tc_n = 0, tc_three = 0;
   const int* act = nullptr;  // running matrices, compacted (-1 past the count); NULL: blockIdx.y is the matrix
   __device__ __forceinline__ int matrix() const { return act ? act[blockIdx.y] : int(blockIdx.y); }
   __device__ float2* v(int k, int b, int c) const {
@@ -95,6 +103,81 @@ __device__ __forceinline__ void block_accumulate(double* slot0, double a, double
   }
 }
 
+// The larger |component|'s bits; ordered as the magnitudes are, NaN above all.
+__device__ __forceinline__ unsigned abs_bits(float2 v) {
+  return max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+}
+// The exponent s with max 2^s in [2^top, 2^(top + 1)) for a maximum given by its bits (0, infinity and NaN included:
+// the power of two stays a normal number).
+__device__ __forceinline__ int scale_exponent(unsigned bits, int top) {
+  const int e = min(max(int(bits >> 23), 1), 254);
+  return min(top + 127 - e, 126);
+}
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float(unsigned(e + 127) << 23); }  // -126 <= e <= 127
+// hi / lo FP16 parts of two values
+__device__ __forceinline__ void tc_split(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x0 - f.x, x1 - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// Byte offset of 16-byte chunk `chunk` of row `row` in a K-major tile of 32-byte rows with the 32-byte swizzle.
+__device__ __forceinline__ int tc_sw32(int row, int chunk) { return row * 32 + ((chunk ^ ((row >> 2) & 1)) << 4); }
+// The scaled maximum lies below 2^(kTcTop + 1): one less for the three-product form, whose sums Ar + Ai double it.
+__device__ __forceinline__ int tc_top(bool three) { return three ? 13 : 14; }
+__host__ __device__ __forceinline__ constexpr int tc_x_slots(bool three) { return three ? 6 : 8; }
+
+// The block's rows of column c of the next product's X (x[k] = row k kVecThreads + threadIdx.x of the block, 0 past
+// n) as the B operand of the tensor-core product: scaled by a power of two that brings the block's largest component
+// to [2^14, 2^15), split into two FP16 terms and stored in the slabs' slots (bicg_tc_matvec_kernel).  Neighbouring
+// lanes hold neighbouring rows; the even one stores the hi terms of both, the odd one the lo terms, 4 bytes at a time.
+// Written here, once a product, the operand costs its 33 row tiles (n = 4112) one bulk copy each instead of a
+// conversion each.
+__device__ __forceinline__ void store_x_image(const View& w, int b, int c, const float2 (&x)[kVecRowsPerThread]) {
+  if (!w.image) return;
+  __shared__ unsigned red[kVecThreads / 32];
+  unsigned m = 0;
+#pragma unroll
+  for (int k = 0; k < kVecRowsPerThread; ++k) m = max(m, abs_bits(x[k]));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kVecThreads / 32; ++i) m = max(m, red[i]);
+  const int e = scale_exponent(m, tc_top(w.tc_three));
+  if (threadIdx.x == 0) w.xexp[(size_t(b) * w.m + c) * w.xblocks + blockIdx.x] = e;
+  const float f = pow2(e);
+  const int plane = w.tc_n * 32, slab_bytes = tc_x_slots(w.tc_three) * plane, slabs = (w.n + 15) / 16;
+  const bool odd = threadIdx.x & 1;
+  uint8_t* img = w.image + size_t(b) * slabs * slab_bytes;
+#pragma unroll
+  for (int k = 0; k < kVecRowsPerThread; ++k) {
+    const int i = blockIdx.x * kVecRows + k * kVecThreads + int(threadIdx.x);
+    uint32_t hi, lo, shi, slo;  // (re, im) pairs; of re + im in the low half
+    const float re = x[k].x * f, im = x[k].y * f;
+    tc_split(re, im, hi, lo);
+    tc_split(re + im, 0.f, shi, slo);
+    const uint32_t own = odd ? lo : hi, other = __shfl_xor_sync(0xffffffffu, odd ? hi : lo, 1);
+    const uint32_t sown = odd ? slo : shi, sother = __shfl_xor_sync(0xffffffffu, odd ? shi : slo, 1);
+    if ((i >> 4) >= slabs) continue;
+    const uint32_t r0 = odd ? other : own, r1 = odd ? own : other;  // the even row's, the odd row's
+    const uint32_t rr = __byte_perm(r0, r1, 0x5410), ii = __byte_perm(r0, r1, 0x7632);
+    uint8_t* q = img + size_t(i >> 4) * slab_bytes + tc_sw32(c, (i >> 3) & 1) + 2 * (i & 6);
+    auto put = [&](int slot, uint32_t u) { *reinterpret_cast<uint32_t*>(q + slot * plane) = u; };
+    if (w.tc_three) {  // Xr hi, lo, Xi hi, lo, (Xr + Xi) hi, lo
+      put(odd ? 1 : 0, rr);
+      put(odd ? 3 : 2, ii);
+      put(odd ? 5 : 4, __byte_perm(odd ? sother : sown, odd ? sown : sother, 0x5410));
+    } else {  // Xr, Xi hi; Xr, Xi lo; -Xi, Xr hi; -Xi, Xr lo
+      put(odd ? 2 : 0, rr);
+      put(odd ? 3 : 1, ii);
+      put(odd ? 6 : 4, ii ^ 0x80008000u);
+      put(odd ? 7 : 5, rr);
+    }
+  }
+}
+
 __device__ __forceinline__ bool column_idle(const View& w, int b, int c, const int* skip) {
   return (skip && skip[b]) || w.done[b] || w.state[size_t(b) * w.m + c] != 0;
 }
@@ -122,7 +205,7 @@ __global__ void bicg_init_kernel(View w, const float2* __restrict__ M32, size_t 
   block_accumulate(sc + kB2, b2, sc + kAcc1, b2, nullptr, 0.0);
 }
 
-// p = r + beta (p - omega v);  p^ = D p
+// p = r + beta (p - omega v);  p^ = D p, which also goes to the product's operand
 __global__ void bicg_p_kernel(View w, const float2* __restrict__ D, const int* skip) {
   const int b = w.matrix(), c = blockIdx.z;
   if (b < 0) return;
@@ -137,14 +220,19 @@ __global__ void bicg_p_kernel(View w, const float2* __restrict__ D, const int* s
   const float2 *r = w.v(kR, b, c), *v = w.v(kV, b, c);
   float2 *p = w.v(kP, b, c), *ph = w.v(kPh, b, c);
   const float2* Db = D ? D + size_t(b) * w.lda : nullptr;
+  float2 xv[kVecRowsPerThread] = {};
+#pragma unroll
   for (int k = 0; k < kVecRowsPerThread; ++k) {
     const int i = blockIdx.x * kVecRows + k * kVecThreads + threadIdx.x;
     if (i >= w.n) break;
     float2 pi = csub(p[i], cmul(of, v[i]));
     pi = cadd(r[i], cmul(bf, pi));
     p[i] = pi;
-    ph[i] = Db ? cmul(Db[i], pi) : pi;
+    const float2 x = Db ? cmul(Db[i], pi) : pi;
+    ph[i] = x;
+    xv[k] = x;
   }
+  store_x_image(w, b, c, xv);
 }
 
 // Y = A X for the FP32 system matrices: 128 rows x 16 columns per CTA, each
@@ -253,84 +341,93 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 }
 
 // ---------------------------------------------------------------------------
-// Tensor-core product (tcgen05, split TF32): the same Y = A X, slices and
-// partial products as bicg_matvec_kernel, with the complex products on the
-// 5th-generation tensor cores.  Each of the four operand warps owns one row of
-// the CTA's 128-row tile: it loads the row's 16 A entries of a slab with
-// coalesced global loads (two slabs ahead in registers), splits them into TF32
-// hi / lo parts and stores the four real planes (re hi, re lo, im hi, im lo)
-// in the K-major 64-byte-swizzled UMMA layout; the X slab becomes six slots
-// (-im hi, re hi, im hi, -im lo, re lo, im lo) in an order where each adjacent
-// pair is one 2N-row B operand.  One thread issues 6 MMAs of 2N columns per K
-// step of 8 into the adjacent TMEM accumulators [Yr | Yi] (N = 16 or 32):
-//     Yr += Ar Xr + Ai (-Xi)        Yi += Ar Xi + Ai Xr,
-// each real product hi*hi + hi*lo + lo*hi, one A plane against [Xr | Xi] or
-// [-Xi | Xr] at a time (half the MMA instructions of N-column products, as
-// many multiply-adds).  Two plane stages let the operand
-// warps fill one while the MMAs read the other.  Every wait is bounded; a
-// timeout sets *err (the solve then hands its matrices to the LU) and the
-// CTA drains its MMAs and frees its tensor memory before it returns.
-constexpr int kTcRows = 128, kTcK = 16, kTcThreads = 160, kTcStages = 2;
+// Tensor-core product (tcgen05, two FP16 terms a value): the same Y = A X with
+// the complex products on the 5th-generation tensor cores.  Every real number
+// is scaled by a power of two (one a row of A, from the row's largest entry;
+// one a column and vector block of X, store_x_image) so that the largest lands
+// in [2^14, 2^15), and taken as hi + lo, two FP16 values: 22 bits, as in a
+// split into two TF32 values, for entries down to 2^-17 of the largest, an
+// absolute error of 2^-40 of the largest below.  A CTA takes 128 rows and a
+// slice of the columns, in slabs of 16 columns:
+//   warp 5      bulk copies, three slabs ahead: 16 columns of 128 rows of A
+//               (1 KB each) and the slab of X's operand;
+//   warps 0-3   a row of A each thread: 16 entries from shared memory, scaled
+//               and split into the four real planes (re hi, re lo, im hi,
+//               im lo) in the K-major 32-byte-swizzled UMMA layout (two
+//               stages);
+//   warp 4      one thread issues 4 MMAs a slab,
+//     Ar hi x [Xr | Xi] hi, lo and Ai hi x [-Xi | Xr] hi, lo   (4N columns)
+//     Ar lo x [Xr | Xi] hi     and Ai lo x [-Xi | Xr] hi       (2N columns)
+//               into TMEM columns [Yr Yi | yr yi]; the second pair takes the
+//               three small products, so that they do not disturb the FP32
+//               accumulation of the large ones.
+// Every 256 columns warps 0-3 take the accumulators, add the two parts, take
+// the scales back and add to the row's sums in registers.  Every wait is
+// bounded; a timeout sets *err (the solve then hands its matrices to the LU)
+// and the CTA drains its copies and MMAs and frees its tensor memory before it
+// returns.
+// Bound by HBM and the row threads' conversions: n = 4112, 12 matrices, 16
+// columns 346 us under a profiler (1.65 GB read at 62% of the HBM peak); a split
+// into two TF32 terms by the row's thread, loads in registers, the operand of X
+// converted by every CTA and 12 MMAs a slab took 460 us.  Slices of 256 columns
+// instead of 512 and register loads with FP16 terms: 400 us.  A ring of three or
+// of four slabs: the same.
+constexpr int kTcRows = 128, kTcK = 16, kTcThreads = 192, kTcStages = 2, kTcSub = 256;
 constexpr long long kTcBicgPolls = 1LL << 26;  // poll budget of each wait (about 1 s is the other bound)
-constexpr int kTcAPlane = kTcRows * 64;  // 8 KB: 128 rows of 16 TF32 values
+constexpr int kTcAPlane = kTcRows * 32;             // 4 KB: 128 rows of 16 FP16 values
+constexpr int kTcRaw = kTcRows * kTcK * int(sizeof(float2));  // 16 KB of A as stored
+static_assert(kVecRows % kTcSub == 0 && kBicgTcSliceCols % kTcSub == 0, "one scale of X per accumulation");
 
 // k3M: the three-product form P1 = Ar Xr, P2 = Ai Xi, P3 = (Ar + Ai)(Xr + Xi),
-// Yr = P1 - P2, Yi = P3 - P1 - P2 (9 MMAs per K step; six A planes, three
-// accumulators); otherwise the four products above (12 MMAs, two accumulators).
+// Yr = P1 - P2, Yi = P3 - P1 - P2 (six A planes, 6 MMAs of 2N or N columns,
+// large and small accumulators of three products); otherwise the four products
+// above.
 template <int N, bool k3M = false> struct TcMv {
   static constexpr int kAPlanes = k3M ? 6 : 4;
   static constexpr int kA = kAPlanes * kTcAPlane;
-  static constexpr int kBPlane = N * 64;
-  static constexpr int kB = 6 * kBPlane;
-  static constexpr int kStage = kA + kB;
-  static constexpr int kBars = 128;        // barriers, TMEM slot, abort flag
-  static constexpr int kSmem = kTcStages * kStage + kBars + 1024;
-  // TMEM columns (a power of two >= 32): Yr, Yi, or P1, P2, P3
-  static constexpr uint32_t kCols = k3M ? (3 * N <= 64 ? 64u : 128u) : 2u * N;
-  // kind::tf32, D = F32, A = B = TF32, both K-major, M = 128; N columns per MMA for the three-product
-  // form, 2N (one A plane against two adjacent B slots) for the four-product form
-  static constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t((k3M ? N : 2 * N) >> 3) << 17) |
-                                     (uint32_t(kTcRows >> 4) << 24);
+  static constexpr int kBPlane = N * 32;
+  static constexpr int kB = tc_x_slots(k3M) * kBPlane;
+  static constexpr int kRing = kTcRaw + kB;
+  static constexpr int kDepth = N == 16 && !k3M ? 4 : 3;  // two CTAs an SM but for the three products with N = 32
+  static constexpr int kBars = 256;        // barriers, TMEM slot, abort flag
+  static constexpr int kSmem = kDepth * kRing + kTcStages * kA + kBars + 256;
+  // TMEM columns (a power of two >= 32): [Yr Yi | yr yi], or three of [P | p]
+  static constexpr uint32_t kCols = k3M ? 8u * N : 4u * N;
 };
+// kind::f16, D = F32, A = B = FP16, both K-major, M = 128
+__device__ __forceinline__ constexpr uint32_t tc_idesc(int n) {
+  return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(kTcRows >> 4) << 24);
+}
 
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ uint32_t tc_tf32(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return r;
+// start >> 4, LBO 1 (unused when swizzled), SBO = 8 rows x 32 B, version 1, 32-byte swizzle (layout 6)
+__device__ __forceinline__ uint64_t tc_desc32(uint32_t saddr) {
+  return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(1) << 16) | (uint64_t(256 >> 4) << 32) | (uint64_t(1) << 46) |
+         (uint64_t(6) << 61);
 }
-// hi / lo TF32 parts of the real and imaginary parts
-__device__ __forceinline__ void tc_split(float2 v, uint32_t out[4]) {
-  const uint32_t rh = tc_tf32(v.x), ih = tc_tf32(v.y);
-  out[0] = rh;
-  out[1] = tc_tf32(v.x - __uint_as_float(rh));
-  out[2] = ih;
-  out[3] = tc_tf32(v.y - __uint_as_float(ih));
-}
-// Byte offset of (row, k), k < 16, in a K-major tile of 64-byte rows with the
-// 64-byte swizzle: the 16-byte chunk index XOR (row / 2) % 4.
-__device__ __forceinline__ int tc_sw64(int row, int k) {
-  return row * 64 + ((((k >> 2) ^ ((row >> 1) & 3))) << 4) + ((k & 3) << 2);
-}
-// start >> 4, LBO 1 (unused when swizzled), SBO = 8 rows x 64 B, version 1, 64-byte swizzle (layout 4)
-__device__ __forceinline__ uint64_t tc_desc64(uint32_t saddr) {
-  return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(1) << 16) | (uint64_t(512 >> 4) << 32) | (uint64_t(1) << 46) |
-         (uint64_t(4) << 61);
-}
-template <uint32_t kIdesc>
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate));
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 __device__ __forceinline__ void tc_bar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
 __device__ __forceinline__ void tc_bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// bytes (a multiple of 16) from global to shared memory, both 16-byte aligned; completes on `bar`
+__device__ __forceinline__ void tc_bulk(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -352,235 +449,276 @@ __device__ __forceinline__ bool tc_try(uint32_t bar, uint32_t parity) {
 // Bounded wait (poll budget, or 1 s); a timeout raises the CTA's abort flag and *err.
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err,
                                         long long polls) {
-  const uint64_t t0 = tc_now();
+  uint64_t t0 = 0;  // the clock is read only by a wait that is already long
   for (long long it = 0; it < polls; ++it) {
     if (tc_try(bar, parity)) return true;
-    if ((it & 255) == 255) {
+    if ((it & 63) == 63) {
       if (*abort_flag) return false;
-      if (tc_now() - t0 > 1000000000ull) break;
+      const uint64_t t = tc_now();
+      if (t0 == 0) t0 = t;
+      if (t - t0 > 1000000000ull) break;
     }
   }
   *abort_flag = 1;
   atomicExch(err, 1);
   return false;
 }
+// Bounded wait of a warp or thread that is about to leave, for what it has started.
+__device__ __forceinline__ void tc_drain(uint32_t bar, uint32_t parity, long long polls) {
+  const uint64_t t0 = tc_now();
+  for (long long it = 0; it < polls; ++it)
+    if (tc_try(bar, parity) || ((it & 1023) == 1023 && tc_now() - t0 > 1000000000ull)) break;
+}
+
+// amax[b lda + r] = bits of row r's largest |component| over A's columns (zeroed before; grid z: column slices).  Once
+// a batch of matrices, one read of A: 0.26 ms for 12 matrices of n = 4112, beside the products of some 300 iterations.
+constexpr int kScaleCols = 512;
+__global__ void __launch_bounds__(128) bicg_row_max_kernel(View w, const float2* __restrict__ M32, size_t stride,
+                                                           const int* skip) {
+  const int b = blockIdx.y, r = blockIdx.x * 128 + threadIdx.x;
+  if ((skip && skip[b]) || r >= w.n) return;
+  const int c0 = blockIdx.z * kScaleCols, c1 = min(w.n, c0 + kScaleCols);
+  const float2* A = M32 + size_t(b) * stride + r;
+  unsigned m = 0;
+#pragma unroll 16
+  for (int c = c0; c < c1; ++c) m = max(m, abs_bits(__ldcs(A + size_t(w.lda) * c)));
+  atomicMax(w.amax + size_t(b) * w.lda + r, m);
+}
 
 template <int N, bool k3M>
-__global__ void __launch_bounds__(kTcThreads) bicg_tc_matvec_kernel(View w, const float2* __restrict__ M32,
-                                                                     size_t stride, int src, int dst, int kchunk,
+__global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, const float2* __restrict__ M32,
+                                                                     size_t stride, int dst, int kchunk,
                                                                      const int* skip, int* err, long long polls) {
   using L = TcMv<N, k3M>;
+  constexpr int kMaxSubs = kBicgTcSliceCols / kTcSub;
   const int b = w.matrix();
   // decided once for the whole CTA (another CTA may raise the error flag meanwhile), before any tensor
   // memory is taken; a raised error skips the product
   __shared__ int go;
+  __shared__ int xexp[kMaxSubs][N];  // the scale exponents of X's columns
   if (threadIdx.x == 0) go = !(b < 0 || (skip && skip[b]) || w.done[b] || *reinterpret_cast<volatile int*>(err));
   __syncthreads();
   if (!go) return;
   extern __shared__ uint8_t tsm[];
   const uint32_t raw = tc_smem_u32(tsm);
-  const uint32_t sbase = (raw + 1023u) & ~1023u;
-  uint8_t* const gbase = tsm + (sbase - raw);
-  uint8_t* const meta = gbase + kTcStages * L::kStage;
-  // barriers: full[2] (128 operand threads), empty[2] (commit), acc (commit), drain (commit)
+  const uint32_t sbase = (raw + 255u) & ~255u;  // the swizzle repeats after 256 bytes
+  uint8_t* const gbase = tsm + (sbase - raw);  // [kTcStages] planes, [kTcRing] (A as stored, X operand)
+  constexpr int kTcRing = L::kDepth, kRingBase = kTcStages * L::kA;
+  uint8_t* const meta = gbase + kRingBase + kTcRing * L::kRing;
+  // barriers: planes full[2] (4 warps) and empty[2] (commit); ring full[] (copies) and empty[] (4 warps, commit);
+  // accumulators (commit); drain (commit)
   auto bar = [&](int i) { return tc_smem_u32(meta + 8 * i); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + 64);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + 68);
+  constexpr int kFull = 0, kEmpty = kTcStages, kRFull = 2 * kTcStages, kREmpty = kRFull + kTcRing,
+                kAcc = kREmpty + kTcRing, kDrain = kAcc + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + 192);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + 196);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int slice = blockIdx.z;
   const int n = w.n, r0 = blockIdx.x * kTcRows;
   const int kbeg = slice * kchunk, kend = min(n, kbeg + kchunk);
   const int slabs = (kend - kbeg + kTcK - 1) / kTcK;  // >= 1: slices start below n
-  const float2* A = M32 + size_t(b) * stride;
+  constexpr int kSubSlabs = kTcSub / kTcK;
 
+  if (tid == 0) {
+    for (int i = 0; i < kTcStages; ++i) {
+      tc_bar_init(bar(kFull + i), 4);
+      tc_bar_init(bar(kEmpty + i), 1);
+    }
+    for (int i = 0; i < kTcRing; ++i) {
+      tc_bar_init(bar(kRFull + i), 1);
+      tc_bar_init(bar(kREmpty + i), 5);
+    }
+    tc_bar_init(bar(kAcc), 1);
+    tc_bar_init(bar(kDrain), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();  // the copies start beside the rest of the preparation
   if (warp == 4) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)),
                  "r"(L::kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid == 0) {
-    for (int i = 0; i < kTcStages; ++i) {
-      tc_bar_init(bar(i), 128);            // full: every operand thread
-      tc_bar_init(bar(kTcStages + i), 1);  // empty: one commit
+  uint32_t tmem = 0;
+  if (warp < 5) {
+    for (int i = tid; i < kMaxSubs * N; i += 160) {
+      const int sub = i / N, c = i % N, k = kbeg + sub * kTcSub;
+      xexp[sub][c] = c < w.m && k < kend ? w.xexp[(size_t(b) * w.m + c) * w.xblocks + k / kVecRows] : 0;
     }
-    tc_bar_init(bar(2 * kTcStages), 1);      // accumulators complete
-    tc_bar_init(bar(2 * kTcStages + 1), 1);  // drain
-    *abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync 1, 160;" ::: "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tmem = *tmem_slot;
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tmem_slot;
 
   if (warp < 4) {
-    // ---- operand warps: row r0 + tid of A, and the X slab ----
+    // ---- operand warps: row r0 + tid of A ----
     const int row = r0 + tid;
     const bool row_ok = row < n;
-    auto load = [&](int sl, float2 (&v)[kTcK]) {
-      const int k0 = kbeg + sl * kTcK;
+    const int aexp = scale_exponent(row_ok ? w.amax[size_t(b) * w.lda + row] : 0u, tc_top(k3M));
+    const float as = pow2(aexp);
+    float2 y[N];
 #pragma unroll
-      for (int kk = 0; kk < kTcK; ++kk)
-        v[kk] = (row_ok && sl < slabs && k0 + kk < kend) ? __ldcs(A + size_t(row) + size_t(w.lda) * (k0 + kk))
-                                                          : make_float2(0.f, 0.f);
-    };
-    float2 v0[kTcK], v1[kTcK], v2[kTcK];
-    load(0, v0);
-    load(1, v1);
+    for (int c = 0; c < N; ++c) y[c] = make_float2(0.f, 0.f);
     bool ok = true;
-    for (int sl = 0; sl < slabs && ok; ++sl) {
-      load(sl + 2, v2);
+    int rs = 0;           // ring stage and its phase
+    uint32_t rph = 0;
+    for (int sl = 0; sl < slabs; ++sl) {
       const int st = sl & 1;
-      const uint32_t ph = uint32_t((sl >> 1) & 1);
-      ok = tc_wait(bar(kTcStages + st), ph ^ 1u, abort_flag, err, polls);  // the MMAs of slab sl - 2 are done
-      if (!ok) break;
-      uint8_t* const sA = gbase + st * L::kStage;
-      uint8_t* const sB = sA + L::kA;
+      ok = tc_wait(bar(kRFull + rs), rph, abort_flag, err, polls);
+      ok = ok && tc_wait(bar(kEmpty + st), uint32_t((sl >> 1) & 1) ^ 1u, abort_flag, err, polls);  // MMAs of slab sl - 2
+      if (!__all_sync(0xffffffffu, ok)) {
+        ok = false;
+        break;
+      }
+      const float2* ra = reinterpret_cast<const float2*>(gbase + kRingBase + rs * L::kRing) + tid;
+      float2 v[kTcK];
 #pragma unroll
-      for (int k4 = 0; k4 < kTcK / 4; ++k4) {
+      for (int kk = 0; kk < kTcK; ++kk) v[kk] = ra[kk * kTcRows];
+      const int left = kend - (kbeg + sl * kTcK);
+      if (left < kTcK) {  // the matrix's last slab: columns that were not copied
+#pragma unroll
+        for (int kk = 0; kk < kTcK; ++kk)
+          if (kk >= left) v[kk] = make_float2(0.f, 0.f);
+      }
+      uint8_t* const sA = gbase + st * L::kA;
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
         uint32_t q[L::kAPlanes][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float2 a = v0[4 * k4 + i];
-          uint32_t sv[4];
-          tc_split(a, sv);
-#pragma unroll
-          for (int pl = 0; pl < 4; ++pl) q[pl][i] = sv[pl];
-          if constexpr (k3M) {  // Ar + Ai, hi and lo
-            const float sum = a.x + a.y;
-            const uint32_t hi = tc_tf32(sum);
-            q[4][i] = hi;
-            q[5][i] = tc_tf32(sum - __uint_as_float(hi));
-          }
+          const float2 a0 = v[8 * ch + 2 * i], a1 = v[8 * ch + 2 * i + 1];
+          const float r0s = a0.x * as, r1s = a1.x * as, i0s = a0.y * as, i1s = a1.y * as;
+          tc_split(r0s, r1s, q[0][i], q[1][i]);
+          tc_split(i0s, i1s, q[2][i], q[3][i]);
+          if constexpr (k3M) tc_split(r0s + i0s, r1s + i1s, q[4][i], q[5][i]);  // Ar + Ai
         }
-        const int off = tc_sw64(tid, 4 * k4);
+        const int off = tc_sw32(tid, ch);
 #pragma unroll
         for (int pl = 0; pl < L::kAPlanes; ++pl)
           *reinterpret_cast<uint4*>(sA + pl * kTcAPlane + off) = make_uint4(q[pl][0], q[pl][1], q[pl][2], q[pl][3]);
       }
-      const int k0 = kbeg + sl * kTcK;
-#pragma unroll
-      for (int j = 0; j < N * kTcK / 128; ++j) {
-        const int e = tid + 128 * j, kk = e % kTcK, c = e / kTcK;
-        const float2 x = (c < w.m && k0 + kk < kend) ? w.v(src, b, c)[k0 + kk] : make_float2(0.f, 0.f);
-        uint32_t sv[4];
-        tc_split(x, sv);
-        const int off = tc_sw64(c, kk);
-        auto put = [&](int slot, uint32_t v) { *reinterpret_cast<uint32_t*>(sB + slot * L::kBPlane + off) = v; };
-        if constexpr (k3M) {  // Xr hi, Xr lo, Xi hi, Xi lo, (Xr + Xi) hi, lo
-#pragma unroll
-          for (int pl = 0; pl < 4; ++pl) put(pl, sv[pl]);
-          const float sum = x.x + x.y;
-          const uint32_t hi = tc_tf32(sum);
-          put(4, hi);
-          put(5, tc_tf32(sum - __uint_as_float(hi)));
-        } else {
-          // slots -Xi hi, Xr hi, Xi hi, -Xi lo, Xr lo, Xi lo: each adjacent pair is one 2N-row B operand
-          put(0, sv[2] ^ 0x80000000u);
-          put(1, sv[0]);
-          put(2, sv[2]);
-          put(3, sv[3] ^ 0x80000000u);
-          put(4, sv[1]);
-          put(5, sv[3]);
-        }
-      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the planes are read by the tensor cores
-      tc_bar_arrive(bar(st));
-#pragma unroll
-      for (int kk = 0; kk < kTcK; ++kk) {
-        v0[kk] = v1[kk];
-        v1[kk] = v2[kk];
+      __syncwarp();
+      if (lane == 0) {
+        tc_bar_arrive(bar(kFull + st));
+        tc_bar_arrive(bar(kREmpty + rs));
       }
-    }
-    // ---- epilogue: the tile's rows of Y (or of this slice's partial product) ----
-    const bool ready = ok && tc_wait(bar(2 * kTcStages), 0u, abort_flag, err, polls);
-    if (__all_sync(0xffffffffu, ready)) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t tr = tmem + (uint32_t(warp * 32) << 16), ti = tr + uint32_t(N);
-      auto ld8 = [](uint32_t addr, uint32_t (&o)[8]) {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7])
-                     : "r"(addr));
-      };
+      if (++rs == kTcRing) {
+        rs = 0;
+        rph ^= 1u;
+      }
+      if ((sl + 1) % kSubSlabs == 0 || sl + 1 == slabs) {
+        // ---- the accumulators of these columns ----
+        const int sub = sl / kSubSlabs;
+        ok = tc_wait(bar(kAcc), uint32_t(sub & 1), abort_flag, err, polls);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tr = tmem + (uint32_t(warp * 32) << 16);
+        auto ld8 = [](uint32_t addr, uint32_t (&o)[8]) {
+          asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7])
+                       : "r"(addr));
+        };
 #pragma unroll
-      for (int cb = 0; cb < N / 8; ++cb) {
-        uint32_t yr[8], yi[8], y3[8];
-        ld8(tr + uint32_t(cb * 8), yr);
-        ld8(ti + uint32_t(cb * 8), yi);
-        if constexpr (k3M) ld8(ti + uint32_t(N + cb * 8), y3);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row_ok) {
+        for (int cb = 0; cb < N / 8; ++cb) {
+          // accumulator groups of N columns: Yr, Yi, yr, yi, or P1, p1, P2, p2, P3, p3
+          constexpr int kGroups = k3M ? 6 : 4;
+          uint32_t g[kGroups][8];
+#pragma unroll
+          for (int i = 0; i < kGroups; ++i) ld8(tr + uint32_t(i * N + cb * 8), g[i]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int c = cb * 8 + j;
-            if (c < w.m) {
-              float2* y = slice == 0 ? w.v(dst, b, c) : w.pv(slice, b, c);
-              float2 out;
-              if constexpr (k3M) {  // Yr = P1 - P2, Yi = P3 - P1 - P2
-                const float p1 = __uint_as_float(yr[j]), p2 = __uint_as_float(yi[j]), p3 = __uint_as_float(y3[j]);
-                out = make_float2(p1 - p2, p3 - p1 - p2);
-              } else {
-                out = make_float2(__uint_as_float(yr[j]), __uint_as_float(yi[j]));
-              }
-              y[row] = out;
+            auto sum = [&](int hi, int lo) { return __uint_as_float(g[hi][j]) + __uint_as_float(g[lo][j]); };
+            float2 out;
+            if constexpr (k3M) {  // Yr = P1 - P2, Yi = P3 - P1 - P2
+              const float p1 = sum(0, 1), p2 = sum(2, 3), p3 = sum(4, 5);
+              out = make_float2(p1 - p2, p3 - p1 - p2);
+            } else {
+              out = make_float2(sum(0, 2), sum(1, 3));
             }
+            const int e = -(aexp + xexp[sub][c]), e1 = e >> 1;
+            const float f1 = pow2(e1), f2 = pow2(e - e1);
+            y[c] = cadd(y[c], make_float2(out.x * f1 * f2, out.y * f1 * f2));
           }
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the next slab's MMAs overwrite them
       }
     }
-  } else if (lane == 0) {
+    if (ok && row_ok) {
+#pragma unroll
+      for (int c = 0; c < N; ++c)
+        if (c < w.m) (slice == 0 ? w.v(dst, b, c) : w.pv(slice, b, c))[row] = y[c];
+    }
+  } else if (warp == 4 && lane == 0) {
     // ---- MMA issuer ----
     bool issued = false, ok = true;
+    int rs = 0;
     for (int sl = 0; sl < slabs; ++sl) {
       const int st = sl & 1;
-      ok = tc_wait(bar(st), uint32_t((sl >> 1) & 1), abort_flag, err, polls);
+      // the planes; their warps have waited for the slab's copies
+      ok = tc_wait(bar(kFull + st), uint32_t((sl >> 1) & 1), abort_flag, err, polls);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t sA = sbase + uint32_t(st * L::kStage), sB = sA + uint32_t(L::kA);
+      const uint32_t sA = sbase + uint32_t(st * L::kA), sB = sbase + uint32_t(kRingBase + rs * L::kRing + kTcRaw);
+      auto ad = [&](int pl) { return tc_desc32(sA + uint32_t(pl * kTcAPlane)); };
+      auto bd = [&](int pl) { return tc_desc32(sB + uint32_t(pl * L::kBPlane)); };
+      const uint32_t a0 = sl % kSubSlabs == 0 ? 0u : 1u;
+      if constexpr (k3M) {
 #pragma unroll
-      for (int ks = 0; ks < kTcK / 8; ++ks) {
-        const uint32_t koff = uint32_t(ks * 32);
-        auto ad = [&](int pl) { return tc_desc64(sA + uint32_t(pl * kTcAPlane) + koff); };
-        auto bd = [&](int pl) { return tc_desc64(sB + uint32_t(pl * L::kBPlane) + koff); };
-        const uint32_t a0 = (sl == 0 && ks == 0) ? 0u : 1u;
-        const uint32_t tr = tmem, ti = tmem + uint32_t(N);
-        if constexpr (k3M) {
-          const uint32_t t3 = tmem + uint32_t(2 * N);
-          // P1 = Ar Xr, P2 = Ai Xi, P3 = (Ar + Ai)(Xr + Xi), each hi*hi + hi*lo + lo*hi
-          tc_mma<L::kIdesc>(tr, ad(0), bd(0), a0);
-          tc_mma<L::kIdesc>(tr, ad(0), bd(1), 1u);
-          tc_mma<L::kIdesc>(tr, ad(1), bd(0), 1u);
-          tc_mma<L::kIdesc>(ti, ad(2), bd(2), a0);
-          tc_mma<L::kIdesc>(ti, ad(2), bd(3), 1u);
-          tc_mma<L::kIdesc>(ti, ad(3), bd(2), 1u);
-          tc_mma<L::kIdesc>(t3, ad(4), bd(4), a0);
-          tc_mma<L::kIdesc>(t3, ad(4), bd(5), 1u);
-          tc_mma<L::kIdesc>(t3, ad(5), bd(4), 1u);
-        } else {
-          // [Yr | Yi] (2N columns) += A-plane x [left | right] B slots:
-          //   Ar hi [Xr hi | Xi hi], Ar hi [Xr lo | Xi lo], Ar lo [Xr hi | Xi hi],
-          //   Ai hi [-Xi hi | Xr hi], Ai hi [-Xi lo | Xr lo], Ai lo [-Xi hi | Xr hi]
-          // i.e. Yr += Ar Xr + Ai (-Xi), Yi += Ar Xi + Ai Xr, each hi*hi + hi*lo + lo*hi, six MMAs
-          (void)ti;
-          tc_mma<L::kIdesc>(tr, ad(0), bd(1), a0);
-          tc_mma<L::kIdesc>(tr, ad(0), bd(4), 1u);
-          tc_mma<L::kIdesc>(tr, ad(1), bd(1), 1u);
-          tc_mma<L::kIdesc>(tr, ad(2), bd(0), 1u);
-          tc_mma<L::kIdesc>(tr, ad(2), bd(3), 1u);
-          tc_mma<L::kIdesc>(tr, ad(3), bd(0), 1u);
+        for (int p = 0; p < 3; ++p) {  // [P | p] += hi [hi | lo], p += lo hi
+          const uint32_t t = tmem + uint32_t(2 * N * p);
+          tc_mma(t, ad(2 * p), bd(2 * p), tc_idesc(2 * N), a0);
+          tc_mma(t + uint32_t(N), ad(2 * p + 1), bd(2 * p), tc_idesc(N), 1u);
         }
+      } else {
+        tc_mma(tmem, ad(0), bd(0), tc_idesc(4 * N), a0);
+        tc_mma(tmem, ad(2), bd(4), tc_idesc(4 * N), 1u);
+        tc_mma(tmem + uint32_t(2 * N), ad(1), bd(0), tc_idesc(2 * N), 1u);
+        tc_mma(tmem + uint32_t(2 * N), ad(3), bd(4), tc_idesc(2 * N), 1u);
       }
       issued = true;
-      tc_commit(bar(kTcStages + st));  // the stage is free once these MMAs have read it
+      tc_commit(bar(kEmpty + st));   // the planes and
+      tc_commit(bar(kREmpty + rs));  // the ring stage are free once these MMAs have read them
+      if ((sl + 1) % kSubSlabs == 0 || sl + 1 == slabs) tc_commit(bar(kAcc));
+      if (++rs == kTcRing) rs = 0;
     }
-    if (ok) tc_commit(bar(2 * kTcStages));  // Y complete
     if (issued) {
       // every MMA of this CTA has completed before the tensor memory is freed
-      tc_commit(bar(2 * kTcStages + 1));
-      const uint64_t t0 = tc_now();
-      for (long long it = 0; it < polls; ++it)
-        if (tc_try(bar(2 * kTcStages + 1), 0u) || ((it & 1023) == 1023 && tc_now() - t0 > 1000000000ull)) break;
+      tc_commit(bar(kDrain));
+      tc_drain(bar(kDrain), 0u, polls);
     }
+  } else if (warp == 5) {
+    // ---- copies: lane q brings column q of the slab, lane 16 the X operand ----
+    const uint32_t col_bytes = uint32_t(min(kTcRows, w.lda - r0)) * 8u;
+    const float2* A = M32 + size_t(b) * stride + r0;
+    const uint8_t* X = w.image + (size_t(b) * ((n + kTcK - 1) / kTcK) + kbeg / kTcK) * L::kB;
+    int rs = 0, sl = 0;
+    uint32_t rph = 0;
+    for (; sl < slabs; ++sl) {
+      int ok = 1;
+      if (lane == 0) ok = tc_wait(bar(kREmpty + rs), rph ^ 1u, abort_flag, err, polls);
+      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+      const int k0 = kbeg + sl * kTcK, cols = min(kTcK, kend - k0);
+      const uint32_t dstA = sbase + uint32_t(kRingBase + rs * L::kRing);
+      if (lane == 0) tc_bar_expect(bar(kRFull + rs), uint32_t(cols) * col_bytes + uint32_t(L::kB));
+      __syncwarp();
+      if (lane < cols)
+        tc_bulk(dstA + uint32_t(lane * kTcRows * 8), A + size_t(w.lda) * (k0 + lane), col_bytes, bar(kRFull + rs));
+      if (lane == kTcK) tc_bulk(dstA + uint32_t(kTcRaw), X + size_t(sl) * L::kB, uint32_t(L::kB), bar(kRFull + rs));
+      if (++rs == kTcRing) {
+        rs = 0;
+        rph ^= 1u;
+      }
+    }
+    // no copy outlives the CTA: the last ones started
+    if (lane == 0)
+      for (int q = max(0, sl - kTcRing); q < sl; ++q) tc_drain(bar(kRFull + q % kTcRing), uint32_t((q / kTcRing) & 1), polls);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -642,6 +780,8 @@ __global__ void bicg_block_apply_kernel(View w, int src, int dst, const float2* 
   if (column_idle(w, b, c, skip)) return;
   const float2* in = w.v(src, b, c);
   float2* out = w.v(dst, b, c);
+  float2 xv[kVecRowsPerThread] = {};
+#pragma unroll
   for (int k = 0; k < kVecRowsPerThread; ++k) {
     const int i = blockIdx.x * kVecRows + k * kVecThreads + threadIdx.x;
     if (i >= w.n) break;
@@ -650,10 +790,12 @@ __global__ void bicg_block_apply_kernel(View w, int src, int dst, const float2* 
     float2 acc = make_float2(0.f, 0.f);
     for (int q2 = 0; q2 < cnt; ++q2) cfma(acc, row[q2], in[s0 + q2]);
     out[i] = acc;
+    xv[k] = acc;
   }
+  store_x_image(w, b, c, xv);
 }
 
-// s = r - alpha v (in r);  s^ = D s
+// s = r - alpha v (in r);  s^ = D s, which also goes to the product's operand
 __global__ void bicg_s_kernel(View w, const float2* __restrict__ D, const int* skip) {
   const int b = w.matrix(), c = blockIdx.z;
   if (b < 0) return;
@@ -663,13 +805,18 @@ __global__ void bicg_s_kernel(View w, const float2* __restrict__ D, const int* s
   float2 *r = w.v(kR, b, c), *sh = w.v(kSh, b, c);
   const float2* v = w.v(kV, b, c);
   const float2* Db = D ? D + size_t(b) * w.lda : nullptr;
+  float2 xv[kVecRowsPerThread] = {};
+#pragma unroll
   for (int k = 0; k < kVecRowsPerThread; ++k) {
     const int i = blockIdx.x * kVecRows + k * kVecThreads + threadIdx.x;
     if (i >= w.n) break;
     const float2 si = csub(r[i], cmul(af, v[i]));
     r[i] = si;
-    sh[i] = Db ? cmul(Db[i], si) : si;
+    const float2 x = Db ? cmul(Db[i], si) : si;
+    sh[i] = x;
+    xv[k] = x;
   }
+  store_x_image(w, b, c, xv);
 }
 
 // acc2 += (t, s), acc3 += |t|^2
@@ -836,6 +983,23 @@ int bicg_slices(int n, bool tensor, int* chunk) {
   return (n + c - 1) / c;
 }
 
+size_t bicg_image_bytes(int n, int m, int batch) {
+  return m > 32 ? 0 : size_t(batch) * size_t((n + kTcK - 1) / kTcK) * tc_x_slots(false) * (m <= 16 ? 16 : 32) * 32;
+}
+size_t bicg_exponents(int n, int m, int batch) { return size_t(batch) * m * size_t((n + kVecRows - 1) / kVecRows); }
+
+cudaError_t bicg_row_scales(const BatchLayout& lay, int batch, const float2* M32, const BicgWork& w, const int* skip,
+                            cudaStream_t s) {
+  if (!w.tensor || !w.tc_err || lay.m > 32) return cudaSuccess;
+  View v{lay.n, lay.m, lay.lda, batch, w.vec, w.sc, w.state, w.done, w.part, 1};
+  v.amax = w.amax;
+  cudaMemsetAsync(w.amax, 0, size_t(batch) * lay.lda * sizeof(unsigned), s);
+  count_launch();
+  const dim3 grid(unsigned((lay.n + 127) / 128), unsigned(batch), unsigned((lay.n + kScaleCols - 1) / kScaleCols));
+  bicg_row_max_kernel<<<grid, 128, 0, s>>>(v, M32, lay.stride, skip);
+  return cudaGetLastError();
+}
+
 cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const float2* D, const BlockPrecond* blk,
                            const BicgWork& w, double tol, int max_iter, int poll, const int* skip, int* failed,
                            cudaStream_t s) {
@@ -848,14 +1012,22 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
     if (e != cudaSuccess) return e;
   }
   // the tensor-core product for up to 32 right-hand sides (N = 16 or 32 accumulator columns)
-  const bool tensor = w.tensor && w.tc_err && lay.m <= 32;
+  const bool tensor = w.tensor && w.tc_err && lay.m <= 32 && (w.part || lay.n <= kBicgTcSliceCols);
   const bool n16 = lay.m <= 16, three = w.tensor == 2;
+  if (tensor) {
+    v.amax = w.amax;
+    v.xexp = w.xexp;
+    v.image = w.image;
+    v.xblocks = (lay.n + kVecRows - 1) / kVecRows;
+    v.tc_n = n16 ? 16 : 32;
+    v.tc_three = three;
+  }
   // the four instantiations: N = 16 / 32 accumulator columns, four or three products
-  auto tc_launch = [&](auto kN, auto k3, const dim3& grid, const View& view, int src, int dst, int chunk) {
+  auto tc_launch = [&](auto kN, auto k3, const dim3& grid, const View& view, int dst, int chunk) {
     constexpr int N = decltype(kN)::value;
     constexpr bool M3 = decltype(k3)::value;
-    bicg_tc_matvec_kernel<N, M3><<<grid, kTcThreads, TcMv<N, M3>::kSmem, s>>>(view, M32, lay.stride, src, dst, chunk,
-                                                                              skip, w.tc_err, kTcBicgPolls);
+    bicg_tc_matvec_kernel<N, M3><<<grid, kTcThreads, TcMv<N, M3>::kSmem, s>>>(view, M32, lay.stride, dst, chunk, skip,
+                                                                              w.tc_err, kTcBicgPolls);
   };
   auto tc_attr = [&](auto kN, auto k3) {
     constexpr int N = decltype(kN)::value;
@@ -911,17 +1083,18 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
   }
   View vr = v;  // the view of the iteration's launches
   vr.act = compact ? w.act : nullptr;
-  // dst = A src over the running matrices: V = A P^ or T = A S^
+  // dst = A src over the running matrices: V = A P^ or T = A S^ (the tensor-core product's operand is w.image, written
+  // with src)
   auto product = [&](unsigned rows_y, int src, int dst) {
     count_launch();
     if (tensor) {
       const dim3 tgrid(tc_row_blocks, rows_y, unsigned(nsplit));
       if (n16) {
-        if (three) tc_launch(I16{}, T3{}, tgrid, vr, src, dst, chunk);
-        else tc_launch(I16{}, T4{}, tgrid, vr, src, dst, chunk);
+        if (three) tc_launch(I16{}, T3{}, tgrid, vr, dst, chunk);
+        else tc_launch(I16{}, T4{}, tgrid, vr, dst, chunk);
       } else {
-        if (three) tc_launch(I32{}, T3{}, tgrid, vr, src, dst, chunk);
-        else tc_launch(I32{}, T4{}, tgrid, vr, src, dst, chunk);
+        if (three) tc_launch(I32{}, T3{}, tgrid, vr, dst, chunk);
+        else tc_launch(I32{}, T4{}, tgrid, vr, dst, chunk);
       }
     } else {
       const dim3 mgrid(unsigned(row_blocks), rows_y, unsigned(groups * nsplit));
@@ -933,8 +1106,10 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
     vr.nsplit = nsplit;  // the dot kernels sum the slices
     const unsigned rows_y = unsigned(compact ? running : batch);
     const dim3 rgrid(vgrid.x, rows_y, vgrid.z);
+    View vec = vr;
+    if (blk) vec.image = nullptr;  // bicg_block_apply_kernel writes the operand
     count_launch();
-    bicg_p_kernel<<<rgrid, kVecThreads, 0, s>>>(vr, blk ? nullptr : D, skip);
+    bicg_p_kernel<<<rgrid, kVecThreads, 0, s>>>(vec, blk ? nullptr : D, skip);
     if (blk) {
       count_launch();
       bicg_block_apply_kernel<<<rgrid, kVecThreads, 0, s>>>(vr, kP, kPh, blk->B, blk->state_atom, blk->atom_off,
@@ -946,7 +1121,7 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
     count_launch();
     bicg_alpha_kernel<<<sblocks, sthreads, 0, s>>>(v, skip);
     count_launch();
-    bicg_s_kernel<<<rgrid, kVecThreads, 0, s>>>(vr, blk ? nullptr : D, skip);
+    bicg_s_kernel<<<rgrid, kVecThreads, 0, s>>>(vec, blk ? nullptr : D, skip);
     if (blk) {
       count_launch();
       bicg_block_apply_kernel<<<rgrid, kVecThreads, 0, s>>>(vr, kR, kSh, blk->B, blk->state_atom, blk->atom_off,

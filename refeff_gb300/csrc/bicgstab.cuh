@@ -12,10 +12,11 @@ constexpr int kBicgVectors = 8;
 constexpr int kBicgScalars = 16;
 // Column slices of the matrix-vector product (partial products summed by the
 // dot kernels): slices of at least 512 columns, at most 16, on the CUDA cores;
-// slices of 256 columns on the tensor cores, whose FP32 accumulation is
-// exact only for short sums.  bicg_slices gives the count for n.
+// slices of 512 columns on the tensor cores, which accumulate 256 of them at
+// a time (their FP32 sums are exact only when short) and add the two in
+// registers.  bicg_slices gives the count for n.
 constexpr int kBicgMaxSplit = 16;
-constexpr int kBicgTcSliceCols = 256;
+constexpr int kBicgTcSliceCols = 512;
 int bicg_slices(int n, bool tensor, int* chunk = nullptr);
 
 struct BicgWork {
@@ -28,6 +29,9 @@ struct BicgWork {
   float2* part = nullptr;    // (slices - 1) * batch * lda * m: partial products of the split product
   int* act = nullptr;        // batch: compacted list of running matrices
   int* tc_err = nullptr;     // 1 int: set when a wait of the tensor-core product gave up
+  unsigned* amax = nullptr;  // batch * lda: bits of the largest |component| of each row of A (bicg_row_scales)
+  int* xexp = nullptr;       // bicg_exponents: scales of the tensor-core product's operand
+  uint8_t* image = nullptr;  // bicg_image_bytes: that operand
   int tensor = 0;            // products on the tensor cores (up to 32 right-hand sides)
 };
 
@@ -49,6 +53,12 @@ struct BlockPrecond {
   const int* atom_off = nullptr;
   int N = 0, C = 0;
 };
+size_t bicg_image_bytes(int n, int m, int batch);
+size_t bicg_exponents(int n, int m, int batch);
+// The row maxima that the tensor-core product scales A's rows by: once for a
+// batch of matrices, before its bicgstab_solve calls.
+cudaError_t bicg_row_scales(const BatchLayout& lay, int batch, const float2* M32, const BicgWork& w, const int* skip,
+                            cudaStream_t s);
 // blk (nullable) replaces D when given.
 cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const float2* D, const BlockPrecond* blk,
                            const BicgWork& w, double tol, int max_iter, int poll, const int* skip, int* failed,

@@ -455,6 +455,9 @@ struct Workspace {
   // BiCGSTAB form: solver vectors and scalars, the preconditioner diagonal,
   // per-atom features and network outputs
   DevBuf<float2> bicg_vec, precond_D;
+  DevBuf<unsigned> bicg_amax;  // row maxima, operand scales and operand of the tensor-core product
+  DevBuf<int> bicg_xexp;
+  DevBuf<uint8_t> bicg_image;
   DevBuf<float2> bicg_part;  // partial products of the split matrix-vector product
   DevBuf<int> bicg_act;      // compacted list of the running matrices
   DevBuf<int> bicg_err;      // set when a wait of the tensor-core product gave up
@@ -1101,6 +1104,9 @@ BicgWork bicg_work(Workspace& ws) {
   w.part = ws.bicg_part.p;
   w.act = ws.bicg_act.p;
   w.tc_err = ws.bicg_err.p;
+  w.amax = ws.bicg_amax.p;
+  w.xexp = ws.bicg_xexp.p;
+  w.image = ws.bicg_image.p;
   return w;
 }
 
@@ -1141,7 +1147,9 @@ cudaError_t refine_bicgstab(Workspace& ws, int batch, const float2* D, const Blo
     add_iterations_kernel<<<(batch + 127) / 128, 128, 0, s>>>(batch, ws.bicg_iters.p, ws.bicg_total.p);
     return e != cudaSuccess ? e : cudaGetLastError();
   };
-  cudaError_t e = span(1, [&] {
+  cudaError_t e = bicg_row_scales(lay, batch, ws.M32.p, w, nullptr, s);
+  if (e != cudaSuccess) return e;
+  e = span(1, [&] {
     cudaError_t e1 = solve();
     launch_accumulate_correction(lay, batch, ws.M32.p, ws.rnorm.p, ws.X64.p, true, nullptr, nullptr, nullptr, s);
     return e1;
@@ -1448,6 +1456,9 @@ int solve_device_energies_enqueue(refeff_fms_plan& p, int E, const double2* d_k,
     RF_CUDA(ctx, ws.bicg_vec.alloc(size_t(kBicgVectors) * cols * ws.lay.lda));
     const int slices = std::max(bicg_slices(p.n, false), bicg_slices(p.n, ctx->bicg_tensor != 0));
     RF_CUDA(ctx, ws.bicg_part.alloc(size_t(slices - 1) * cols * ws.lay.lda));
+    RF_CUDA(ctx, ws.bicg_amax.alloc(size_t(ws.batch) * ws.lay.lda));
+    RF_CUDA(ctx, ws.bicg_xexp.alloc(bicg_exponents(p.n, p.m, ws.batch)));
+    RF_CUDA(ctx, ws.bicg_image.alloc(bicg_image_bytes(p.n, p.m, ws.batch)));
     RF_CUDA(ctx, ws.bicg_act.alloc(size_t(ws.batch)));
     RF_CUDA(ctx, ws.bicg_err.alloc(1));
     RF_CUDA(ctx, ws.bicg_sc.alloc(cols * kBicgScalars));
