@@ -205,26 +205,28 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(BatchLayout lay, i
 
 template <typename T, int NB, bool kSolve>
 __device__ __forceinline__ void rhs_lower_column(const BatchLayout& lay, int k, int kb, cplx<T>* colp, const LuWork& w,
-                                                 int b, const cplx<T> (*L11)[NB + 1], int lane) {
+                                                 int b, const cplx<T> (*L11)[NB + 1], int lane, int moves) {
   using C = cplx<T>;
   const int panel = k / NB;
-  const size_t pidx = size_t(b) * w.npanels + panel;
-  const int np = w.nperm[pidx];
-  const int2* pm = w.perm + pidx * (2 * NB);
-  constexpr int kMoves = (2 * NB + 31) / 32;
-  C v[kMoves];
-  int dst[kMoves];
+  for (int q = 0; q < moves; ++q) {
+    const size_t pidx = size_t(b) * w.npanels + panel + q;
+    const int np = w.nperm[pidx];
+    const int2* pm = w.perm + pidx * (2 * NB);
+    constexpr int kMoves = (2 * NB + 31) / 32;
+    C v[kMoves];
+    int dst[kMoves];
 #pragma unroll
-  for (int t = 0; t < kMoves; ++t) {
-    const int i = lane + 32 * t;
-    dst[t] = -1;
-    if (i < np) { const int2 mv = pm[i]; dst[t] = mv.x; v[t] = colp[mv.y]; }
+    for (int t = 0; t < kMoves; ++t) {
+      const int i = lane + 32 * t;
+      dst[t] = -1;
+      if (i < np) { const int2 mv = pm[i]; dst[t] = mv.x; v[t] = colp[mv.y]; }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < kMoves; ++t)
+      if (dst[t] >= 0) colp[dst[t]] = v[t];
+    __syncwarp();
   }
-  __syncwarp();
-#pragma unroll
-  for (int t = 0; t < kMoves; ++t)
-    if (dst[t] >= 0) colp[dst[t]] = v[t];
-  __syncwarp();
   if constexpr (!kSolve) return;
   constexpr int kRows = (NB + 31) / 32;
   C x[kRows];
@@ -257,12 +259,13 @@ __device__ __forceinline__ void rhs_lower_column(const BatchLayout& lay, int k, 
 
 // Columns [c_begin, c_end), kRhsColsPerWarp per warp (one after another, so
 // that each CTA reads L11 once for 8 * kRhsColsPerWarp columns): apply the
-// panel's row moves, then solve the panel rows with the unit lower L11.
+// row moves of `moves` panels from this one on, then solve the panel rows with
+// the unit lower L11.
 constexpr int kRhsColsPerWarp = 4;
 
 template <typename T, int NB, bool kSolve = true>
 __global__ void __launch_bounds__(256) rhs_lower_kernel(BatchLayout lay, int k, int c_begin, int c_end,
-                                                        cplx<T>* __restrict__ M, LuWork w, const int* skip) {
+                                                        cplx<T>* __restrict__ M, LuWork w, const int* skip, int moves) {
   using C = cplx<T>;
   const int b = blockIdx.y;
   if (skip && skip[b]) return;
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(256) rhs_lower_kernel(BatchLayout lay, int k, 
   for (int cw = 0; cw < kRhsColsPerWarp; ++cw) {
     const int col = first + cw * (blockDim.x / 32);
     if (col >= c_end) return;
-    rhs_lower_column<T, NB, kSolve>(lay, k, kb, Mb + size_t(lay.lda) * col, w, b, L11, lane);
+    rhs_lower_column<T, NB, kSolve>(lay, k, kb, Mb + size_t(lay.lda) * col, w, b, L11, lane, moves);
   }
 }
 // The outer block row of the two-level FP32 elimination as a product:
@@ -916,13 +919,13 @@ static cudaError_t launch_panel(const PanelConfig& pc, const BatchLayout& lay, i
 
 template <typename T, int NB, bool kSolve = true>
 static void launch_rhs_lower(const BatchLayout& lay, int batch, int k, int c_begin, int c_end, cplx<T>* M,
-                             const LuWork& w, const int* skip, cudaStream_t s) {
+                             const LuWork& w, const int* skip, cudaStream_t s, int moves = 1) {
   const int ncols = c_end - c_begin;
   if (ncols <= 0) return;
   const int per_cta = 8 * kRhsColsPerWarp;
   dim3 grid(unsigned((ncols + per_cta - 1) / per_cta), unsigned(batch));
   count_launch();
-  rhs_lower_kernel<T, NB, kSolve><<<grid, 256, 0, s>>>(lay, k, c_begin, c_end, M, w, skip);
+  rhs_lower_kernel<T, NB, kSolve><<<grid, 256, 0, s>>>(lay, k, c_begin, c_end, M, w, skip, moves);
 }
 
 // Composes the row moves of the P inner panels of an outer block into one
@@ -1006,15 +1009,15 @@ static void gemm_any(int nb, const BatchLayout& lay, int batch, int r_begin, int
 
 template <typename T, bool kSolve = true>
 static void rhs_lower_any(int nb, const BatchLayout& lay, int batch, int k, int c_begin, int c_end, cplx<T>* M,
-                          const LuWork& w, const int* skip, cudaStream_t s) {
+                          const LuWork& w, const int* skip, cudaStream_t s, int moves = 1) {
   if constexpr (sizeof(T) == 8) {
     static_assert(kSolve, "the FP64 panels have no inner panels whose moves go to earlier columns");
     launch_trsm64(false, lay, batch, k, min(nb, lay.n - k), c_begin, c_end, M, w, skip, s);
   } else {
     switch (nb) {
-      case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
-      case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
-      default: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+      case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
+      case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
+      default: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
     }
   }
 }
@@ -1175,7 +1178,10 @@ void lu_forward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cp
   const int n = lay.n, col_end = lay.n + lay.m;
   for (int k = 0; k < n; k += pc.nb) {
     const int kb = min(pc.nb, n - k);
-    rhs_lower_any<T>(pc.nb, lay, batch, k, n, col_end, M, w, skip, s);
+    // paired blocks: the second block's moves were also applied to the first one's L, so both come before the first
+    // solve (they only touch rows below the first block)
+    const int moves = !w.pair128 ? 1 : k / pc.nb % 2 ? 0 : k + pc.nb < n ? 2 : 1;
+    rhs_lower_any<T>(pc.nb, lay, batch, k, n, col_end, M, w, skip, s, moves);
     gemm_any<T>(pc.nb, lay, batch, k + kb, n, n, col_end, k, kb, M, skip, s);
   }
 }
@@ -1308,8 +1314,6 @@ template cudaError_t lu_eliminate<double>(const PanelConfig&, const BatchLayout&
                                           cudaStream_t);
 template cudaError_t lu_eliminate<float>(const PanelConfig&, const BatchLayout&, int, float2*, const LuWork&,
                                          cudaStream_t);
-template void lu_forward_rhs<double>(const PanelConfig&, const BatchLayout&, int, double2*, const LuWork&, const int*,
-                                     cudaStream_t);
 template void lu_forward_rhs<float>(const PanelConfig&, const BatchLayout&, int, float2*, const LuWork&, const int*,
                                     cudaStream_t);
 template void lu_backward_rhs<double>(const PanelConfig&, const BatchLayout&, int, double2*, const int*, cudaStream_t,

@@ -870,10 +870,9 @@ size_t bytes_per_system(const BatchLayout& lay, bool fp32) {
 }
 
 // Paired 64-column blocks (one K = 128 tensor-core update per pair) when the
-// tensor cores run the FP32 LU and the fused forward sweep replays its moves.
+// tensor cores run the FP32 LU.
 int want_pair128(const Workspace& ws) {
-  return ws.paired_pref && ws.fp32 && ws.use_tc && ws.pc32.inner_nb && fused_sweep_available(ws.pc32.nb, ws.lay)
-             ? 1 : 0;
+  return ws.paired_pref && ws.fp32 && ws.use_tc && ws.pc32.inner_nb ? 1 : 0;
 }
 
 int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, int batch, bool fp32,

@@ -279,19 +279,6 @@ bool fused_forward_sweep(int nb, const BatchLayout& lay, int batch, float2* M, c
   return false;
 }
 
-bool fused_sweep_available(int nb, const BatchLayout& lay) {
-  const int need = lay.m < 4 ? lay.m : 4;  // the narrowest column group launch_sweep_cg accepts
-  if (nb == 64) return SweepSmem<64, 8>::bytes(lay.n) <= kSwSmemBudget ||
-                       (need <= 4 && SweepSmem<64, 4>::bytes(lay.n) <= kSwSmemBudget) ||
-                       (need <= 2 && SweepSmem<64, 2>::bytes(lay.n) <= kSwSmemBudget) ||
-                       (need <= 1 && SweepSmem<64, 1>::bytes(lay.n) <= kSwSmemBudget);
-  if (nb == 32) return SweepSmem<32, 8>::bytes(lay.n) <= kSwSmemBudget ||
-                       (need <= 4 && SweepSmem<32, 4>::bytes(lay.n) <= kSwSmemBudget) ||
-                       (need <= 2 && SweepSmem<32, 2>::bytes(lay.n) <= kSwSmemBudget) ||
-                       (need <= 1 && SweepSmem<32, 1>::bytes(lay.n) <= kSwSmemBudget);
-  return false;
-}
-
 bool fused_backward_sweep(int nb, const BatchLayout& lay, int batch, float2* M, const int* skip, cudaStream_t s) {
   if (nb == 64) return launch_sweep_nb<64>(false, lay, batch, M, nullptr, skip, s);
   if (nb == 32) return launch_sweep_nb<32>(false, lay, batch, M, nullptr, skip, s);
