@@ -655,8 +655,8 @@ def ours(args, world, rank, local):
                 "algorithmic_bytes_per_launch": c_bytes / max(tc_launches, 1),
                 "launches": tc_launches, "launch_ms_avg": tc_ms / max(tc_launches, 1),
                 "tensor_view": {"achieved": tc_tf, "unit": "TFLOP/s", "peak": bf16, "frac": tc_tf / bf16,
-                                "note": "useful complex-FP32 flops; split TF32 issues 3 tensor products per useful "
-                                        "one at a TF32 rate half the bf16 peak (useful ceiling ~1/6 of it)"},
+                                "note": "useful complex-FP32 flops; the two-term FP16 split issues 3 tensor products "
+                                        "per useful one at the bf16 rate (useful ceiling ~1/3 of the peak)"},
                 "traffic_note": (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of {tr['captured']} over their "
                                  "algorithmic C bytes, times this sweep's algorithmic bytes per launch "
                                  "(profiles/ncu_traffic.json)" if tr else "no ncu record"),

@@ -106,9 +106,10 @@ unsigned long long refeff_fms_kernel_launches(void);
 
 /* Context options; they apply to plans created and dense solves started
  * after the call.
- *   REFEFF_FMS_OPT_TENSOR_CORES: 1 (default) runs the trailing updates of the
- *     FP32 LU on the tcgen05 tensor cores (split TF32, FP32 accumulation);
- *     0 runs them on the CUDA cores.
+ *   REFEFF_FMS_OPT_TENSOR_CORES: 1 (default) runs the block updates of the LU
+ *     on the tcgen05 tensor cores: FP32 values as two FP16 terms with FP32
+ *     accumulation, FP64 values as eight 8-bit digits whose products are summed
+ *     exactly; 0 runs them on the CUDA cores.
  *   REFEFF_FMS_OPT_DENSE_REFINEMENT: corrections allowed in
  *     refeff_complex_lu_solve_batched with REFEFF_FMS_FORM_FP32_REFINED
  *     (default 10; 0 returns the plain FP32 LU solution, flagged NOT_CONVERGED).
@@ -118,7 +119,10 @@ unsigned long long refeff_fms_kernel_launches(void);
  *     gives up marks the call's tensor-core result void and every energy of
  *     the call is solved again with the FP64 LU (status 0, same results as
  *     REFEFF_FMS_FORM_FP64_LU; refeff_fms_last_error names the timeout).
- *     Applies from the next solve call of every plan of the context.
+ *     Applies from the next solve call of every plan of the context.  The FP64
+ *     updates of the dense solves take the same budget; a CTA of theirs whose
+ *     wait gives up finishes its tiles on the FP64 pipe inside the kernel, so
+ *     the call still succeeds.
  *   REFEFF_FMS_OPT_PAIRED_BLOCKS: 1 (default) lets the FP32 LU on the tensor
  *     cores take its 64-column blocks in pairs, with one K = 128 trailing
  *     update per pair (half the trailing-matrix traffic); 0 updates after

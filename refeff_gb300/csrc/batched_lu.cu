@@ -4,17 +4,19 @@
 // the factors (crates/refeff-linalg/src/lu.rs:400-529 solve semantics).
 //
 // One elimination step k (panel width NB):
-//   panel_kernel      the (n-k) x NB panel lives in the distributed shared
-//                     memory of a thread-block cluster (rows split across the
-//                     CTAs); one cluster barrier per column: local arg-max,
-//                     cluster arg-max over DSMEM, pivot row read over DSMEM,
-//                     rank-1 update of the CTA's own rows.  Rows are not moved
-//                     while the panel is factored; the permutation is applied
-//                     when the panel is written back, and its row moves are
-//                     stored per panel.
-//   rhs_lower_kernel  applies the panel's row moves to the trailing columns and
-//                     solves U12 = L11^-1 A12 (one warp per column).
-//   gemm_update       A22 -= L21 U12 on the trailing block (B included).
+//   panel      the (n-k) x NB panel, its rows split across the CTAs of a
+//              thread-block cluster; rows are not moved while it is factored,
+//              the permutation is applied when the panel is written back, and
+//              its row moves are stored per panel.  FP64: panel64.cu.  FP32:
+//              panel32.cu, rows in registers; panel_kernel here, rows in
+//              shared memory, where a CTA has more rows than that serves.
+//   block row  the panel's row moves on the trailing columns and U12 = L11^-1
+//              A12.  FP64: trsm64.cu.  FP32: rhs_lower_kernel (one warp per
+//              column) inside a 64-column block, rhs_lower_tile_kernel (a
+//              product with the inverse of L11) for the block itself.
+//   update     A22 -= L21 U12 on the trailing block (B included), on the
+//              tensor cores (tc_update64.cu, tc_update.cu); gemm_update_kernel
+//              here inside the FP32 blocks, and without the tensor cores.
 // Columns left of the panel are never permuted.  A later forward sweep
 // applies each panel's moves to the new right-hand side just before that
 // panel's L columns, which is the same permutation order the elimination saw.
@@ -1022,7 +1024,8 @@ static void rhs_lower_any(int nb, const BatchLayout& lay, int batch, int k, int 
   }
 }
 
-// Cluster panel of width nb: FP32 uses 32 / 16, FP64 32 / 16 / 8.
+// Cluster panel of width nb: FP32 uses 32 / 16, FP64 32 / 16 / 8 (dispatch above: a CTA of panel32.cu holds 512 or 1024
+// rows of 32 or 16 columns).
 template <typename T>
 static cudaError_t panel_any(const PanelConfig& pc, int nb, const BatchLayout& lay, int batch, int k, cplx<T>* M,
                              const LuWork& w, cudaStream_t s) {
