@@ -15,7 +15,6 @@
 //   v = A p^;  alpha = rho_new / (r~, v);   s = r - alpha v;  s^ = D s
 //   t = A s^;  omega = (t, s) / (t, t);     x += alpha p^ + omega s^;  r = s - omega t
 //   rho_new = (r~, r);  stop when |r| <= tol |b|.
-#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -350,8 +349,8 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 // split into two TF32 values, for entries down to 2^-17 of the largest, an
 // absolute error of 2^-40 of the largest below.  A CTA takes 128 rows and a
 // slice of the columns, in slabs of 16 columns:
-//   warp 5      copies, three or four slabs ahead: 16 columns of 128 rows of A
-//               as one box of a tensor map, and the slab of X's operand;
+//   warp 5      bulk copies, three slabs ahead: 16 columns of 128 rows of A
+//               (1 KB each) and the slab of X's operand;
 //   warps 0-3   a row of A each thread: 16 entries from shared memory, scaled
 //               and split into the four real planes (re hi, re lo, im hi,
 //               im lo) in the K-major 32-byte-swizzled UMMA layout (two
@@ -367,13 +366,12 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 // bounded; a timeout sets *err (the solve then hands its matrices to the LU)
 // and the CTA drains its copies and MMAs and frees its tensor memory before it
 // returns.
-// Bound by HBM (A is read once).  The form at n = 4112, 12 matrices, 16 columns
-// (576 products and the vector kernels): 71.2 ms; with a bulk copy of 1 KB for
-// each column of a slab instead of the box 81.6, where twice the row warps,
-// another ring stage or 1024-column slices changed nothing: the copies' issue
-// bound it (1.65 GB in 346 us under a profiler); FP16 terms with loads in
-// registers and 256-column slices 92.8; split by the row's thread into two TF32
-// terms, 12 MMAs a slab, 101.9.
+// Bound by HBM and the row threads' conversions: n = 4112, 12 matrices, 16
+// columns 346 us under a profiler (1.65 GB read at 62% of the HBM peak); a split
+// into two TF32 terms by the row's thread, loads in registers, the operand of X
+// converted by every CTA and 12 MMAs a slab took 460 us.  Slices of 256 columns
+// instead of 512 and register loads with FP16 terms: 400 us.  A ring of three or
+// of four slabs: the same.
 constexpr int kTcRows = 128, kTcK = 16, kTcThreads = 192, kTcStages = 2, kTcSub = 256;
 constexpr long long kTcBicgPolls = 1LL << 26;  // poll budget of each wait (about 1 s is the other bound)
 constexpr int kTcAPlane = kTcRows * 32;             // 4 KB: 128 rows of 16 FP16 values
@@ -430,13 +428,6 @@ __device__ __forceinline__ void tc_bulk(uint32_t dst, const void* src, uint32_t 
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
-}
-// the box of the tensor map at (x, y, z), x a multiple of four floats
-__device__ __forceinline__ void tc_box(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -495,9 +486,9 @@ __global__ void __launch_bounds__(128) bicg_row_max_kernel(View w, const float2*
 }
 
 template <int N, bool k3M>
-__global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, const __grid_constant__ CUtensorMap amap,
-                                                                        int dst, int kchunk, const int* skip, int* err,
-                                                                        long long polls) {
+__global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, const float2* __restrict__ M32,
+                                                                     size_t stride, int dst, int kchunk,
+                                                                     const int* skip, int* err, long long polls) {
   using L = TcMv<N, k3M>;
   constexpr int kMaxSubs = kBicgTcSliceCols / kTcSub;
   const int b = w.matrix();
@@ -703,16 +694,23 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
       tc_drain(bar(kDrain), 0u, polls);
     }
   } else if (warp == 5) {
-    // ---- copies ----
+    // ---- copies: lane q brings column q of the slab, lane 16 the X operand ----
+    const uint32_t col_bytes = uint32_t(min(kTcRows, w.lda - r0)) * 8u;
+    const float2* A = M32 + size_t(b) * stride + r0;
     const uint8_t* X = w.image + (size_t(b) * ((n + kTcK - 1) / kTcK) + kbeg / kTcK) * L::kB;
     int rs = 0, sl = 0;
     uint32_t rph = 0;
-    for (; sl < slabs && lane == 0; ++sl) {
-      if (!tc_wait(bar(kREmpty + rs), rph ^ 1u, abort_flag, err, polls)) break;
+    for (; sl < slabs; ++sl) {
+      int ok = 1;
+      if (lane == 0) ok = tc_wait(bar(kREmpty + rs), rph ^ 1u, abort_flag, err, polls);
+      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+      const int k0 = kbeg + sl * kTcK, cols = min(kTcK, kend - k0);
       const uint32_t dstA = sbase + uint32_t(kRingBase + rs * L::kRing);
-      tc_bar_expect(bar(kRFull + rs), uint32_t(L::kRing));
-      tc_box(dstA, &amap, 2 * r0, kbeg + sl * kTcK, b, bar(kRFull + rs));
-      tc_bulk(dstA + uint32_t(kTcRaw), X + size_t(sl) * L::kB, uint32_t(L::kB), bar(kRFull + rs));
+      if (lane == 0) tc_bar_expect(bar(kRFull + rs), uint32_t(cols) * col_bytes + uint32_t(L::kB));
+      __syncwarp();
+      if (lane < cols)
+        tc_bulk(dstA + uint32_t(lane * kTcRows * 8), A + size_t(w.lda) * (k0 + lane), col_bytes, bar(kRFull + rs));
+      if (lane == kTcK) tc_bulk(dstA + uint32_t(kTcRaw), X + size_t(sl) * L::kB, uint32_t(L::kB), bar(kRFull + rs));
       if (++rs == kTcRing) {
         rs = 0;
         rph ^= 1u;
@@ -977,24 +975,6 @@ __global__ void bicg_finish_kernel(View w, float2* __restrict__ M32, size_t stri
 
 }  // namespace
 
-// The batch's systems as (2 lda floats, n + m columns, batch), boxes of 128 rows x kTcK columns.
-static bool system_map(const BatchLayout& lay, int batch, const float2* M32, CUtensorMap& map) {
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult found;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-      found != cudaDriverEntryPointSuccess || !fn) {
-    cudaGetLastError();
-    return false;
-  }
-  const cuuint64_t dim[3] = {cuuint64_t(2) * lay.lda, cuuint64_t(lay.n) + lay.m, cuuint64_t(batch)};
-  const cuuint64_t pitch[2] = {cuuint64_t(lay.lda) * sizeof(float2), cuuint64_t(lay.stride) * sizeof(float2)};
-  const cuuint32_t box[3] = {2 * kTcRows, kTcK, 1}, step[3] = {1, 1, 1};
-  return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(fn)(
-             &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float2*>(M32), dim, pitch, box, step,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 int bicg_slices(int n, bool tensor, int* chunk) {
   int c = tensor ? kBicgTcSliceCols
                  : std::max(kMvSliceCols, ((n + kBicgMaxSplit - 1) / kBicgMaxSplit + kMvK - 1) / kMvK * kMvK);
@@ -1032,9 +1012,7 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
     if (e != cudaSuccess) return e;
   }
   // the tensor-core product for up to 32 right-hand sides (N = 16 or 32 accumulator columns)
-  CUtensorMap amap{};
-  const bool tensor = w.tensor && w.tc_err && lay.m <= 32 && (w.part || lay.n <= kBicgTcSliceCols) &&
-                      system_map(lay, batch, M32, amap);
+  const bool tensor = w.tensor && w.tc_err && lay.m <= 32 && (w.part || lay.n <= kBicgTcSliceCols);
   const bool n16 = lay.m <= 16, three = w.tensor == 2;
   if (tensor) {
     v.amax = w.amax;
@@ -1048,7 +1026,7 @@ cudaError_t bicgstab_solve(const BatchLayout& lay, int batch, float2* M32, const
   auto tc_launch = [&](auto kN, auto k3, const dim3& grid, const View& view, int dst, int chunk) {
     constexpr int N = decltype(kN)::value;
     constexpr bool M3 = decltype(k3)::value;
-    bicg_tc_matvec_kernel<N, M3><<<grid, kTcThreads, TcMv<N, M3>::kSmem, s>>>(view, amap, dst, chunk, skip,
+    bicg_tc_matvec_kernel<N, M3><<<grid, kTcThreads, TcMv<N, M3>::kSmem, s>>>(view, M32, lay.stride, dst, chunk, skip,
                                                                               w.tc_err, kTcBicgPolls);
   };
   auto tc_attr = [&](auto kN, auto k3) {
