@@ -349,12 +349,11 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 // split into two TF32 values, for entries down to 2^-17 of the largest, an
 // absolute error of 2^-40 of the largest below.  A CTA takes 128 rows and a
 // slice of the columns, in slabs of 16 columns:
-//   warp 5      bulk copies, three slabs ahead: 16 columns of 128 rows of A
-//               (1 KB each) and the slab of X's operand;
-//   warps 0-3   a row of A each thread: 16 entries from shared memory, scaled
-//               and split into the four real planes (re hi, re lo, im hi,
-//               im lo) in the K-major 32-byte-swizzled UMMA layout (two
-//               stages);
+//   warp 5      bulk copies of X's operand, three or four slabs ahead;
+//   warps 0-3   32 rows of A each, by cp.async as far ahead; a row a thread, 16
+//               entries from shared memory, scaled and split into the four
+//               real planes (re hi, re lo, im hi, im lo) in the K-major
+//               32-byte-swizzled UMMA layout (two stages);
 //   warp 4      one thread issues 4 MMAs a slab,
 //     Ar hi x [Xr | Xi] hi, lo and Ai hi x [-Xi | Xr] hi, lo   (4N columns)
 //     Ar lo x [Xr | Xi] hi     and Ai lo x [-Xi | Xr] hi       (2N columns)
@@ -366,12 +365,12 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 // bounded; a timeout sets *err (the solve then hands its matrices to the LU)
 // and the CTA drains its copies and MMAs and frees its tensor memory before it
 // returns.
-// Bound by HBM and the row threads' conversions: n = 4112, 12 matrices, 16
-// columns 346 us under a profiler (1.65 GB read at 62% of the HBM peak); a split
-// into two TF32 terms by the row's thread, loads in registers, the operand of X
-// converted by every CTA and 12 MMAs a slab took 460 us.  Slices of 256 columns
-// instead of 512 and register loads with FP16 terms: 400 us.  A ring of three or
-// of four slabs: the same.
+// Bound by HBM (A is read once).  The form at n = 4112, 12 matrices, 16 columns
+// (576 products and the vector kernels): 73.4 ms; with A in bulk copies of 1 KB,
+// one a column of a slab, 81.5, bound by their issue (1.65 GB in 346 us under a
+// profiler; another ring stage, twice the row warps or 1024-column slices
+// changed nothing); FP16 terms with loads in registers and 256-column slices
+// 92.8; split by the row's thread into two TF32 terms, 12 MMAs a slab, 101.9.
 constexpr int kTcRows = 128, kTcK = 16, kTcThreads = 192, kTcStages = 2, kTcSub = 256;
 constexpr long long kTcBicgPolls = 1LL << 26;  // poll budget of each wait (about 1 s is the other bound)
 constexpr int kTcAPlane = kTcRows * 32;             // 4 KB: 128 rows of 16 FP16 values
@@ -505,7 +504,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
   uint8_t* const gbase = tsm + (sbase - raw);  // [kTcStages] planes, [kTcRing] (A as stored, X operand)
   constexpr int kTcRing = L::kDepth, kRingBase = kTcStages * L::kA;
   uint8_t* const meta = gbase + kRingBase + kTcRing * L::kRing;
-  // barriers: planes full[2] (4 warps) and empty[2] (commit); ring full[] (copies) and empty[] (4 warps, commit);
+  // barriers: planes full[2] (4 warps) and empty[2] (commit); X full[] (copy) and empty[] (commit);
   // accumulators (commit); drain (commit)
   auto bar = [&](int i) { return tc_smem_u32(meta + 8 * i); };
   constexpr int kFull = 0, kEmpty = kTcStages, kRFull = 2 * kTcStages, kREmpty = kRFull + kTcRing,
@@ -526,7 +525,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
     }
     for (int i = 0; i < kTcRing; ++i) {
       tc_bar_init(bar(kRFull + i), 1);
-      tc_bar_init(bar(kREmpty + i), 5);
+      tc_bar_init(bar(kREmpty + i), 1);
     }
     tc_bar_init(bar(kAcc), 1);
     tc_bar_init(bar(kDrain), 1);
@@ -560,13 +559,33 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
     float2 y[N];
 #pragma unroll
     for (int c = 0; c < N; ++c) y[c] = make_float2(0.f, 0.f);
+    // a slab of the warp's 32 rows: lanes 0-15 the row pairs of its even columns, 16-31 of its odd ones; zeros past the
+    // matrix's columns and rows.  Only this warp reads them.
+    const int prow = r0 + warp * 32 + 2 * (lane & 15), pcol = lane >> 4;
+    const float2* const ap = M32 + size_t(b) * stride + (prow < w.lda ? prow : 0);
+    auto fetch = [&](int sl) {
+      if (sl < slabs) {
+        const int k0 = kbeg + sl * kTcK;
+        float2* to = reinterpret_cast<float2*>(gbase + kRingBase + (sl % kTcRing) * L::kRing) + (prow - r0);
+#pragma unroll
+        for (int q = 0; q < kTcK / 2; ++q) {
+          const int col = 2 * q + pcol;
+          const bool in = k0 + col < kend && prow < w.lda;
+          cp_async16(to + col * kTcRows, in ? ap + size_t(w.lda) * (k0 + col) : ap, in ? 16 : 0);
+        }
+      }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int sl = 0; sl < kTcRing - 1; ++sl) fetch(sl);
     bool ok = true;
-    int rs = 0;           // ring stage and its phase
-    uint32_t rph = 0;
+    int rs = 0;  // ring stage
     for (int sl = 0; sl < slabs; ++sl) {
       const int st = sl & 1;
-      ok = tc_wait(bar(kRFull + rs), rph, abort_flag, err, polls);
-      ok = ok && tc_wait(bar(kEmpty + st), uint32_t((sl >> 1) & 1) ^ 1u, abort_flag, err, polls);  // MMAs of slab sl - 2
+      fetch(sl + kTcRing - 1);  // into the stage that slab sl - 1 has left
+      cp_async_wait<kTcRing - 1>();
+      __syncwarp();
+      ok = tc_wait(bar(kEmpty + st), uint32_t((sl >> 1) & 1) ^ 1u, abort_flag, err, polls);  // the MMAs of slab sl - 2
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
         break;
@@ -575,12 +594,6 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
       float2 v[kTcK];
 #pragma unroll
       for (int kk = 0; kk < kTcK; ++kk) v[kk] = ra[kk * kTcRows];
-      const int left = kend - (kbeg + sl * kTcK);
-      if (left < kTcK) {  // the matrix's last slab: columns that were not copied
-#pragma unroll
-        for (int kk = 0; kk < kTcK; ++kk)
-          if (kk >= left) v[kk] = make_float2(0.f, 0.f);
-      }
       uint8_t* const sA = gbase + st * L::kA;
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
@@ -600,14 +613,8 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the planes are read by the tensor cores
       __syncwarp();
-      if (lane == 0) {
-        tc_bar_arrive(bar(kFull + st));
-        tc_bar_arrive(bar(kREmpty + rs));
-      }
-      if (++rs == kTcRing) {
-        rs = 0;
-        rph ^= 1u;
-      }
+      if (lane == 0) tc_bar_arrive(bar(kFull + st));
+      if (++rs == kTcRing) rs = 0;
       if ((sl + 1) % kSubSlabs == 0 || sl + 1 == slabs) {
         // ---- the accumulators of these columns ----
         const int sub = sl / kSubSlabs;
@@ -650,6 +657,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");  // the next slab's MMAs overwrite them
       }
     }
+    cp_async_wait<0>();  // no copy outlives the CTA
     if (ok && row_ok) {
 #pragma unroll
       for (int c = 0; c < N; ++c)
@@ -659,10 +667,11 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
     // ---- MMA issuer ----
     bool issued = false, ok = true;
     int rs = 0;
+    uint32_t rph = 0;
     for (int sl = 0; sl < slabs; ++sl) {
       const int st = sl & 1;
-      // the planes; their warps have waited for the slab's copies
-      ok = tc_wait(bar(kFull + st), uint32_t((sl >> 1) & 1), abort_flag, err, polls);
+      ok = tc_wait(bar(kRFull + rs), rph, abort_flag, err, polls) &&                          // the slab of X
+           tc_wait(bar(kFull + st), uint32_t((sl >> 1) & 1), abort_flag, err, polls);  // the planes
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t sA = sbase + uint32_t(st * L::kA), sB = sbase + uint32_t(kRingBase + rs * L::kRing + kTcRaw);
@@ -686,7 +695,10 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
       tc_commit(bar(kEmpty + st));   // the planes and
       tc_commit(bar(kREmpty + rs));  // the ring stage are free once these MMAs have read them
       if ((sl + 1) % kSubSlabs == 0 || sl + 1 == slabs) tc_commit(bar(kAcc));
-      if (++rs == kTcRing) rs = 0;
+      if (++rs == kTcRing) {
+        rs = 0;
+        rph ^= 1u;
+      }
     }
     if (issued) {
       // every MMA of this CTA has completed before the tensor memory is freed
@@ -694,23 +706,15 @@ __global__ void __launch_bounds__(kTcThreads, 2) bicg_tc_matvec_kernel(View w, c
       tc_drain(bar(kDrain), 0u, polls);
     }
   } else if (warp == 5) {
-    // ---- copies: lane q brings column q of the slab, lane 16 the X operand ----
-    const uint32_t col_bytes = uint32_t(min(kTcRows, w.lda - r0)) * 8u;
-    const float2* A = M32 + size_t(b) * stride + r0;
+    // ---- copies of X's operand ----
     const uint8_t* X = w.image + (size_t(b) * ((n + kTcK - 1) / kTcK) + kbeg / kTcK) * L::kB;
     int rs = 0, sl = 0;
     uint32_t rph = 0;
-    for (; sl < slabs; ++sl) {
-      int ok = 1;
-      if (lane == 0) ok = tc_wait(bar(kREmpty + rs), rph ^ 1u, abort_flag, err, polls);
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-      const int k0 = kbeg + sl * kTcK, cols = min(kTcK, kend - k0);
-      const uint32_t dstA = sbase + uint32_t(kRingBase + rs * L::kRing);
-      if (lane == 0) tc_bar_expect(bar(kRFull + rs), uint32_t(cols) * col_bytes + uint32_t(L::kB));
-      __syncwarp();
-      if (lane < cols)
-        tc_bulk(dstA + uint32_t(lane * kTcRows * 8), A + size_t(w.lda) * (k0 + lane), col_bytes, bar(kRFull + rs));
-      if (lane == kTcK) tc_bulk(dstA + uint32_t(kTcRaw), X + size_t(sl) * L::kB, uint32_t(L::kB), bar(kRFull + rs));
+    for (; sl < slabs && lane == 0; ++sl) {
+      if (!tc_wait(bar(kREmpty + rs), rph ^ 1u, abort_flag, err, polls)) break;
+      tc_bar_expect(bar(kRFull + rs), uint32_t(L::kB));
+      tc_bulk(sbase + uint32_t(kRingBase + rs * L::kRing + kTcRaw), X + size_t(sl) * L::kB, uint32_t(L::kB),
+              bar(kRFull + rs));
       if (++rs == kTcRing) {
         rs = 0;
         rph ^= 1u;
