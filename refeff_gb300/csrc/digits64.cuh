@@ -46,41 +46,48 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
-// v 2^ex rounded to FP64 in integer operations: the conversion instruction runs on the FP64 pipe, where a warp's
-// instruction takes 64 cycles of its quarter of the SM.
-__device__ __forceinline__ double scaled_double(long long v, int ex) {
-  if (v == 0) return 0.0;
+// v 2^ex rounded to FP64 in integer operations, for results in the normal range (or zero): the conversion instruction
+// runs on the FP64 pipe, where a warp's instruction takes 64 cycles of its quarter of the SM.
+__device__ __forceinline__ double normal_double(long long v, int ex) {
   const uint32_t sign = uint32_t(static_cast<unsigned long long>(v) >> 32) & 0x80000000u;
   const unsigned long long a = static_cast<unsigned long long>(v < 0 ? -v : v);
-  const int lz = __clzll(static_cast<long long>(a));
+  const int lz = __clzll(static_cast<long long>(a | 1));
   const unsigned long long m = a << lz;  // leading one at bit 63
-  const int field = 1023 + 63 - lz + ex;
-  if (field > 0 && field < 2046) {
-    // 53 bits, rounded half up; a carry out of the mantissa moves into the exponent as it should
-    const unsigned long long bits = (m >> 11) + ((m >> 10) & 1) + (static_cast<unsigned long long>(field - 1) << 52);
-    return __hiloint2double(int(uint32_t(bits >> 32) | sign), int(uint32_t(bits)));
-  }
-  return scalbn(__ll2double_rn(v), ex);
+  // 53 bits, rounded half up; a carry out of the mantissa moves into the exponent as it should
+  const unsigned long long bits = (m >> 11) + ((m >> 10) & 1) + (static_cast<unsigned long long>(1023 + 62 - lz + ex) << 52);
+  return v == 0 ? 0.0 : __hiloint2double(int(uint32_t(bits >> 32) | sign), int(uint32_t(bits)));
+}
+constexpr int kSafeExp = 900;  // sums of grids 2^e, |e| <= kSafeExp, are normal numbers
+__device__ __forceinline__ double scaled_double(long long v, int ex) {
+  return ex >= -kSafeExp && ex <= kSafeExp ? normal_double(v, ex) : scalbn(__ll2double_rn(v), ex);
 }
 
 // The eight exact level sums of one real output (levels 2 .. 9, weights 2^-12 .. 2^-68 of 2^e, bit patterns of
-// integer-valued floats) as an FP64 number.  Integers up to 2^22 are read off the mantissa after adding 1.5 x 2^23;
-// kWide (more than 16 products per pair, K > 8): levels 7 and 8 can exceed that and are converted, level 9 may then be
-// off by one unit of 2^-68.
+// integer-valued floats) as an integer in units of 2^unit of 2^e: 2^-56, or 2^-68 where the sum lies below 2^-7 (the
+// sum's grid is finer than FP64's there).  Integers up to 2^22 are read off the mantissa after adding 1.5 x 2^23, which
+// holds for the levels 2 .. 6 at K = 32 (the first digit is at most 64).  kWide (K > 8): levels 7 and 8 can exceed that
+// and are converted; level 9, up to 7/8 of 2^23, is read after adding 1.5 x 2^24, to an even integer.
 template <bool kWide>
-__device__ __forceinline__ double join_levels(const uint32_t* s, int e) {
-  constexpr int kBase = 0x4B400000;  // the pattern of 1.5 x 2^23
-  auto pat = [&](int i) { return __float_as_int(__uint_as_float(s[i]) + 12582912.0f); };
-  auto sum = [&](int i) { return kWide ? __float2int_rn(__uint_as_float(s[i])) : pat(i) - kBase; };
-  const int p = pat(0) * 256 + pat(1) - int(257u * uint32_t(kBase));
-  const int q = pat(2) * 256 + pat(3) - int(257u * uint32_t(kBase));
-  const int r = (pat(4) - kBase) * 256 + sum(5);
-  const int l = sum(6) * 256 + (pat(7) - kBase);
-  // h = the levels 2 .. 7 in units of 2^-52: |h| < 2^59; l holds levels 8 and 9, 16 bits further down
-  const long long h = (static_cast<long long>(p) * 4294967296LL) + static_cast<long long>(q) * 65536 + r;
-  const bool small = ((h + (1ll << 45)) >> 46) == 0;
-  const long long v = small ? h * 65536 + l : h + ((l + 32768) >> 16);
-  return scaled_double(v, e - (small ? 68 : 52));
+__device__ __forceinline__ long long join_levels(const uint32_t* s, int& unit) {
+  constexpr uint32_t kBase = 0x4B400000u, kBase9 = 0x4BC00000u;  // the patterns of 1.5 x 2^23 and 1.5 x 2^24
+  auto pat = [&](int i) { return __float_as_uint(__uint_as_float(s[i]) + 12582912.0f); };
+  auto sum = [&](int i) { return kWide ? __float2int_rn(__uint_as_float(s[i])) : int(pat(i) - kBase); };
+  const int p = int(pat(0) * 256u + pat(1) - 257u * kBase);
+  const int q = int(pat(2) * 256u + pat(3) - 257u * kBase);
+  const int r = int(pat(4) - kBase) * 256 + sum(5);
+  const int l9 = kWide ? 2 * int(__float_as_uint(__uint_as_float(s[7]) + 25165824.0f) - kBase9) : int(pat(7) - kBase);
+  const int l = sum(6) * 256 + l9;
+  // h = the levels 2 .. 7 in units of 2^-56: |h| < 2^63; l holds levels 8 and 9, 12 bits further down
+  const long long h = static_cast<long long>(p) * (1ll << 36) + static_cast<long long>(q) * (1 << 20) + static_cast<long long>(r) * 16;
+  const bool small = uint32_t(static_cast<unsigned long long>(h) >> 32) + (1u << 17) < (1u << 18);  // |h| < 2^49
+  unit = small ? -68 : -56;
+  return small ? h * 4096 + l : h + ((l + 2048) >> 12);
+}
+template <bool kWide>
+__device__ __forceinline__ double join_double(const uint32_t* s, int e) {
+  int unit;
+  const long long v = join_levels<kWide>(s, unit);
+  return scaled_double(v, e + unit);
 }
 
 // ---------------------------------------------------------------------------
@@ -191,7 +198,7 @@ __device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t
         li[s] = __float_as_uint(ci[s][2 * h + q]);
       }
       const int e = a.e[h] + ecol[2 * t + q];
-      p[h][q] = make_double2(join_levels<false>(lr, e), join_levels<false>(li, e));
+      p[h][q] = make_double2(join_double<false>(lr, e), join_double<false>(li, e));
     }
 }
 

@@ -44,7 +44,8 @@
 // Every wait on an mbarrier is bounded.  A CTA whose waits ran out drains its
 // copies and MMAs, and its epilogue warps finish their remaining tiles with
 // FP64 multiply-adds from the matrix, so the update is complete in any case;
-// rows and columns that hold an infinity or NaN take the same path.
+// rows and columns that hold an infinity or NaN, or whose products lie near the
+// ends of the FP64 range, take the same path.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = 0; j < 4; ++j) cn[j] = j < have ? cur[size_t(lda) * j] : make_double2(0.0, 0.0);
     }
     while (more) {
-      const int er = rexp[(size_t(t.b) * nbm_all + t.bm) * kRows + quarter * 32 + lane];
+      int er = rexp[(size_t(t.b) * nbm_all + t.bm) * kRows + quarter * 32 + lane];
       const int4 ec4 = *reinterpret_cast<const int4*>(cexp + (size_t(t.b) * nbn_all + t.bn) * kCols + 4 * g);
       const int ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w};
       const int tb = t.b, tcol = c_begin + t.bn * kCols + 4 * g, trow = r_begin + t.bm * kRows + quarter * 32 + lane;
@@ -466,6 +467,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const bool ready = role_wait(bar(kAccFull + int(buf)), (tiles >> 1) & 1, abort_flag, polls);
         direct = !__all_sync(0xffffffffu, ready);
       }
+      if (direct) er = kNonfinite;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // one column at a time: the level sums of more would not fit in registers beside C, and C spilled to local
       // memory stalls on its own loads (4 us a tile)
@@ -494,11 +496,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (c < have) {
           double2 p;
-          if (direct || er == kNonfinite || ec[c] == kNonfinite) {
+          const int e = er + ec[c];  // kNonfinite or more with an infinity or NaN, or where the waits ran out
+          if (unsigned(e + kSafeExp) <= 2u * kSafeExp) {
+            int ur, ui;
+            const long long vr = join_levels<true>(lv, ur), vi = join_levels<true>(lv + kDig, ui);
+            p = make_double2(normal_double(vr, e + ur), normal_double(vi, e + ui));
+          } else {
             const double2* Mb = M + size_t(tb) * lay.stride;
             p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
-          } else {
-            p = make_double2(join_levels<true>(lv, er + ec[c]), join_levels<true>(lv + kDig, er + ec[c]));
           }
           cur[size_t(lda) * c] = make_double2(cn[c].x - p.x, cn[c].y - p.y);
         }
