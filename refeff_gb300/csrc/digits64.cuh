@@ -62,11 +62,20 @@ __device__ __forceinline__ double scaled_double(long long v, int ex) {
   return ex >= -kSafeExp && ex <= kSafeExp ? normal_double(v, ex) : scalbn(__ll2double_rn(v), ex);
 }
 
+// The grid's errors weigh some 2^-57 of 2^e in a sum of up to 32 complex products.  A sum below 2^(e - kWeak) beside a
+// C below that may therefore have lost its terms; they are sound if the largest of them reaches 2^(e - kLost): the
+// errors are then below 2^-49 of it, what the rounding of such a sum may come to.
+constexpr int kWeak = 7, kLost = 6;
+// both parts below 2^e (infinities and NaN are not)
+__device__ __forceinline__ bool below(double2 v, int e) { return max(field_of(v.x), field_of(v.y)) < e + 1023; }
+
 // The eight exact level sums of one real output (levels 2 .. 9, weights 2^-12 .. 2^-68 of 2^e, bit patterns of
 // integer-valued floats) as an integer in units of 2^unit of 2^e: 2^-56, or 2^-68 where the sum lies below 2^-7 (the
 // sum's grid is finer than FP64's there).  Integers up to 2^22 are read off the mantissa after adding 1.5 x 2^23, which
 // holds for the levels 2 .. 6 at K = 32 (the first digit is at most 64).  kWide (K > 8): levels 7 and 8 can exceed that
-// and are converted; level 9, up to 7/8 of 2^23, is read after adding 1.5 x 2^24, to an even integer.
+// and are converted; level 9, up to 7/8 of 2^23, is read after adding 1.5 x 2^24, to an even integer.  The sum lies below
+// 2^-kWeak where unit is kFineUnit.
+constexpr int kFineUnit = -68;
 template <bool kWide>
 __device__ __forceinline__ long long join_levels(const uint32_t* s, int& unit) {
   constexpr uint32_t kBase = 0x4B400000u, kBase9 = 0x4BC00000u;  // the patterns of 1.5 x 2^23 and 1.5 x 2^24
@@ -79,8 +88,9 @@ __device__ __forceinline__ long long join_levels(const uint32_t* s, int& unit) {
   const int l = sum(6) * 256 + l9;
   // h = the levels 2 .. 7 in units of 2^-56: |h| < 2^63; l holds levels 8 and 9, 12 bits further down
   const long long h = static_cast<long long>(p) * (1ll << 36) + static_cast<long long>(q) * (1 << 20) + static_cast<long long>(r) * 16;
-  const bool small = uint32_t(static_cast<unsigned long long>(h) >> 32) + (1u << 17) < (1u << 18);  // |h| < 2^49
-  unit = small ? -68 : -56;
+  constexpr uint32_t kSmall = 1u << (56 - kWeak - 32);
+  const bool small = uint32_t(static_cast<unsigned long long>(h) >> 32) + kSmall < 2 * kSmall;
+  unit = small ? kFineUnit : -56;
   return small ? h * 4096 + l : h + ((l + 2048) >> 12);
 }
 template <bool kWide>

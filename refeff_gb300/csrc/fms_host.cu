@@ -959,9 +959,13 @@ int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int b
   if (!rc && lu64 && ws.use_tc64) {
     // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); without room
     // for them the updates stay on the CUDA cores
-    const size_t one = tc64_image_bytes(n, m, 1), room = ws.use_tc ? ws.tc_image_size : size_t(1) << 30;
-    ws.tc64_batch = int(std::min<size_t>(size_t(ws.batch), std::max<size_t>(1, room / one)));
-    while (ws.use_tc && ws.tc64_batch > 1 && tc64_image_bytes(n, m, ws.tc64_batch) > room) --ws.tc64_batch;
+    const size_t room = ws.use_tc ? ws.tc_image_size : size_t(1) << 30;
+    ws.tc64_batch = 1;
+    for (int hi = ws.batch; ws.tc64_batch < hi;) {  // the most systems that fit
+      const int mid = ws.tc64_batch + (hi - ws.tc64_batch + 1) / 2;
+      if (tc64_image_bytes(n, m, mid) <= room) ws.tc64_batch = mid;
+      else hi = mid - 1;
+    }
     const size_t bytes = ws.use_tc ? 0 : tc64_image_bytes(n, m, ws.tc64_batch), na = size_t(ws.tc64_batch) * 32;
     if (ws.tc64_images.n < bytes || ws.tc_alpha.n < na) {
       ws.drop_graphs();

@@ -14,7 +14,8 @@
 //     column of A is small in every row (graded systems: without it a system
 //     whose columns span 24 orders of magnitude loses every digit in the back
 //     substitution); row r of A is then scaled by a power of two 2^-e_r so that
-//     its real and imaginary parts lie in (-1, 1), column c of B by 2^-f_c;
+//     its real and imaginary parts lie in (-1, 1), column c of B by 2^-f_c; a
+//     row of B that meets a zero column of A takes no part in f_c;
 //   * each scaled value is rounded to a 62-bit fixed-point number and cut into
 //     eight signed digits of weights 2^-6, 2^-14, ..., 2^-62 (|t| <= 128, exact
 //     in bf16);
@@ -22,7 +23,11 @@
 //     one level s = i + j (2 .. 9, 36 pairs) without rounding: at most 8 pairs
 //     x 2 real products x 32 columns x 2^14 = 2^23 < 2^24;
 //   * the epilogue adds the eight exact level sums in 64-bit integers, converts
-//     the total to FP64 (one rounding) and subtracts it from C (one rounding).
+//     the total to FP64 (one rounding) and subtracts it from C (one rounding);
+//   * where neither the sum nor C reaches 2^-7 of 2^(e_r + f_c), the products may
+//     be too small for the grid (sparse and badly scaled systems): the epilogue
+//     lists the entry, and tc64_recheck_kernel looks up its largest product and
+//     forms the sum again in FP64 multiply-adds where that is below 2^-6 of it.
 //
 // Dropped and cut parts weigh about 2^-62 of 2^(e_r + f_c) per product, less
 // than what the FMA chain it replaces rounds away in its 32 steps: on FMS
@@ -164,13 +169,25 @@ __device__ __forceinline__ double2 direct_sum(const double2* arow, const double2
   return acc;
 }
 
+// An entry whose sum the grid may have lost: C at (row, col) of matrix b is untouched yet; p the digit sum, of grid 2^e.
+struct alignas(16) Tc64Entry {
+  double2 p;
+  int row, col, b, e;
+};
+// Entries a block of tc64_recheck_kernel takes at a time: each CTA lists its own ones (counted in shared memory: a global
+// counter's latency held the epilogues up, 28.6 instead of 26.8 ms of updates of 16 systems of n = 2256) and hands them
+// on as chunks (first entry, count), since a few CTAs have most.
+constexpr int kChunk = 64;
+
 }  // namespace
 
 // alpha[b][k] = 2048 + max over the rows of (exponent of A[row, k] - exponent of the row's largest entry), 0 where column k
-// is zero: g_k = 2048 - alpha.  The table is zero before and is cleared again by the update kernel.
+// is zero in every row without infinities and NaN: g_k = 2048 - alpha.  The table is zero before and is cleared again by the update kernel.
 __global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int r_begin, int r_end, int ka, int kb,
-                                                           const double2* __restrict__ M, int* __restrict__ alpha) {
+                                                           const double2* __restrict__ M, int* __restrict__ alpha,
+                                                           int* __restrict__ chunks) {
   __shared__ int cmax[32];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *chunks = 0;  // of the update that follows
   const int b = blockIdx.y, lane = threadIdx.x & 31, row = r_begin + blockIdx.x * kRows + int(threadIdx.x);
   if (threadIdx.x < 32) cmax[threadIdx.x] = 0;
   const double2* A = M + size_t(b) * lay.stride + size_t(row) + size_t(lay.lda) * ka;
@@ -182,7 +199,7 @@ __global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int 
   int mine = 0;
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
-    const int v = __reduce_max_sync(0xffffffffu, f[k] > 0 && top < 0x7ff ? f[k] - top + 2048 : 0);
+    const int v = __reduce_max_sync(0xffffffffu, f[k] >= 0 && top < 0x7ff ? max(f[k], 1) - max(top, 1) + 2048 : 0);
     if (lane == k) mine = v;
   }
   __syncthreads();
@@ -194,18 +211,20 @@ __global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int 
 // Digits of both operands.  Blocks x < nbm: a row tile of A, image[b][bm][K step][re 1..8, im 1..8][128 rows of 16 bf16]
 // and the row exponents, two threads per row, 16 columns each.  The others: a column tile of B,
 // image[b][bn][K step][P, Q][digit 1..8][32 rows of 16 bf16] with P = [Br | Bi], Q = [-Bi | Br] (16 columns each) and the
-// column exponents, one warp per column, one lane per row.
+// column exponents, one warp per column, one lane per row.  rdef and cdef: 32 bytes a row of A and a column of B, how many
+// powers of two each (balanced) entry lies below the grid (127: 127 or more, or zero).
 __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end,
                                                          int ka, int kb, const double2* __restrict__ M,
                                                          const int* __restrict__ alpha, uint8_t* __restrict__ aimg,
                                                          uint8_t* __restrict__ bimg, int* __restrict__ rexp,
-                                                         int* __restrict__ cexp, int nbm, int nbm_all, int nbn_all) {
+                                                         int* __restrict__ cexp, uint8_t* __restrict__ rdef,
+                                                         uint8_t* __restrict__ cdef, int nbm, int nbm_all, int nbn_all) {
   __shared__ __align__(16) uint8_t sm[kBTile];
-  __shared__ int gk[32];
+  __shared__ int gk[32];  // kNoEntry: column k of A is zero
   const int b = blockIdx.y;
   if (threadIdx.x < 32) {
     const int a = alpha[b * 32 + int(threadIdx.x)];
-    gk[threadIdx.x] = a > 0 ? 2048 - a : 0;
+    gk[threadIdx.x] = a > 0 ? 2048 - a : kNoEntry;
   }
   __syncthreads();
   const double2* Mb = M + size_t(b) * lay.stride;
@@ -221,16 +240,24 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int f = field_of(v[i]);
-      if (f >= 0) e = max(e, f == 0x7ff ? kNonfinite : f - 1022 + gk[16 * h + i]);
+      if (f >= 0) e = max(e, f == 0x7ff ? kNonfinite : max(f, 1) - 1022 + gk[16 * h + i]);
     }
     if (h == 0) rowmax[r] = e;
     __syncthreads();
     if (h == 1) rowmax[r] = max(rowmax[r], e);
     __syncthreads();
     e = rowmax[r];
-    if (e == kNoEntry) e = 0;
-    if (h == 0) rexp[(size_t(b) * nbm_all + bm) * kRows + r] = e;
+    const size_t at = (size_t(b) * nbm_all + bm) * kRows + r;
+    if (h == 0) rexp[at] = e;
+    uint32_t below_grid[4] = {};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int f = field_of(v[i]);
+      below_grid[i / 4] |= uint32_t(f < 0 ? 127 : min(max(e - (max(f, 1) - 1022 + gk[16 * h + i]), 0), 127)) << (8 * (i % 4));
+    }
+    *reinterpret_cast<uint4*>(rdef + at * 32 + 16 * h) = make_uint4(below_grid[0], below_grid[1], below_grid[2], below_grid[3]);
     if (h * 16 >= kb) return;  // a K step that is not multiplied
+    const bool none = e == kNonfinite || e == kNoEntry;
     uint8_t* out = aimg + (size_t(b) * nbm_all + bm) * kATile + size_t(h) * kAHalf;
 #pragma unroll
     for (int ch = 0; ch < 2; ++ch)
@@ -240,7 +267,8 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const double x = part ? v[8 * ch + i].y : v[8 * ch + i].x;
-          y[i] = biased_digits(e == kNonfinite ? 0.0 : x, e - gk[16 * h + 8 * ch + i]);
+          const int g = gk[16 * h + 8 * ch + i];
+          y[i] = none || g == kNoEntry ? biased_digits(0.0, 0) : biased_digits(x, e - g);
         }
 #pragma unroll
         for (int d = 0; d < kDig; ++d) {
@@ -260,12 +288,14 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
     const int col = c_begin + bn * kCols + c;
     double2 v = make_double2(0.0, 0.0);
     if (col < c_end && k < kb) v = Mb[size_t(ka + k) + size_t(lay.lda) * col];
-    const int f = field_of(v);
-    int e = __reduce_max_sync(0xffffffffu, f < 0 ? kNoEntry : f == 0x7ff ? kNonfinite : f - 1022 - gk[k]);
-    if (e == kNoEntry) e = 0;
+    // an entry that meets only zeros of A must not set the column's grid (an infinity or NaN still marks the column)
+    const int f = field_of(v), g = gk[k];
+    const int e = __reduce_max_sync(0xffffffffu, f == 0x7ff ? kNonfinite : f < 0 || g == kNoEntry ? kNoEntry : max(f, 1) - 1022 - g);
     if (k == 0) cexp[(size_t(b) * nbn_all + bn) * kCols + c] = e;
-    if (e == kNonfinite) v = make_double2(0.0, 0.0);
-    const uint2 yr = biased_digits(v.x, e + gk[k]), yi = biased_digits(v.y, e + gk[k]);
+    const bool none = e == kNonfinite || e == kNoEntry || g == kNoEntry;
+    cdef[((size_t(b) * nbn_all + bn) * kCols + c) * 32 + k] = uint8_t(none || f < 0 ? 127 : min(e - (max(f, 1) - 1022 - g), 127));
+    if (none) v = make_double2(0.0, 0.0);
+    const uint2 yr = biased_digits(v.x, none ? 0 : e + g), yi = biased_digits(v.y, none ? 0 : e + g);
 #pragma unroll
     for (int d = 0; d < kDig; ++d) {
       const float re = digit_of(yr, d), im = digit_of(yi, d);
@@ -317,7 +347,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc64_update_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end, int ka, int kb,
                        double2* __restrict__ M, const uint8_t* __restrict__ aimg, const uint8_t* __restrict__ bimg,
                        const int* __restrict__ rexp, const int* __restrict__ cexp, int nbm_all, int nbn_all,
-                       Tc64Work w, int* __restrict__ alpha, int alpha_n, long long polls) {
+                       Tc64Work w, int* __restrict__ alpha, int alpha_n, Tc64Entry* __restrict__ list,
+                       int2* __restrict__ chunk, int* __restrict__ chunks, int capacity, long long polls) {
   extern __shared__ uint8_t smraw[];
   const uint32_t raw = smem_u32(smraw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -325,6 +356,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto bar = [&](int i) { return smem_u32(meta) + 8u * uint32_t(i); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(meta + 128);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(meta + 132);
+  int* const entries = reinterpret_cast<int*>(meta + 136);  // listed by this CTA, and those that found no room
+  const int list0 = blockIdx.x * capacity;                  // this CTA's part of the list
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nk = kb > 16 ? 2 : 1;  // K steps
   if (blockIdx.x == 0)
@@ -339,6 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < kBars; ++i)
       mbar_init(bar(i), i == kAccEmpty || i == kAccEmpty + 1 ? uint32_t(kEpiWarps) : 1u);
     *abort_flag = 0;
+    *entries = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -495,17 +529,37 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         if (c < have) {
-          double2 p;
+          double2 p = make_double2(0.0, 0.0);
+          bool store = true;
+          auto direct_entry = [&] {
+            const double2* Mb = M + size_t(tb) * lay.stride;
+            return direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
+          };
           const int e = er + ec[c];  // kNonfinite or more with an infinity or NaN, or where the waits ran out
           if (unsigned(e + kSafeExp) <= 2u * kSafeExp) {
             int ur, ui;
             const long long vr = join_levels<true>(lv, ur), vi = join_levels<true>(lv + kDig, ui);
             p = make_double2(normal_double(vr, e + ur), normal_double(vi, e + ui));
-          } else {
-            const double2* Mb = M + size_t(tb) * lay.stride;
-            p = direct_sum(Mb + size_t(trow) + size_t(lda) * ka, Mb + size_t(ka) + size_t(lda) * (tcol + c), lda, kb);
+            if (ur + ui == 2 * kFineUnit && below(cn[c], e - kWeak)) {
+              // a full list is not counted on: the counter stays within the threads that race for its last places
+              const int at = *static_cast<volatile int*>(entries) < capacity ? atomicAdd(entries, 1) : capacity;
+              store = at >= capacity;
+              if (store) {  // no room
+                p = direct_entry();
+              } else {
+                Tc64Entry entry;
+                entry.p = p;
+                entry.row = trow;
+                entry.col = tcol + c;
+                entry.b = tb;
+                entry.e = e;
+                list[list0 + at] = entry;
+              }
+            }
+          } else if (e > kNoEntry / 2) {  // else a row or column of zeros
+            p = direct_entry();
           }
-          cur[size_t(lda) * c] = make_double2(cn[c].x - p.x, cn[c].y - p.y);
+          if (store) cur[size_t(lda) * c] = make_double2(cn[c].x - p.x, cn[c].y - p.y);
         }
         cn[c] = c < nhave ? nxt[size_t(lda) * c] : make_double2(0.0, 0.0);
       }
@@ -516,7 +570,63 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (warp == 1) {
+    const int have = min(*entries, capacity), mine = (have + kChunk - 1) / kChunk;
+    int at = 0;
+    if (mine > 0 && lane == 0) at = atomicAdd(chunks, mine);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int q = lane; q < mine; q += 32) chunk[at + q] = make_int2(list0 + q * kChunk, min(kChunk, have - q * kChunk));
+  }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+}
+
+// The listed entries: C -= p where a product reaches 2^(e - kLost), else C -= the sum in FP64 multiply-adds.  Four lanes
+// an entry, eight terms each.  A kernel of its own: these entries gather in few rows of few tiles (0.3 .. 0.6% of all on
+// symmetric clusters, whose structural zeros are rounding noise in C), where warps that summed their own ones would hold
+// their tiles up.  Most are sound, and the bytes of rdef and cdef tell it without A and B.
+__global__ void __launch_bounds__(4 * kChunk, 2) tc64_recheck_kernel(BatchLayout lay, int r_begin, int c_begin, int ka, int kb,
+                                                                     double2* __restrict__ M, const uint8_t* __restrict__ rdef,
+                                                                     const uint8_t* __restrict__ cdef, int nbm_all, int nbn_all,
+                                                                     const Tc64Entry* __restrict__ list,
+                                                                     const int2* __restrict__ chunk,
+                                                                     const int* __restrict__ chunks) {
+  const int total = *chunks, i = int(threadIdx.x) / 4, part = threadIdx.x & 3;
+  const size_t lda = size_t(lay.lda);
+  for (int ch = blockIdx.x; ch < total; ch += gridDim.x) {
+    const int2 cc = chunk[ch];
+    const Tc64Entry q = list[cc.x + min(i, cc.y - 1)];
+    double2* const Mb = M + size_t(q.b) * lay.stride;
+    double2* const c = Mb + size_t(q.row) + lda * size_t(q.col);
+    double2 z = *c, p = q.p;
+    const uint2 da = *reinterpret_cast<const uint2*>(rdef + (size_t(q.b) * nbm_all * kRows + (q.row - r_begin)) * 32 + 8 * part);
+    const uint2 db = *reinterpret_cast<const uint2*>(cdef + (size_t(q.b) * nbn_all * kCols + (q.col - c_begin)) * 32 + 8 * part);
+    uint32_t d = __vminu4(da.x + db.x, da.y + db.y);  // at most 254 a byte
+    d = __vminu4(d, __shfl_xor_sync(0xffffffffu, d, 1));
+    d = __vminu4(d, __shfl_xor_sync(0xffffffffu, d, 2));
+    d = __vminu4(d, d >> 16);
+    const bool again = min(d & 255u, (d >> 8) & 255u) > uint32_t(kLost);
+    if (__any_sync(0xffffffffu, again)) {
+      const double2* const a = Mb + size_t(q.row) + lda * size_t(ka);
+      const double2* const b = Mb + size_t(ka) + lda * size_t(q.col);
+      double2 va[8], vb[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int k = part + 4 * j;
+        va[j] = again && k < kb ? a[lda * size_t(k)] : make_double2(0.0, 0.0);
+        vb[j] = again && k < kb ? b[k] : make_double2(0.0, 0.0);
+      }
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) cfma(s, va[j], vb[j]);
+#pragma unroll
+      for (int w = 1; w < 4; w *= 2) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, w);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, w);
+      }
+      if (again) p = s;
+    }
+    if (part == 0 && i < cc.y) *c = csub(z, p);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -525,7 +635,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 namespace {
 struct Tc64Images {
   int nbm, nbn;
-  size_t a, b, r, c, total;  // byte offsets of the A and B images, the row and column exponents
+  size_t a, b, r, c, rd, cd, list, chunk, chunks, total;  // byte offsets: A and B images, row and column exponents, rdef, cdef, listed entries
+  int capacity;                                           // entries a CTA may list
 };
 Tc64Images tc64_images(int n, int m, int batch) {
   Tc64Images v;
@@ -535,7 +646,16 @@ Tc64Images tc64_images(int n, int m, int batch) {
   v.b = v.a + size_t(batch) * v.nbm * kATile;
   v.r = v.b + size_t(batch) * v.nbn * kBTile;
   v.c = v.r + size_t(batch) * v.nbm * kRows * sizeof(int);
-  v.total = v.c + size_t(batch) * v.nbn * kCols * sizeof(int);
+  v.rd = v.c + size_t(batch) * v.nbn * kCols * sizeof(int);
+  v.cd = v.rd + size_t(batch) * v.nbm * kRows * 32;
+  v.list = v.cd + size_t(batch) * v.nbn * kCols * 32;
+  const int sms = current_sm_count();
+  // a tile's entries at least, a quarter of the share of a CTA, 128 MB in all at most
+  const size_t share = size_t(batch) * n * (n + m) / 4 / sms;
+  v.capacity = int(std::max<size_t>(kRows * kCols, std::min<size_t>((size_t(1) << 22) / sms, share))) / kChunk * kChunk;
+  v.chunk = v.list + size_t(sms) * v.capacity * sizeof(Tc64Entry);
+  v.chunks = v.chunk + size_t(sms) * v.capacity / kChunk * sizeof(int2);
+  v.total = v.chunks + 16;
   return v;
 }
 }  // namespace
@@ -549,6 +669,9 @@ void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int 
   const Tc64Images im = tc64_images(lay.n, lay.m, image_batch);
   int* rexp = reinterpret_cast<int*>(images + im.r);
   int* cexp = reinterpret_cast<int*>(images + im.c);
+  Tc64Entry* list = reinterpret_cast<Tc64Entry*>(images + im.list);
+  int2* chunk = reinterpret_cast<int2*>(images + im.chunk);
+  int* chunks = reinterpret_cast<int*>(images + im.chunks);
   const int sms = current_sm_count();
   ensure_smem_limit(reinterpret_cast<const void*>(tc64_update_kernel), size_t(kSmem));
   for (int b0 = 0; b0 < batch; b0 += image_batch) {
@@ -565,15 +688,19 @@ void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int 
     w.chunk = (w.nbn + w.nseg - 1) / w.nseg;
     w.units = nb * w.nbm * w.nseg;
     count_launch();
-    tc64_scale_kernel<<<dim3(unsigned(w.nbm), unsigned(nb)), kRows, 0, s>>>(lay, r_begin, r_end, ka, kb, Mb, alpha);
+    tc64_scale_kernel<<<dim3(unsigned(w.nbm), unsigned(nb)), kRows, 0, s>>>(lay, r_begin, r_end, ka, kb, Mb, alpha, chunks);
     count_launch();
     tc64_split_kernel<<<dim3(unsigned(w.nbm + w.nbn), unsigned(nb)), 256, 0, s>>>(
-        lay, r_begin, r_end, c_begin, c_end, ka, kb, Mb, alpha, images + im.a, images + im.b, rexp, cexp, w.nbm, im.nbm,
-        im.nbn);
+        lay, r_begin, r_end, c_begin, c_end, ka, kb, Mb, alpha, images + im.a, images + im.b, rexp, cexp,
+        images + im.rd, images + im.cd, w.nbm, im.nbm, im.nbn);
     count_launch();
-    tc64_update_kernel<<<unsigned(std::min(w.units, sms)), kThreads, kSmem, s>>>(
+    const unsigned ctas = unsigned(std::min(w.units, sms));
+    tc64_update_kernel<<<ctas, kThreads, kSmem, s>>>(
         lay, r_begin, r_end, c_begin, c_end, ka, kb, Mb, images + im.a, images + im.b, rexp, cexp, im.nbm, im.nbn, w,
-        alpha, nb * 32, wait_polls > 0 ? wait_polls : kTcWaitPolls);
+        alpha, nb * 32, list, chunk, chunks, im.capacity, wait_polls > 0 ? wait_polls : kTcWaitPolls);
+    count_launch();
+    tc64_recheck_kernel<<<unsigned(2 * sms), 4 * kChunk, 0, s>>>(lay, r_begin, c_begin, ka, kb, Mb, images + im.rd, images + im.cd,
+                                                                 im.nbm, im.nbn, list, chunk, chunks);
   }
 }
 

@@ -1,0 +1,69 @@
+"""LU solves of sparse and badly scaled systems: block triangular ones whose rows have other units, columns of L with one
+entry, entries that are small in their row and column but decide a sum.  The digit products of the FP64 form and the
+FP16 terms of the FP32 form lie on a grid set by a row's and a column's largest entries; what that grid cannot hold has
+to be summed another way.
+
+Tolerance: Gaussian elimination with partial pivoting in FP64 (any order of its sums) solves (A + E) x = b with
+|E| <= g |L| |U| componentwise, g = 3 n u sqrt(8) < 10 n u for complex arithmetic; |L| |U| is LAPACK's (the same pivot
+rule), row by row.
+"""
+import numpy as np
+import pytest
+
+from refeff_gb300 import fms
+
+scipy_linalg = pytest.importorskip("scipy.linalg")
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -53
+
+
+def _normal(rng, *shape):
+    return rng.normal(size=shape) + 1j * rng.normal(size=shape)
+
+
+def _block_system(n, n1, q, rng, border):
+    """[[s A11, s A12], [E, A22]], s = 2^q; E zero, or its row `border` of the size of the rows above."""
+    A, b = _normal(rng, n, n), _normal(rng, n, 3)
+    A[n1:, :n1] = 0
+    if border is not None:
+        A[n1 + border, :n1] = _normal(rng, n1) * 0.3
+        A[n1 + border, :n1] *= 2.0 ** q
+    A[:n1] *= 2.0 ** q
+    b[:n1] *= 2.0 ** q
+    return A, b
+
+
+def _solve(A, b, form=fms.FORM_FP64_LU, tensor=1):
+    c = fms.Context(0)
+    c.set_option(c.OPT_TENSOR_CORES, tensor)
+    X, st, _ = fms.complex_lu_solve_batched(c, A[None], b[None], form)
+    c.close()
+    return X[0], int(st[0])
+
+
+def _worst(A, X, b):
+    """The largest |A X - b| of a row over its |L| |U| |X| + |b|."""
+    L, U = scipy_linalg.lu(A, permute_l=True)
+    return float((np.abs(A @ X - b) / (np.abs(L) @ (np.abs(U) @ np.abs(X)) + np.abs(b))).max())
+
+
+@pytest.mark.parametrize("q", [10, 40, 100])
+@pytest.mark.parametrize("border", [None, 5])
+@pytest.mark.parametrize("n", [48, 170, 700])
+def test_blocks_of_other_units(n, border, q):
+    A, b = _block_system(n, 16, q, np.random.default_rng(n + q), border)
+    X, st = _solve(A, b)
+    assert st == 0 and _worst(A, X, b) < 10 * n * EPS
+
+
+def test_products_of_small_and_large_entries():
+    """x[32] = 2^-70 / (3 2^-70 - (1 2^-70 + 2^-70 1)): neither product reaches 2^-69 of its row's largest entry times
+    its column's."""
+    n, t = 34, 2.0 ** -70
+    A = np.eye(n, dtype=complex)
+    A[32, 32], A[32, 0], A[32, 1], A[0, 32] = 3 * t, 1, t, t
+    A[33, 1] = A[1, 32] = A[33, 32] = 1
+    b = np.zeros((n, 1), complex)
+    b[32] = t
+    X, st = _solve(A, b)
+    assert st == 0 and abs(X[32, 0] - 1) < 10 * n * EPS
