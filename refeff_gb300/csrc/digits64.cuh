@@ -59,7 +59,7 @@ __device__ __forceinline__ double normal_double(long long v, int ex) {
 }
 constexpr int kSafeExp = 900;  // sums of grids 2^e, |e| <= kSafeExp, are normal numbers
 __device__ __forceinline__ double scaled_double(long long v, int ex) {
-  return ex >= -kSafeExp && ex <= kSafeExp ? normal_double(v, ex) : scalbn(__ll2double_rn(v), ex);
+  return v == 0 || (ex >= -kSafeExp && ex <= kSafeExp) ? normal_double(v, ex) : scalbn(__ll2double_rn(v), ex);
 }
 
 // The grid's errors weigh some 2^-57 of 2^e in a sum of up to 32 complex products.  A sum below 2^(e - kWeak) beside a
@@ -93,12 +93,6 @@ __device__ __forceinline__ long long join_levels(const uint32_t* s, int& unit) {
   unit = small ? kFineUnit : -56;
   return small ? h * 4096 + l : h + ((l + 2048) >> 12);
 }
-template <bool kWide>
-__device__ __forceinline__ double join_double(const uint32_t* s, int e) {
-  int unit;
-  const long long v = join_levels<kWide>(s, unit);
-  return scaled_double(v, e + unit);
-}
 
 // ---------------------------------------------------------------------------
 // Warp-level form: C (16 x 8 complex) -= A (16 x 8) B (8 x 8) by mma.sync on the
@@ -119,7 +113,7 @@ __device__ __forceinline__ void mma_k16(float (&d)[4], uint32_t a0, uint32_t a1,
 
 struct DigitTileA {
   uint32_t re[kDig][2], im[kDig][2];  // rows g and g + 8
-  int e[2];                           // their exponents
+  int e[2];                           // their exponents (kNoEntry: zeros)
 };
 // A column of A that lies 2^-s below the rows' largest entries in all 16 rows keeps 62 - s bits: a tile with one beyond
 // this s (fewer than FP64's 53) is left to the FP64 pipe, as is one with an infinity or NaN.
@@ -148,9 +142,10 @@ __device__ __forceinline__ bool cut_tile_a(const double2 (&v)[2][2], DigitTileA&
   if (__any_sync(0xffffffffu, bad)) return false;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    a.e[h] = top[h] < 0 ? 0 : top[h] - 1022;
-    const uint2 r0 = biased_digits(v[h][0].x, a.e[h]), r1 = biased_digits(v[h][1].x, a.e[h]);
-    const uint2 i0 = biased_digits(v[h][0].y, a.e[h]), i1 = biased_digits(v[h][1].y, a.e[h]);
+    a.e[h] = top[h] < 0 ? kNoEntry : max(top[h], 1) - 1022;
+    const int e = top[h] < 0 ? 0 : a.e[h];
+    const uint2 r0 = biased_digits(v[h][0].x, e), r1 = biased_digits(v[h][1].x, e);
+    const uint2 i0 = biased_digits(v[h][0].y, e), i1 = biased_digits(v[h][1].y, e);
 #pragma unroll
     for (int d = 0; d < kDig; ++d) {
       a.re[d][h] = pack_bf16(digit_of(r0, d), digit_of(r1, d));
@@ -161,15 +156,15 @@ __device__ __forceinline__ bool cut_tile_a(const double2 (&v)[2][2], DigitTileA&
 }
 
 // Digits of B for one 8-column group, stored as words [2 d + part][lane] (part 0 re, 1 im) and the column exponents;
-// v[q] = B[2t + q][g].  A column with an infinity or NaN gets the exponent kNonfinite.
+// v[q] = B[2t + q][g].  A column with an infinity or NaN gets the exponent kNonfinite, one of zeros kNoEntry.
 __device__ __forceinline__ void cut_tile_b(const double2 (&v)[2], uint32_t* words, int* ecol) {
   const int lane = threadIdx.x & 31;
   int t = max(field_of(v[0]), field_of(v[1]));
   t = max(t, __shfl_xor_sync(0xffffffffu, t, 1));
   t = max(t, __shfl_xor_sync(0xffffffffu, t, 2));
-  const int e = t == 0x7ff ? kNonfinite : t < 0 ? 0 : t - 1022;
-  if ((lane & 3) == 0) ecol[lane >> 2] = e;
-  const bool bad = e == kNonfinite;
+  if ((lane & 3) == 0) ecol[lane >> 2] = t == 0x7ff ? kNonfinite : t < 0 ? kNoEntry : max(t, 1) - 1022;
+  const bool bad = t == 0x7ff || t < 0;
+  const int e = bad ? 0 : max(t, 1) - 1022;
   const uint2 r0 = biased_digits(bad ? 0.0 : v[0].x, e), r1 = biased_digits(bad ? 0.0 : v[1].x, e);
   const uint2 i0 = biased_digits(bad ? 0.0 : v[0].y, e), i1 = biased_digits(bad ? 0.0 : v[1].y, e);
 #pragma unroll
@@ -179,9 +174,10 @@ __device__ __forceinline__ void cut_tile_b(const double2 (&v)[2], uint32_t* word
   }
 }
 
-// p[h][q] = sum_k A[g + 8 h][k] B[k][2t + q] of the digits in `a` and of the words of cut_tile_b.
-__device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t* words, const int* ecol,
-                                             double2 (&p)[2][2]) {
+// p[h][q] = sum_k A[g + 8 h][k] B[k][2t + q] of the digits in `a` and of the words of cut_tile_b, on the grid
+// 2^(a.e[h] + ecol[2t + q]).  Bit 2 h + q of the result: the sum lies below 2^-kWeak of it.
+__device__ __forceinline__ uint32_t tile_product(const DigitTileA& a, const uint32_t* words, const int* ecol,
+                                                 double2 (&p)[2][2]) {
   const int lane = threadIdx.x & 31, t = lane & 3;
   float cr[kDig][4], ci[kDig][4];
 #pragma unroll
@@ -197,6 +193,7 @@ __device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t
       mma_k16(ci[i + j], a.re[i][0], a.re[i][1], a.im[i][0], a.im[i][1], bi, br);
     }
   }
+  uint32_t weak = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -208,8 +205,14 @@ __device__ __forceinline__ void tile_product(const DigitTileA& a, const uint32_t
         li[s] = __float_as_uint(ci[s][2 * h + q]);
       }
       const int e = a.e[h] + ecol[2 * t + q];
-      p[h][q] = make_double2(join_double<false>(lr, e), join_double<false>(li, e));
+      int ur, ui;
+      const long long vr = join_levels<false>(lr, ur);
+      p[h][q].x = scaled_double(vr, e + ur);
+      const long long vi = join_levels<false>(li, ui);
+      p[h][q].y = scaled_double(vi, e + ui);
+      if (ur + ui == 2 * kFineUnit && e > kNoEntry / 2) weak |= 1u << (2 * h + q);  // else a row or column of zeros
     }
+  return weak;
 }
 
 }  // namespace rfx

@@ -10,7 +10,10 @@
 //     and the block's rank-8 update of the remaining columns runs on the tensor
 //     path in exact 8-bit digit products (digits64.cuh, mma.sync on 16-row tiles
 //     that lie at the same rows whatever the cluster size, so that the result
-//     does not depend on it);
+//     does not depend on it), with FP64 multiply-adds for the sums that the
+//     digits' grid may have lost (structural zeros, sparse or badly scaled
+//     systems: a panel of 688 rows takes 115 us without such sums, up to 180
+//     with many);
 //   * the block's columns of a thread's row stay in registers (NB = 32; the
 //     narrower panels of large systems hold several rows a thread and work in
 //     shared memory); each warp publishes its pivot candidate's row with its
@@ -315,8 +318,9 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads == 256 ? 2 : 1)
 #pragma unroll
           for (int q = 0; q < 8; ++q) bad |= ecol[gr][q] == kNonfinite;
           double2 p[2][2];
+          uint32_t weak = 0, direct = 0;
           if (fits && !bad) {
-            tile_product(a, words[gr], ecol[gr], p);
+            weak = tile_product(a, words[gr], ecol[gr], p);
           } else {
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -335,9 +339,20 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads == 256 ? 2 : 1)
               const int r = r0 + g + 8 * h, c = 8 * gr + 2 * t + q;
               if (r < nloc && !done[r] && c < rest) {
                 double2& z = pan[size_t(ce + c) * rpc_max + r];
-                z = csub(z, p[h][q]);
+                const double2 old = z;
+                if ((weak >> (2 * h + q) & 1u) && below(old, a.e[h] + ecol[gr][2 * t + q] - kWeak)) direct |= 1u << (2 * h + q);
+                else z = csub(old, p[h][q]);
               }
             }
+          // in FP64 multiply-adds: sums whose products may have been lost on their grid (below kWeak of it, as C is)
+          for (; direct; direct &= direct - 1) {
+            const int bit = __ffs(direct) - 1, r = r0 + g + 8 * (bit >> 1), c = 8 * gr + 2 * t + (bit & 1);
+            double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int i = 0; i < kSub; ++i) cfma(s, pan[size_t(c0 + i) * rpc_max + r], U12[i][c]);
+            double2& z = pan[size_t(ce + c) * rpc_max + r];
+            z = csub(z, s);
+          }
         }
       }
       __syncthreads();

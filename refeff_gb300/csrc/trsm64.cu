@@ -11,7 +11,8 @@
 // blocks of the triangle, cut once per CTA.  The product is formed transposed,
 // C^T -= X^T L^T, so that X, the operand X^T and C^T share one register layout
 // (lane (g, t): columns g and g + 8, rows 2t and 2t + 1 of the block) and
-// nothing moves between lanes but the substitution's own broadcasts.
+// nothing moves between lanes but the substitution's own broadcasts.  Sums that
+// the digits' grid may have lost are formed again in FP64 multiply-adds.
 #include <cuda_runtime.h>
 #include "batched_lu.cuh"
 #include "cplx.cuh"
@@ -158,20 +159,30 @@ __global__ void __launch_bounds__(32 * kWarps) trsm64_kernel(BatchLayout lay, in
 #pragma unroll
       for (int i = 0; i < 8; ++i) bad |= ecol[at][i] == kNonfinite;
       double2 d[2][2];
+      // entries (bit 2 h + i) to be summed in FP64 multiply-adds: all of a tile that the digits cannot hold, and those
+      // whose products may have been lost on their grid (below kWeak of it, as C is)
+      uint32_t direct = 15;
       if (fits && !bad) {
-        tile_product(a, words[at], ecol[at], d);
-      } else {
+        direct = tile_product(a, words[at], ecol[at], d);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int i = 0; i < 2; ++i) d[h][i] = make_double2(0.0, 0.0);
-#pragma unroll 1
-        for (int j = 0; j < kBlk; ++j)
+          for (int i = 0; i < 2; ++i)
+            if (!below(x[p][h][i], a.e[h] + ecol[at][2 * t + i] - kWeak)) direct &= ~(1u << (2 * h + i));
+      }
+      if (__any_sync(0xffffffffu, direct)) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const double2 xj = shfl2(j & 1 ? x[q][h][1] : x[q][h][0], (lane & 28) + (j >> 1));
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int i = 0; i < 2; ++i) cfma(d[h][i], T[p * kBlk + 2 * t + i][q * kBlk + j], xj);
+          for (int i = 0; i < 2; ++i) {
+            if (!__any_sync(0xffffffffu, direct >> (2 * h + i) & 1u)) continue;
+            double2 s = make_double2(0.0, 0.0);
+#pragma unroll 2
+            for (int j = 0; j < kBlk; ++j) {
+              const double2 xj = shfl2(j & 1 ? x[q][h][1] : x[q][h][0], (lane & 28) + (j >> 1));
+              cfma(s, T[p * kBlk + 2 * t + i][q * kBlk + j], xj);
+            }
+            if (direct >> (2 * h + i) & 1u) d[h][i] = s;
           }
       }
 #pragma unroll

@@ -67,3 +67,26 @@ def test_products_of_small_and_large_entries():
     b[32] = t
     X, st = _solve(A, b)
     assert st == 0 and abs(X[32, 0] - 1) < 10 * n * EPS
+
+
+@pytest.mark.parametrize("q", [40, 100])
+@pytest.mark.parametrize("n1", [4, 20])
+@pytest.mark.parametrize("n", [24, 48, 170, 700])
+def test_units_that_change_inside_a_block_of_eight(n, n1, q):
+    """Rows of other units inside the 8-row blocks of the panels and block solves, on half of the columns."""
+    rng = np.random.default_rng(n + n1 + q)
+    A, b = _block_system(n, n1, q, rng, None)
+    b = np.concatenate([b, _normal(rng, n, 13)], 1)
+    A[:n1, n1:] *= rng.choice([0, 1], n - n1)
+    b[:n1] *= rng.choice([0, 1], 16)
+    X, st = _solve(A, b)
+    assert st == 0 and _worst(A, X, b) < 10 * n * EPS
+
+
+@pytest.mark.parametrize("n", [24, 48, 170])
+def test_entries_of_all_sizes(n):
+    rng = np.random.default_rng(n)
+    A = _normal(rng, n, n) * 2.0 ** rng.integers(-60, 61, (n, n)) * (rng.uniform(size=(n, n)) < 0.3) + np.diag(_normal(rng, n))
+    b = _normal(rng, n, 16) * 2.0 ** rng.integers(-60, 61, (n, 16))
+    X, st = _solve(A, b)
+    assert st == 0 and _worst(A, X, b) < 10 * n * EPS
