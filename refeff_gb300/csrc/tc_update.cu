@@ -11,10 +11,16 @@
 // FP16 carries the same 11 significant bits as TF32 at twice the rate and half
 // the operand bytes; what it lacks is exponent range, which power-of-two scales
 // give back: column k of A and row k of B are balanced by 2^g_k (so that no
-// column of A is small in every row), each row of A and each column of B is
-// scaled to a largest entry in [2^13, 2^14), and the epilogue takes the scales
-// out again.  Entries more than 2^16 below their row's largest lose relative,
-// not absolute, accuracy.
+// column of A is small in every row; a row of B that meets a zero column of A
+// counts as zeros), each row of A and each column of B is scaled to a largest
+// entry in [2^13, 2^14), and the epilogue takes the scales out again.  Entries
+// more than 2^16 below their row's largest keep 2^-39 of that instead of their
+// 22 bits, some 2^-35 of the largest product of row and column in a sum of 128.
+// Where neither the sum nor C reaches 2^-11 of that product (2^28 in the scaled
+// operands) the epilogue looks the entry's largest product up and, below 2^-9 of
+// it, forms the sum again in FP32 multiply-adds (recheck_column).  Most such entries
+// are sums of large products that cancel (2% of a symmetric cluster's), and a
+// bit mask of the row's and the column's large entries tells it at once.
 // The operands are first written by tc_split_kernel into tile images that are
 // already in the UMMA shared-memory layout (K-major, 64-byte rows, 64-byte
 // swizzle), so the update kernel moves them with plain cp.async.bulk copies
@@ -56,14 +62,18 @@ __device__ __forceinline__ int sw_offset(int row, int k) {
 
 // 2^e, e clamped to the normal range
 __device__ __forceinline__ float pow2(int e) { return __int_as_float(min(max(e + 127, 1), 254) << 23); }
+// 2^-shift, also below the normal range (exact: shift_of ends at 140)
+__device__ __forceinline__ float unscale(int shift) { return shift <= 126 ? pow2(-shift) : __int_as_float(1 << (149 - shift)); }
 // v 2^x for |x| beyond what one factor holds
 __device__ __forceinline__ float scaled(float v, int x) { return v * pow2(x >> 1) * pow2(x - (x >> 1)); }
-// the shift that brings values below 2^e below 2^14, within what the epilogue's factor 2^-shift can undo
-__device__ __forceinline__ int shift_of(int e) { return min(max(14 - e, -112), 112); }
-// larger exponent field of the two parts (0: zero or denormal)
+// the shift that brings values below 2^e below 2^14 (denormals alone: all their bits above FP16's last)
+__device__ __forceinline__ int shift_of(int e) { return min(14 - e, 140); }
+// larger exponent field of the two parts (0: zero; denormals as 1)
 __device__ __forceinline__ int field_of(float2 v) {
-  return int(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu) >> 23);
+  const uint32_t m = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+  return int(max(m >> 23, min(m, 1u)));
 }
+constexpr int kNone = -(1 << 20);  // exponent of a row or column of zeros, balance of a zero column of A
 // the FP16 terms of a scaled value
 __device__ __forceinline__ void split2(float x, __half& hi, __half& lo) {
   hi = __float2half_rn(x);
@@ -112,13 +122,82 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
+constexpr float kWeakSum = 131072.f;  // 2^(28 - 11)
+constexpr int kLost = 9, kLostRow = 4, kLostCol = kLost - kLostRow;
+// How many powers of two a scaled value lies below 2^14 (127: 127 or more, or zero).
+__device__ __forceinline__ uint32_t deficit(float2 v) {
+  const int f = field_of(v);
+  return f == 0 ? 127u : uint32_t(min(max(140 - f, 0), 127));
+}
+// One column of a warp's 32 rows, in the lanes marked `mine`, whose sums (pr, pi) and C are small: C -= the sum where the
+// entry's largest product reaches 2^(28 - kLost) or C is not small, else C -= the sum in FP32 multiply-adds, the rows one
+// after another, 32 terms at a time (a lane a row takes 128 loads one after another, 13 us, however few lanes have one).
+// rdef, cdef: the deficits of this lane's row and of the column; a0: A's first row of the warp, bcol: B's column.
+__device__ __forceinline__ void recheck_column(bool mine, float2* c, float rs, float cf, float pr, float pi, const uint8_t* rdef,
+                                            const uint8_t* cdef, const float2* a0, const float2* bcol, int lda, int kb) {
+  const int lane = threadIdx.x & 31;
+  bool again = false;
+  float2 v = make_float2(0.f, 0.f);
+  if (mine) {
+    v = *c;
+    const uint4 *ra = reinterpret_cast<const uint4*>(rdef), *cb = reinterpret_cast<const uint4*>(cdef);
+    uint32_t d = 0xfefefefeu;  // the smallest sum of two bytes (at most 254 each)
+#pragma unroll 4
+    for (int q = 0; q < (kb + 15) / 16; ++q) {
+      const uint4 x = ra[q], y = cb[q];
+      d = __vminu4(__vminu4(d, x.x + y.x), __vminu4(x.y + y.y, __vminu4(x.z + y.z, x.w + y.w)));
+    }
+    d = __vminu4(d, d >> 16);
+    again = min(d & 255u, d >> 8 & 255u) > uint32_t(kLost) && fmaxf(fabsf(v.x), fabsf(v.y)) < (kWeakSum * rs) * cf;
+  }
+  float2 p = make_float2(0.f, 0.f);
+  for (uint32_t rows = __ballot_sync(0xffffffffu, again); rows; rows &= rows - 1) {
+    const int r = __ffs(rows) - 1;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kTcKMax / 32; ++j) {
+      const int k = 32 * j + lane;
+      if (k < kb) cfma(acc, a0[size_t(lda) * k + r], bcol[k]);
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w /= 2) {
+      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, w);
+      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, w);
+    }
+    if (lane == r) p = acc;
+  }
+  if (mine) *c = again ? csub(v, p) : make_float2(fmaf(-(pr * rs), cf, v.x), fmaf(-(pi * rs), cf, v.y));
+}
+// Bit j of a row's or column's mask stands for g consecutive k from g j on, g = 1, 2 or 4 for kb <= 32, 64 or 128: all of
+// the row's entries lie within 2^kLostRow of its largest, one of the column's within 2^kLostCol; a common bit means a
+// product above 2^(28 - kLost).
+__device__ __forceinline__ uint32_t large_mask(const uint8_t* def, int kb, bool row) {
+  const uint32_t limit = 0x01010101u * uint32_t(row ? kLostRow : kLostCol);
+  const uint32_t* d = reinterpret_cast<const uint32_t*>(def);
+  uint32_t mask = 0;
+#pragma unroll 4
+  for (int q = 0; q < (kb + 3) / 4; ++q) {  // the bytes of a chunk beyond kb are 127
+    const uint32_t in = __vcmpleu4(d[q], limit);
+    if (kb <= 32) {
+      mask |= (in & 1u | in >> 7 & 2u | in >> 14 & 4u | in >> 21 & 8u) << (4 * q);
+    } else if (kb <= 64) {
+      const uint32_t lo = in & 0xffffu, hi = in >> 16;
+      mask |= (row ? uint32_t(lo == 0xffffu) | uint32_t(hi == 0xffffu) << 1 : uint32_t(lo != 0) | uint32_t(hi != 0) << 1) << (2 * q);
+    } else {
+      mask |= uint32_t(row ? in == 0xffffffffu : in != 0) << q;
+    }
+  }
+  return mask;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// scales and operand images: A[b][bm][chunk][plane] (8 KB), B[b][bn][chunk][plane] (4 KB), chunks of KC = 32
+// scales and operand images: A[b][bm][chunk][plane] (8 KB), B[b][bn][chunk][plane] (4 KB), chunks of KC = 32; rdef and
+// cdef, the deficit of each entry of A and B, a byte each, kTcKMax a row of A and a column of B
 // ---------------------------------------------------------------------------
 // alpha[b][k] = 256 + max over the rows of (exponent of A[row, k] - exponent of the row's largest entry), 0 where column k
-// is zero: g_k = 256 - alpha.  The table is zero before and is cleared again by the update kernel.
+// is zero in every row without infinities and NaN: g_k = 256 - alpha.  The table is zero before and is cleared again by the update kernel.
 template <int kK>  // kb <= kK, a multiple of 32
 __global__ void __launch_bounds__(BM) tc_scale_kernel(BatchLayout lay, int k, int kb, const float2* __restrict__ M,
                                                       int* __restrict__ alpha) {
@@ -129,13 +208,16 @@ __global__ void __launch_bounds__(BM) tc_scale_kernel(BatchLayout lay, int k, in
   uint32_t f[kK / 4];  // exponent fields, four to a word
   int top = 0;
 #pragma unroll
-  for (int q = 0; q < kK / 4; ++q) {
-    f[q] = 0;
+  for (int q = 0; q < kK / 32; ++q) {
+    float2 v[32];  // (loaded first: 32 loads in flight)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int kk = 4 * q + i, v = row < lay.n && kk < kb ? field_of(A[size_t(lay.lda) * kk]) : 0;
-      f[q] |= uint32_t(v) << (8 * i);
-      top = max(top, v);
+    for (int i = 0; i < 32; ++i)
+      v[i] = row < lay.n && 32 * q + i < kb ? A[size_t(lay.lda) * (32 * q + i)] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int x = field_of(v[i]), w = 8 * q + i / 4;
+      f[w] = (i % 4 ? f[w] : 0u) | uint32_t(x) << (8 * (i % 4));
+      top = max(top, x);
     }
   }
   __syncthreads();
@@ -158,15 +240,15 @@ static_assert(BM == kTcKMax, "one thread a column of the table");
 __device__ __forceinline__ void load_balance(const int* alpha, int* gk) {
   if (threadIdx.x < kTcKMax) {
     const int a = alpha[threadIdx.x];
-    gk[threadIdx.x] = a > 0 ? 256 - a : 0;
+    gk[threadIdx.x] = a > 0 ? 256 - a : kNone;
   }
   __syncthreads();
 }
 
 // Operand images: blocks x < nbm take a row tile of A, the others a column tile of B.
 __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int kb, const float2* __restrict__ M,
-                                             const int* gk, uint8_t* __restrict__ img, float* __restrict__ rscale,
-                                             int nbm, uint8_t* smem) {
+                                             const int* gk, uint8_t* __restrict__ img, float2* __restrict__ rscale,
+                                             uint8_t* rdef, int nbm, uint8_t* smem) {
   // The tile is read down the columns (coalesced in the column-major matrix),
   // turned around in shared memory, and written as 16-byte chunks of the
   // swizzled K-major rows.
@@ -179,21 +261,20 @@ __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int 
   const float2* Mb = M + size_t(b) * lay.stride + size_t(lay.lda) * k;
   {
     const int r = threadIdx.x & (BM - 1), h = threadIdx.x / BM;
-    int e = -(1 << 20);
+    int e = kNone;
     if (r0 + r < n)
 #pragma unroll 8
       for (int kk = h; kk < kb; kk += 2) {
         const int f = field_of(Mb[size_t(r0 + r) + size_t(lay.lda) * kk]);
-        if (f > 0) e = max(e, f - 126 + gk[kk]);
+        if (f > 0) e = max(e, gk[kk] == kNone ? 129 : f - 126 + gk[kk]);  // (129: a row with an infinity or NaN)
       }
     rowe[h][r] = e;
     __syncthreads();
     if (h == 0) {
       e = max(e, rowe[1][r]);
-      if (e == -(1 << 20)) e = 0;
-      e = shift_of(e);  // |A| 2^g < 2^e along the row
-      rowe[0][r] = e;
-      rscale[(size_t(b) * nbm + bm) * BM + r] = pow2(-e);
+      const int shift = e == kNone ? 0 : shift_of(e);  // |A| 2^g < 2^e along the row
+      rowe[0][r] = shift;
+      rscale[(size_t(b) * nbm + bm) * BM + r].x = e == kNone ? 0.f : unscale(shift);
     }
     __syncthreads();
   }
@@ -203,7 +284,7 @@ __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int 
       float2 v = make_float2(0.f, 0.f);
       if (r0 + r < n && kcol < kb) {
         v = Mb[size_t(r0 + r) + size_t(lay.lda) * kcol];
-        const int x = rowe[0][r] + gk[kcol];
+        const int g = gk[kcol], x = rowe[0][r] + (g == kNone ? 0 : g);
         v = make_float2(scaled(v.x, x), scaled(v.y, x));
       }
       T[kk * TS + r] = v;
@@ -213,12 +294,15 @@ __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int 
     for (int e = threadIdx.x; e < BM * (KC / 8); e += 256) {
       const int k8 = e % (KC / 8), r = e / (KC / 8);
       __align__(16) __half q[A_PLANES][8];
+      uint32_t d[2] = {0, 0};
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const float2 v = T[(8 * k8 + i) * TS + r];
         split2(v.x, q[0][i], q[1][i]);
         split2(v.y, q[2][i], q[3][i]);
+        d[i / 4] |= deficit(v) << (8 * (i % 4));
       }
+      *reinterpret_cast<uint2*>(rdef + ((size_t(b) * nbm + bm) * BM + r) * kTcKMax + chunk * KC + 8 * k8) = make_uint2(d[0], d[1]);
       const int off = sw_offset(r, 8 * k8);
 #pragma unroll
       for (int p = 0; p < A_PLANES; ++p)
@@ -226,29 +310,34 @@ __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int 
     }
     __syncthreads();
   }
+  if (threadIdx.x < BM) {
+    const size_t at = (size_t(b) * nbm + bm) * BM + threadIdx.x;
+    rscale[at].y = __uint_as_float(large_mask(rdef + at * kTcKMax, kb, true));
+  }
 }
 
 __device__ __forceinline__ void split_b_tile(const BatchLayout& lay, int bn, int k, int kb, int col_end,
                                              const float2* __restrict__ M, const int* gk, uint8_t* __restrict__ img,
-                                             float* __restrict__ cscale, int nbn, uint8_t* smem) {
+                                             float2* __restrict__ cscale, uint8_t* cdef, int nbn, uint8_t* smem) {
   int* cole = reinterpret_cast<int*>(smem);
   const int b = blockIdx.y, c0 = k + kb + bn * BN;
   const float2* Mb = M + size_t(b) * lay.stride + size_t(k);
   // column exponents: one warp a column, lanes down its rows
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int c = wid; c < BN; c += 8) {
-    int e = -(1 << 20);
+    int e = kNone;
     if (c0 + c < col_end)
       for (int kk = lane; kk < kb; kk += 32) {
+        // an entry that meets only zeros of A must not set the column's scale
         const int f = field_of(Mb[size_t(kk) + size_t(lay.lda) * (c0 + c)]);
-        if (f > 0) e = max(e, f - 126 - gk[kk]);
+        if (f > 0 && gk[kk] != kNone) e = max(e, f - 126 - gk[kk]);
+        else if (f == 255) e = max(e, 129);  // an infinity or NaN reaches every row
       }
     e = __reduce_max_sync(0xffffffffu, e);
-    if (e == -(1 << 20)) e = 0;
     if (lane == 0) {
-      e = shift_of(e);  // |B| 2^-g < 2^e along the column
-      cole[c] = e;
-      cscale[(size_t(b) * nbn + bn) * BN + c] = pow2(-e);
+      const int shift = e == kNone ? 0 : shift_of(e);  // |B| 2^-g < 2^e along the column
+      cole[c] = shift;
+      cscale[(size_t(b) * nbn + bn) * BN + c].x = e == kNone ? 0.f : unscale(shift);
     }
   }
   __syncthreads();
@@ -257,14 +346,15 @@ __device__ __forceinline__ void split_b_tile(const BatchLayout& lay, int bn, int
   for (int e = threadIdx.x; e < BN * nch * (KC / 8); e += 256) {
     const int k8 = e % (nch * (KC / 8)), c = e / (nch * (KC / 8)), chunk = k8 / (KC / 8), kin = 8 * (k8 % (KC / 8));
     __align__(16) __half q[B_PLANES][8];
+    uint32_t d[2] = {0, 0};
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int krow = 8 * k8 + i;
       float2 v = make_float2(0.f, 0.f);
       if (c0 + c < col_end && krow < kb) {
         v = Mb[size_t(krow) + size_t(lay.lda) * (c0 + c)];
-        const int x = cole[c] - gk[krow];
-        v = make_float2(scaled(v.x, x), scaled(v.y, x));
+        const int g = gk[krow], x = g == kNone ? 0 : cole[c] - g;
+        v = g == kNone && field_of(v) < 255 ? make_float2(0.f, 0.f) : make_float2(scaled(v.x, x), scaled(v.y, x));
       }
       __half rh, rl, ih, il;
       split2(v.x, rh, rl);
@@ -275,24 +365,32 @@ __device__ __forceinline__ void split_b_tile(const BatchLayout& lay, int bn, int
       q[3][i] = __hneg(il);
       q[4][i] = rl;
       q[5][i] = il;
+      d[i / 4] |= deficit(v) << (8 * (i % 4));
     }
+    *reinterpret_cast<uint2*>(cdef + ((size_t(b) * nbn + bn) * BN + c) * kTcKMax + 8 * k8) = make_uint2(d[0], d[1]);
     uint8_t* base = img + ((size_t(b) * nbn + bn) * kChunks + chunk) * size_t(B_PLANES) * B_PLANE + sw_offset(c, kin);
 #pragma unroll
     for (int p = 0; p < B_PLANES; ++p)
       *reinterpret_cast<uint4*>(base + size_t(p) * B_PLANE) = *reinterpret_cast<const uint4*>(q[p]);
+  }
+  __syncthreads();
+  if (threadIdx.x < BN) {
+    const size_t at = (size_t(b) * nbn + bn) * BN + threadIdx.x;
+    cscale[at].y = __uint_as_float(large_mask(cdef + at * kTcKMax, kb, false));
   }
 }
 
 __global__ void __launch_bounds__(256) tc_split_kernel(BatchLayout lay, int k, int kb, int col_end,
                                                        const float2* __restrict__ M, const int* __restrict__ alpha,
                                                        uint8_t* __restrict__ aimg, uint8_t* __restrict__ bimg,
-                                                       float* __restrict__ rscale, float* __restrict__ cscale, int nbm,
+                                                       float2* __restrict__ rscale, float2* __restrict__ cscale,
+                                                       uint8_t* rdef, uint8_t* cdef, int nbm,
                                                        int nbm_all, int nbn_all) {
   __shared__ __align__(16) uint8_t smem[KC * (BM + 1) * sizeof(float2) + 2 * BM * sizeof(int)];
   __shared__ int gk[kTcKMax];
   load_balance(alpha + blockIdx.y * kTcKMax, gk);
-  if (int(blockIdx.x) < nbm) split_a_tile(lay, k, kb, M, gk, aimg, rscale, nbm_all, smem);
-  else split_b_tile(lay, int(blockIdx.x) - nbm, k, kb, col_end, M, gk, bimg, cscale, nbn_all, smem);
+  if (int(blockIdx.x) < nbm) split_a_tile(lay, k, kb, M, gk, aimg, rscale, rdef, nbm_all, smem);
+  else split_b_tile(lay, int(blockIdx.x) - nbm, k, kb, col_end, M, gk, bimg, cscale, cdef, nbn_all, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -356,8 +454,8 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 
 __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
     BatchLayout lay, int k, int kb, int col_end, float2* __restrict__ M, const uint8_t* __restrict__ aimg,
-    const uint8_t* __restrict__ bimg, const float* __restrict__ rscale, const float* __restrict__ cscale, int nbm_all,
-    int nbn_all, int nbm, int nbn, int batch, int* __restrict__ alpha, int* __restrict__ err_flag, const int* skip,
+    const uint8_t* __restrict__ bimg, const float2* __restrict__ rscale, const float2* __restrict__ cscale,
+    const uint8_t* __restrict__ rdef, const uint8_t* __restrict__ cdef, int nbm_all, int nbn_all, int nbm, int nbn, int batch, int* __restrict__ alpha, int* __restrict__ err_flag, const int* skip,
     long long polls) {
   extern __shared__ uint8_t smraw[];
   const uint32_t raw = smem_u32(smraw);
@@ -525,8 +623,10 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
       const int row = r0 + quarter * 32 + lane;
       const bool row_ok = row < n;
       const int ld = lay.lda;  // column offsets within a tile stay far below 2^31 elements
-      const float rs = rscale[(size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane];
-      const float* cs = cscale + (size_t(b) * nbn_all + bn) * BN;
+      const float2 rsm = rscale[(size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane];
+      const float rs = rsm.x;
+      const uint32_t rmask = __float_as_uint(rsm.y);
+      const float2* cs = cscale + (size_t(b) * nbn_all + bn) * BN;
       float2* crow = M + size_t(b) * lay.stride + size_t(row) + size_t(lay.lda) * size_t(c0);
       // C of 16 columns at a time, an entry of the next part loaded as soon as this one's is used
       float2 cn[16];
@@ -537,8 +637,10 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
       if (!__all_sync(0xffffffffu, ready)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_r = tmem + uint32_t(g * 128) + lane_off, tmem_i = tmem_r + 64;
+      unsigned long long weak_cols = 0;
 #pragma unroll 1
       for (int part = 0; part < BN / 16; ++part) {
+        uint32_t lost = 0;  // columns of the part whose sums may have lost their terms: C stays as it is
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint32_t cr[8], ci[8];
@@ -556,15 +658,34 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
             const int i = h * 8 + j, off = part * 16 + i;
             if (row_ok && c0 + off < col_end) {
               float2 v = cn[i];
-              const float sc = rs * cs[off];
-              v.x = fmaf(-__uint_as_float(cr[j]), sc, v.x);
-              v.y = fmaf(-__uint_as_float(ci[j]), sc, v.y);
-              crow[off * ld] = v;
+              // the row's factor first: the column's may be 2^115, and either may be denormal
+              const float2 csm = cs[off];
+              const float cf = csm.x, pr = __uint_as_float(cr[j]), pi = __uint_as_float(ci[j]);
+              // (no branch here: it would part the loads of C from one another)
+              const bool weak = (fmaxf(fabsf(pr), fabsf(pi)) < kWeakSum) & ((rmask & __float_as_uint(csm.y)) == 0);
+              lost |= weak ? 1u << i : 0u;
+              crow[off * ld] = make_float2(fmaf(weak ? 0.f : -(pr * rs), cf, v.x), fmaf(weak ? 0.f : -(pi * rs), cf, v.y));
             }
             if (part + 1 < BN / 16)
               cn[i] = (row_ok && c0 + off + 16 < col_end) ? crow[(off + 16) * ld] : make_float2(0.f, 0.f);
           }
         }
+        weak_cols |= static_cast<unsigned long long>(lost) << (16 * part);
+      }
+      // the columns in which a row of this warp has one (the accumulators are still there; C's registers are free)
+      unsigned long long any = (static_cast<unsigned long long>(__reduce_or_sync(0xffffffffu, uint32_t(weak_cols >> 32))) << 32) |
+                               __reduce_or_sync(0xffffffffu, uint32_t(weak_cols));
+      for (; any; any &= any - 1) {
+        const int off = __ffsll(static_cast<long long>(any)) - 1;
+        uint32_t ur, ui;
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ur) : "r"(tmem_r + uint32_t(off)));
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ui) : "r"(tmem_i + uint32_t(off)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(ur), "+r"(ui)::"memory");
+        const float2* Mb = M + size_t(b) * lay.stride + size_t(k);
+        recheck_column(weak_cols >> off & 1u, crow + off * ld, rs, cs[off].x, __uint_as_float(ur), __uint_as_float(ui),
+                       rdef + ((size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane) * kTcKMax,
+                       cdef + ((size_t(b) * nbn_all + bn) * BN + off) * kTcKMax,
+                       Mb + size_t(ld) * k + size_t(r0 - k + quarter * 32), Mb + size_t(ld) * (c0 + off), ld, kb);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(bar(kBarAccEmpty + g));  // the accumulator may be overwritten
@@ -581,7 +702,7 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
 namespace {
 struct TcImages {
   int nbm, nbn;
-  size_t a, b, r, c, total;  // byte offsets of the A and B images, the row and column scales
+  size_t a, b, r, c, rd, cd, total;  // byte offsets of the A and B images, the row and column scales (with masks), rdef and cdef
 };
 TcImages tc_images(int n, int m, int batch) {
   TcImages v;
@@ -590,8 +711,10 @@ TcImages tc_images(int n, int m, int batch) {
   v.a = 0;
   v.b = v.a + size_t(batch) * v.nbm * kChunks * A_PLANES * A_PLANE;
   v.r = v.b + size_t(batch) * v.nbn * kChunks * B_PLANES * B_PLANE;
-  v.c = v.r + size_t(batch) * v.nbm * BM * sizeof(float);
-  v.total = v.c + size_t(batch) * v.nbn * BN * sizeof(float);
+  v.c = v.r + size_t(batch) * v.nbm * BM * sizeof(float2);
+  v.rd = v.c + size_t(batch) * v.nbn * BN * sizeof(float2);
+  v.cd = v.rd + size_t(batch) * v.nbm * BM * kTcKMax;
+  v.total = v.cd + size_t(batch) * v.nbn * BN * kTcKMax;
   return v;
 }
 }  // namespace
@@ -605,7 +728,7 @@ void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int co
   if (rows <= 0 || cols <= 0 || kb <= 0) return;
   const TcImages im = tc_images(lay.n, lay.m, batch);
   uint8_t *aimg = images + im.a, *bimg = images + im.b;
-  float *rscale = reinterpret_cast<float*>(images + im.r), *cscale = reinterpret_cast<float*>(images + im.c);
+  float2 *rscale = reinterpret_cast<float2*>(images + im.r), *cscale = reinterpret_cast<float2*>(images + im.c);
   const int nbm_all = im.nbm, nbn_all = im.nbn;
   const int nbm = (rows + BM - 1) / BM, nbn = (cols + BN - 1) / BN;
   const dim3 sgrid{unsigned(nbm), unsigned(batch)};
@@ -615,7 +738,8 @@ void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int co
   else tc_scale_kernel<kTcKMax><<<sgrid, BM, 0, s>>>(lay, k, kb, M, alpha);
   count_launch();
   tc_split_kernel<<<dim3(unsigned(nbm + nbn), unsigned(batch)), 256, 0, s>>>(lay, k, kb, col_end, M, alpha, aimg, bimg,
-                                                                            rscale, cscale, nbm, nbm_all, nbn_all);
+                                                                            rscale, cscale, images + im.rd, images + im.cd, nbm,
+                                                                            nbm_all, nbn_all);
   const int sms = current_sm_count();
   ensure_smem_limit(reinterpret_cast<const void*>(tc_update_persistent_kernel), size_t(kPSmem));
   const long long tiles = (long long)nbm * nbn * batch;
@@ -632,7 +756,8 @@ void tc_trailing_update(const BatchLayout& lay, int batch, int k, int kb, int co
     cudaEventRecord(e0, s);
   }
   count_launch();
-  tc_update_persistent_kernel<<<grid, kPThreads, kPSmem, s>>>(lay, k, kb, col_end, M, aimg, bimg, rscale, cscale, nbm_all,
+  tc_update_persistent_kernel<<<grid, kPThreads, kPSmem, s>>>(lay, k, kb, col_end, M, aimg, bimg, rscale, cscale,
+                                                              images + im.rd, images + im.cd, nbm_all,
                                                               nbn_all, nbm, nbn, batch, alpha, err_flag, skip,
                                                               wait_polls > 0 ? wait_polls : kTcWaitPolls);
   if (prof) {

@@ -90,3 +90,41 @@ def test_entries_of_all_sizes(n):
     b = _normal(rng, n, 16) * 2.0 ** rng.integers(-60, 61, (n, 16))
     X, st = _solve(A, b)
     assert st == 0 and _worst(A, X, b) < 10 * n * EPS
+
+
+def _fp32_solution(A, b):
+    """The FP32 LU's solution as it is, without corrections."""
+    c = fms.Context(0)
+    c.set_option(c.OPT_DENSE_REFINEMENT, 0)
+    X, _, _ = fms.complex_lu_solve_batched(c, A[None], b[None], fms.FORM_FP32_REFINED)
+    c.close()
+    return X[0]
+
+
+@pytest.mark.parametrize("q", [10, 30, 60])
+@pytest.mark.parametrize("border", [None, 5])
+@pytest.mark.parametrize("n", [48, 170, 700])
+def test_fp32_blocks_of_other_units(n, border, q):
+    """The same bound with the unit roundoff of FP32 (A rounded to it among the errors), and the refined solution's."""
+    A, b = _block_system(n, 16, q, np.random.default_rng(n + q), border)
+    assert _worst(A, _fp32_solution(A, b), b) < 10 * n * 2.0 ** -24
+    X, st = _solve(A, b, fms.FORM_FP32_REFINED)
+    assert st == 0 and np.isfinite(X).all()
+
+
+@pytest.mark.parametrize("n", [48, 170, 700])
+def test_fp32_entries_of_all_sizes(n):
+    rng = np.random.default_rng(n)
+    A = _normal(rng, n, n) * 2.0 ** rng.integers(-30, 31, (n, n)) * (rng.uniform(size=(n, n)) < 0.3) + np.diag(_normal(rng, n))
+    b = _normal(rng, n, 16) * 2.0 ** rng.integers(-30, 31, (n, 16))
+    assert _worst(A, _fp32_solution(A, b), b) < 10 * n * 2.0 ** -24
+
+
+def test_fp32_right_hand_sides_near_the_end_of_the_range_keep_their_bits():
+    """Scaling by a power of two changes no bit of an FP32 elimination but where a sum cancels into the denormals, 2^-149
+    each: some 2^-31 of values of 2^-114 over a sum of 170."""
+    n = 170
+    rng = np.random.default_rng(3)
+    A, b = (_normal(rng, n, n) + 3 * np.sqrt(n) * np.eye(n)) / 64, _normal(rng, n, 8)
+    X, Y = _fp32_solution(A, b), _fp32_solution(A, b * 2.0 ** -114) * 2.0 ** 114
+    assert np.abs(X - Y).max() <= 2.0 ** -29 * np.abs(X).max()
