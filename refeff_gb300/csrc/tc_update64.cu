@@ -25,9 +25,10 @@
 //   * the epilogue adds the eight exact level sums in 64-bit integers, converts
 //     the total to FP64 (one rounding) and subtracts it from C (one rounding);
 //   * where neither the sum nor C reaches 2^-7 of 2^(e_r + f_c), the products may
-//     be too small for the grid (sparse and badly scaled systems): the epilogue
-//     lists the entry, and tc64_recheck_kernel looks up its largest product and
-//     forms the sum again in FP64 multiply-adds where that is below 2^-6 of it.
+//     be too small for the grid (sparse and badly scaled systems): unless large
+//     entries of the row and the column meet, the epilogue lists the entry, and
+//     tc64_recheck_kernel looks up its largest product and forms the sum again
+//     in FP64 multiply-adds where that is below 2^-6 of it.
 //
 // Dropped and cut parts weigh about 2^-62 of 2^(e_r + f_c) per product, less
 // than what the FMA chain it replaces rounds away in its 32 steps: on FMS
@@ -169,6 +170,9 @@ __device__ __forceinline__ double2 direct_sum(const double2* arow, const double2
   return acc;
 }
 
+// Most small sums are of large products that cancel: masks of the k at which a row's entries reach 2^-kLostPart of its
+// largest, and a column's of its, tell it by a common bit.
+constexpr int kLostPart = kLost / 2;
 // An entry whose sum the grid may have lost: C at (row, col) of matrix b is untouched yet; p the digit sum, of grid 2^e.
 struct alignas(16) Tc64Entry {
   double2 p;
@@ -211,13 +215,14 @@ __global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int 
 // Digits of both operands.  Blocks x < nbm: a row tile of A, image[b][bm][K step][re 1..8, im 1..8][128 rows of 16 bf16]
 // and the row exponents, two threads per row, 16 columns each.  The others: a column tile of B,
 // image[b][bn][K step][P, Q][digit 1..8][32 rows of 16 bf16] with P = [Br | Bi], Q = [-Bi | Br] (16 columns each) and the
-// column exponents, one warp per column, one lane per row.  rdef and cdef: 32 bytes a row of A and a column of B, how many
-// powers of two each (balanced) entry lies below the grid (127: 127 or more, or zero).
+// column exponents, one warp per column, one lane per row, each exponent with its mask of large entries.  rdef and cdef:
+// 32 bytes a row of A and a column of B, how many powers of two each (balanced) entry lies below the grid (127: 127 or more,
+// or zero).
 __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end,
                                                          int ka, int kb, const double2* __restrict__ M,
                                                          const int* __restrict__ alpha, uint8_t* __restrict__ aimg,
-                                                         uint8_t* __restrict__ bimg, int* __restrict__ rexp,
-                                                         int* __restrict__ cexp, uint8_t* __restrict__ rdef,
+                                                         uint8_t* __restrict__ bimg, int2* __restrict__ rexp,
+                                                         int2* __restrict__ cexp, uint8_t* __restrict__ rdef,
                                                          uint8_t* __restrict__ cdef, int nbm, int nbm_all, int nbn_all) {
   __shared__ __align__(16) uint8_t sm[kBTile];
   __shared__ int gk[32];  // kNoEntry: column k of A is zero
@@ -248,13 +253,16 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
     __syncthreads();
     e = rowmax[r];
     const size_t at = (size_t(b) * nbm_all + bm) * kRows + r;
-    if (h == 0) rexp[at] = e;
-    uint32_t below_grid[4] = {};
+    uint32_t below_grid[4] = {}, large = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const int f = field_of(v[i]);
-      below_grid[i / 4] |= uint32_t(f < 0 ? 127 : min(max(e - (max(f, 1) - 1022 + gk[16 * h + i]), 0), 127)) << (8 * (i % 4));
+      const int f = field_of(v[i]), d = f < 0 ? 127 : min(max(e - (max(f, 1) - 1022 + gk[16 * h + i]), 0), 127);
+      below_grid[i / 4] |= uint32_t(d) << (8 * (i % 4));
+      large |= d <= kLostPart ? 1u << i : 0u;
     }
+    uint16_t* const half_mask = reinterpret_cast<uint16_t*>(&rexp[at].y);
+    half_mask[h] = uint16_t(large);
+    if (h == 0) rexp[at].x = e;
     *reinterpret_cast<uint4*>(rdef + at * 32 + 16 * h) = make_uint4(below_grid[0], below_grid[1], below_grid[2], below_grid[3]);
     if (h * 16 >= kb) return;  // a K step that is not multiplied
     const bool none = e == kNonfinite || e == kNoEntry;
@@ -291,9 +299,12 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
     // an entry that meets only zeros of A must not set the column's grid (an infinity or NaN still marks the column)
     const int f = field_of(v), g = gk[k];
     const int e = __reduce_max_sync(0xffffffffu, f == 0x7ff ? kNonfinite : f < 0 || g == kNoEntry ? kNoEntry : max(f, 1) - 1022 - g);
-    if (k == 0) cexp[(size_t(b) * nbn_all + bn) * kCols + c] = e;
     const bool none = e == kNonfinite || e == kNoEntry || g == kNoEntry;
-    cdef[((size_t(b) * nbn_all + bn) * kCols + c) * 32 + k] = uint8_t(none || f < 0 ? 127 : min(e - (max(f, 1) - 1022 - g), 127));
+    const int d = none || f < 0 ? 127 : min(e - (max(f, 1) - 1022 - g), 127);
+    const size_t at = (size_t(b) * nbn_all + bn) * kCols + c;
+    cdef[at * 32 + k] = uint8_t(d);
+    const uint32_t large = __ballot_sync(0xffffffffu, d <= kLostPart);
+    if (k == 0) cexp[at] = make_int2(e, int(large));
     if (none) v = make_double2(0.0, 0.0);
     const uint2 yr = biased_digits(v.x, none ? 0 : e + g), yi = biased_digits(v.y, none ? 0 : e + g);
 #pragma unroll
@@ -346,7 +357,7 @@ struct Tc64Tile {
 __global__ void __launch_bounds__(kThreads, 1)
     tc64_update_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end, int ka, int kb,
                        double2* __restrict__ M, const uint8_t* __restrict__ aimg, const uint8_t* __restrict__ bimg,
-                       const int* __restrict__ rexp, const int* __restrict__ cexp, int nbm_all, int nbn_all,
+                       const int2* __restrict__ rexp, const int2* __restrict__ cexp, int nbm_all, int nbn_all,
                        Tc64Work w, int* __restrict__ alpha, int alpha_n, Tc64Entry* __restrict__ list,
                        int2* __restrict__ chunk, int* __restrict__ chunks, int capacity, long long polls) {
   extern __shared__ uint8_t smraw[];
@@ -489,9 +500,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = 0; j < 4; ++j) cn[j] = j < have ? cur[size_t(lda) * j] : make_double2(0.0, 0.0);
     }
     while (more) {
-      int er = rexp[(size_t(t.b) * nbm_all + t.bm) * kRows + quarter * 32 + lane];
-      const int4 ec4 = *reinterpret_cast<const int4*>(cexp + (size_t(t.b) * nbn_all + t.bn) * kCols + 4 * g);
-      const int ec[4] = {ec4.x, ec4.y, ec4.z, ec4.w};
+      const int2 erm = rexp[(size_t(t.b) * nbm_all + t.bm) * kRows + quarter * 32 + lane];
+      int er = erm.x;
+      const int4* const ec4 = reinterpret_cast<const int4*>(cexp + (size_t(t.b) * nbn_all + t.bn) * kCols + 4 * g);
+      const int4 ec01 = ec4[0], ec23 = ec4[1];
+      const int ec[4] = {ec01.x, ec01.z, ec23.x, ec23.z}, cmask[4] = {ec01.y, ec01.w, ec23.y, ec23.w};
       const int tb = t.b, tcol = c_begin + t.bn * kCols + 4 * g, trow = r_begin + t.bm * kRows + quarter * 32 + lane;
       more = t.next(w);
       double2* const nxt = more ? c_ptr(t) : M;
@@ -540,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             int ur, ui;
             const long long vr = join_levels<true>(lv, ur), vi = join_levels<true>(lv + kDig, ui);
             p = make_double2(normal_double(vr, e + ur), normal_double(vi, e + ui));
-            if (ur + ui == 2 * kFineUnit && below(cn[c], e - kWeak)) {
+            if (ur + ui == 2 * kFineUnit && !(erm.y & cmask[c]) && below(cn[c], e - kWeak)) {
               // a full list is not counted on: the counter stays within the threads that race for its last places
               const int at = *static_cast<volatile int*>(entries) < capacity ? atomicAdd(entries, 1) : capacity;
               store = at >= capacity;
@@ -645,8 +658,8 @@ Tc64Images tc64_images(int n, int m, int batch) {
   v.a = 0;
   v.b = v.a + size_t(batch) * v.nbm * kATile;
   v.r = v.b + size_t(batch) * v.nbn * kBTile;
-  v.c = v.r + size_t(batch) * v.nbm * kRows * sizeof(int);
-  v.rd = v.c + size_t(batch) * v.nbn * kCols * sizeof(int);
+  v.c = v.r + size_t(batch) * v.nbm * kRows * sizeof(int2);
+  v.rd = v.c + size_t(batch) * v.nbn * kCols * sizeof(int2);
   v.cd = v.rd + size_t(batch) * v.nbm * kRows * 32;
   v.list = v.cd + size_t(batch) * v.nbn * kCols * 32;
   const int sms = current_sm_count();
@@ -667,8 +680,8 @@ void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int 
   const int rows = r_end - r_begin, cols = c_end - c_begin;
   if (rows <= 0 || cols <= 0 || kb <= 0 || image_batch <= 0) return;
   const Tc64Images im = tc64_images(lay.n, lay.m, image_batch);
-  int* rexp = reinterpret_cast<int*>(images + im.r);
-  int* cexp = reinterpret_cast<int*>(images + im.c);
+  int2* rexp = reinterpret_cast<int2*>(images + im.r);
+  int2* cexp = reinterpret_cast<int2*>(images + im.c);
   Tc64Entry* list = reinterpret_cast<Tc64Entry*>(images + im.list);
   int2* chunk = reinterpret_cast<int2*>(images + im.chunk);
   int* chunks = reinterpret_cast<int*>(images + im.chunks);
