@@ -2291,7 +2291,8 @@ refeff_fms_context::~refeff_fms_context() = default;
 
 namespace {
 
-// The context's dense workspace, configured for the call.
+// The context's dense workspace, configured for the call; its timeout flag is lowered (it may be up from an earlier
+// call), and stays up once a batch of this call has raised it.
 int dense_workspace(refeff_fms_context* ctx, int n, int m, int batch, bool fp32, DenseCache*& out) {
   for (int attempt = 0;; ++attempt) {
     const bool fresh = !ctx->dense || ctx->dense->tensor_cores != ctx->use_tensor_cores || attempt;
@@ -2301,6 +2302,7 @@ int dense_workspace(refeff_fms_context* ctx, int n, int m, int batch, bool fp32,
     }
     out = ctx->dense.get();
     const int rc = ensure_workspace(ctx, out->ws, n, m, batch, fp32);
+    if (!rc && out->ws.use_tc) RF_CUDA(ctx, cudaMemsetAsync(out->ws.tc_err.p, 0, sizeof(int), ctx->stream));
     if (rc != REFEFF_FMS_ERR_OUT_OF_MEMORY || fresh) return rc;
     cudaGetLastError();  // buffers kept from other shapes may be in the way: once more from nothing
   }
@@ -2414,7 +2416,6 @@ int dense_solve_device(refeff_fms_context* ctx, Workspace& ws, int batch, bool f
   const BatchLayout& lay = ws.lay;
   RF_CUDA(ctx, cudaMemsetAsync(ws.status.p, 0, size_t(batch) * sizeof(int), s));
   RF_CUDA(ctx, cudaMemsetAsync(ws.info.p, 0, size_t(batch) * sizeof(int), s));
-  if (ws.use_tc) RF_CUDA(ctx, cudaMemsetAsync(ws.tc_err.p, 0, sizeof(int), s));  // the workspace outlives a timed-out call
   if (!fp32) {
     const LuWork w64 = lu_work(ws, ws.pc64, true);
     cudaError_t e = lu_eliminate<double>(ws.pc64, lay, batch, ws.M64.p, w64, s);
