@@ -2498,13 +2498,21 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   }
   if (!std::isfinite(total) || !(total > 0.0))
     return fail(ctx, REFEFF_FMS_ERR_INVALID_ARGUMENT, "reciprocal FMS total k-point weight must be positive and finite");
+  // A structure factor with an infinity or NaN is the first thing refused.  The device looks for it as it packs a batch,
+  // before the batch is solved; where the call ends before that, the host does.
+  auto refuse = [&](int rc, const std::string& what) {
+    for (size_t i = 0; i < nn * size_t(n_kpoints); ++i)
+      if (!std::isfinite(structure_factors[i].re) || !std::isfinite(structure_factors[i].im))
+        return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite structure factor");
+    return fail(ctx, rc, what);
+  };
   // the lattice T by columns, non-zero entries only (FmsReciprocalPlan::new, reciprocal.rs:80-97)
   std::vector<int> ptr(static_cast<size_t>(order) + 1, 0), rows;
   std::vector<double2> vals;
   for (int c = 0; c < order; ++c) {
     for (int r = 0; r < order; ++r) {
       const refeff_complex128 v = t_matrix[size_t(r) + size_t(order) * c];
-      if (!std::isfinite(v.re) || !std::isfinite(v.im)) return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite T");
+      if (!std::isfinite(v.re) || !std::isfinite(v.im)) return refuse(REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite T");
       if (v.re != 0.0 || v.im != 0.0) {
         rows.push_back(r);
         vals.push_back(make_double2(v.re, v.im));
@@ -2527,7 +2535,7 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   DenseCache* dense = nullptr;
   DenseTrim trim{ctx};
   int rc = dense_workspace(ctx, order, order, B, fp32, dense);
-  if (rc) return rc;
+  if (rc) return refuse(rc, std::string(ctx->last_error));
   Workspace& ws = dense->ws;
   const BatchLayout& lay = ws.lay;
   DevBuf<int> d_ptr, d_rows;
@@ -2547,6 +2555,10 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
     const int nb = std::min(B, n_kpoints - k0);
     rc = upload_systems(ctx, *dense, nb, nullptr, structure_factors + size_t(k0) * nn, s, d_nonfinite.p);
     if (rc) return rc;
+    int nonfinite = 0;
+    RF_CUDA(ctx, cudaMemcpyAsync(&nonfinite, d_nonfinite.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    RF_CUDA(ctx, cudaStreamSynchronize(s));
+    if (nonfinite) return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite structure factor");
     count_launch();
     kkr_system_kernel<<<dim3(unsigned((order + 127) / 128), unsigned(order), unsigned(nb)), 128, 0, s>>>(
         lay, ws.M64.p, d_ptr.p, d_rows.p, d_vals.p);
@@ -2559,11 +2571,9 @@ extern "C" int refeff_fms_reciprocal_integrate(refeff_fms_context* ctx, int orde
   }
   std::vector<double2> acc(nn);
   RF_CUDA(ctx, cudaMemcpyAsync(acc.data(), d_acc.p, nn * sizeof(double2), cudaMemcpyDeviceToHost, s));
-  int tc_timeout = 0, nonfinite = 0;
+  int tc_timeout = 0;
   if (ws.use_tc) RF_CUDA(ctx, cudaMemcpyAsync(&tc_timeout, ws.tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RF_CUDA(ctx, cudaMemcpyAsync(&nonfinite, d_nonfinite.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   RF_CUDA(ctx, cudaStreamSynchronize(s));
-  if (nonfinite) return fail(ctx, REFEFF_FMS_ERR_NONFINITE_INPUT, "non-finite structure factor");
   if (tc_timeout) return fail(ctx, REFEFF_FMS_ERR_CUDA, "tensor-core update timed out");
   int first_bad = -1;
   for (int q = 0; q < n_kpoints; ++q) {

@@ -24,3 +24,25 @@ def test_a_wait_that_runs_out_in_the_first_batch_is_reported():
         fms.reciprocal_integrate(ctx, *_inputs(64, 1025), fms.FORM_FP32_REFINED)
     assert "timed out" in str(e.value)
     ctx.close()
+
+
+def test_a_nonfinite_structure_factor_is_refused_first_and_before_anything_is_solved():
+    ctx = fms.Context(0)
+    G, w, T = _inputs(96, 30)
+    fms.reciprocal_integrate(ctx, G, w, T)
+    G[29, 95, 95] = np.nan
+    launches = ctx._lib.refeff_fms_kernel_launches
+    before = launches()
+    with pytest.raises(fms.FmsError) as e:
+        fms.reciprocal_integrate(ctx, G, w, T)
+    assert e.value.name == "NonFiniteInput" and "structure factor" in str(e.value)
+    assert launches() - before <= 2  # the packing of the batch
+    T[3, 3] = np.inf
+    with pytest.raises(fms.FmsError) as e:
+        fms.reciprocal_integrate(ctx, G, w, T)
+    assert "structure factor" in str(e.value)
+    G[29, 95, 95] = 0
+    with pytest.raises(fms.FmsError) as e:
+        fms.reciprocal_integrate(ctx, G, w, T)
+    assert "non-finite T" in str(e.value)
+    ctx.close()
