@@ -578,8 +578,12 @@ def complex_lu_solve_batched(ctx: Context, A, B, form=FORM_FP64_LU):
         B = B[None]
     batch, n, _ = A.shape
     m = B.shape[2]
+    if A.shape[2] != n or B.shape[1] != n:
+        raise ValueError(f"systems of shape {A.shape[1:]} with right-hand sides of shape {B.shape[1:]}")
+    if B.shape[0] < batch:
+        raise IndexError(f"{batch} systems with the right-hand sides of {B.shape[0]}")
     a = np.ascontiguousarray(A.transpose(0, 2, 1))  # column-major systems
-    b = np.ascontiguousarray(B.transpose(0, 2, 1))
+    b = np.ascontiguousarray(B[:batch].transpose(0, 2, 1))
     x = np.zeros((batch, m, n), np.complex128)
     st = np.zeros(batch, np.int32)
     piv = np.zeros(batch, np.int32)
