@@ -1205,7 +1205,7 @@ void lu_backward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, c
         default: rhs_upper_kernel<T, 16><<<grid, 256, 0, s>>>(lay, k, M, skip); break;
       }
     } else {
-      launch_trsm64(true, lay, batch, k, kb, n, col_end, M, LuWork(), skip, s);
+      launch_trsm64(true, lay, batch, k, kb, n, col_end, M, w ? *w : LuWork(), skip, s);
       if (w && w->tc_images && kb <= kTc64Depth && !skip) {
         tc64_update(lay, batch, 0, k, n, col_end, k, kb, M, w->tc_images, w->tc_alpha, w->tc_image_batch,
                     w->tc_wait_polls, s);

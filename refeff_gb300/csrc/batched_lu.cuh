@@ -69,6 +69,8 @@ void tc64_update(const BatchLayout& lay, int batch, int r_begin, int r_end, int 
                  double2* M, uint8_t* images, int* alpha, int image_batch, long long wait_polls, cudaStream_t s);
 
 struct LuWork {
+  // FP64 panels and block solves form their inner updates from digits on the tensor cores; false: in FP64 multiply-adds
+  bool digits = true;
   uint8_t* tc_images = nullptr;  // operand images for the tensor-core updates (FP32 or FP64); null = CUDA cores
   int tc_image_batch = 0;        // systems the FP64 update's images hold
   int* tc_alpha = nullptr;       // the updates' column scales (tc_trailing_update, tc64_update), zero between updates

@@ -439,6 +439,7 @@ struct Workspace {
   bool use_tc = false;               // FP32 trailing update on the tensor cores
   DevBuf<uint8_t> tc_images;         // operand images of the tensor-core update (and the residual's X digits)
   size_t tc_image_size = 0;
+  bool digits = true;                // FP64 panels and block solves with digits on the tensor cores
   bool use_tc64 = false;             // FP64 block updates on the tensor cores
   int tc64_batch = 0;                // systems their operand images hold
   DevBuf<int> tc_alpha;              // column scales of the tensor-core updates, zero between them
@@ -936,7 +937,7 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
   RF_CUDA(ctx, ws.status.alloc(size_t(B)));
   RF_CUDA(ctx, ws.info.alloc(size_t(B)));
   ws.use_tc = ws.fp32 && ctx->use_tensor_cores != 0;
-  ws.use_tc64 = ctx->use_tensor_cores != 0;
+  ws.digits = ws.use_tc64 = ctx->use_tensor_cores != 0;
   if (ws.use_tc) {
     ws.tc_image_size = std::max(tc_image_bytes(n, m, B), tc64_image_bytes(n, m, 1));
     RF_CUDA(ctx, ws.alloc_alpha(size_t(B) * kTcKMax));
@@ -995,6 +996,7 @@ LuWork lu_work(Workspace& ws, const PanelConfig& pc, bool polls = false) {
   w.nb = pc.nb;
   w.npanels = panel_count(ws.lay.n, pc.nb);
   w.pos_scratch = ws.pos_scratch.p;
+  w.digits = ws.digits;
   if (&pc == &ws.pc32) {
     w.perm_in = ws.perm_in.p;
     w.nperm_in = ws.nperm_in.p;

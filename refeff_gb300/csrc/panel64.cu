@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads == 256 ? 2 : 1)
             v[h][q] = r < nloc && !done[r] ? pan[size_t(c0 + 2 * t + q) * rpc_max + r] : make_double2(0.0, 0.0);
           }
         DigitTileA a;
-        const bool fits = cut_tile_a(v, a);
+        const bool fits = w.digits && cut_tile_a(v, a);
         for (int gr = 0; gr < groups; ++gr) {
           int bad = 0;
 #pragma unroll

@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(32 * kWarps) trsm64_kernel(BatchLayout lay, in
     // the other blocks' rows
     if (kUpper ? q == 0 : q + 1 >= nblk) continue;
     DigitTileA a;
-    const bool fits = cut_tile_a(x[q], a);
+    const bool fits = w.digits && cut_tile_a(x[q], a);
 #pragma unroll
     for (int p = 0; p < kMaxBlocks; ++p) {
       if (kUpper ? p >= q : p <= q || p >= nblk) continue;

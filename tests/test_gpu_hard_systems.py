@@ -128,3 +128,24 @@ def test_fp32_right_hand_sides_near_the_end_of_the_range_keep_their_bits():
     A, b = (_normal(rng, n, n) + 3 * np.sqrt(n) * np.eye(n)) / 64, _normal(rng, n, 8)
     X, Y = _fp32_solution(A, b), _fp32_solution(A, b * 2.0 ** -114) * 2.0 ** 114
     assert np.abs(X - Y).max() <= 2.0 ** -29 * np.abs(X).max()
+
+
+@pytest.mark.parametrize("n", [9, 32, 64, 170, 300])
+def test_without_tensor_cores_no_digits_are_used(n):
+    """Option 0 runs the panels, block solves and updates in FP64 multiply-adds: within the bound of the digit form's
+    solution, and rounded differently (at n = 9 and 32 there is a panel and no block update)."""
+    rng = np.random.default_rng(n)
+    A, b = _normal(rng, n, n), _normal(rng, n, 16)
+    X, X0 = _solve(A, b)[0], _solve(A, b, tensor=0)[0]
+    L, U = scipy_linalg.lu(A, permute_l=True)
+    bound = np.abs(np.linalg.inv(A)) @ (np.abs(L) @ (np.abs(U) @ np.abs(X)) + np.abs(b))
+    assert (np.abs(X - X0) <= 20 * n * EPS * bound).all()
+    assert not np.array_equal(X, X0)
+
+
+@pytest.mark.parametrize("q", [40, 100])
+@pytest.mark.parametrize("n1", [4, 16])
+def test_blocks_of_other_units_without_tensor_cores(n1, q):
+    A, b = _block_system(170, n1, q, np.random.default_rng(n1 + q), 5)
+    X, st = _solve(A, b, tensor=0)
+    assert st == 0 and _worst(A, X, b) < 10 * 170 * EPS
