@@ -61,14 +61,6 @@ struct alignas(16) RankSlot {
   unsigned long long val;
   int row;
 };
-// 1 / d for d well inside the FP64 range: an approximation r of 20 bits or more, then r (1 + e + e^2) with e = 1 - d r.
-__device__ __forceinline__ double reciprocal(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // kRpt rows per thread: kRpt * blockDim.x >= rpc_max, blockDim.x <= kMaxThreads
 template <int NB, int kMaxThreads, int kRpt>
 __global__ void __launch_bounds__(kMaxThreads, kMaxThreads == 256 ? 2 : 1)
@@ -231,7 +223,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMaxThreads == 256 ? 2 : 1)
       for (int i = 0; i < kRpt; ++i) any = any || open[i];
       if (mode && any && field > 1023 - 440 && field < 1023 + 440) {
         mode = 1;
-        const double inv = reciprocal(fma(u[0].x, u[0].x, u[0].y * u[0].y));
+        const double inv = 1.0 / fma(u[0].x, u[0].x, u[0].y * u[0].y);
         pr = make_double2(u[0].x * inv, -u[0].y * inv);
       }
 #pragma unroll
