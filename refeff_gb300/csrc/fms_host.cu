@@ -442,6 +442,7 @@ struct Workspace {
   bool digits = true;                // FP64 panels and block solves with digits on the tensor cores
   bool use_tc64 = false;             // FP64 block updates on the tensor cores
   int tc64_batch = 0;                // systems their operand images hold
+  int tc64_want = 0;                 // systems asked for when they were allocated (0: not yet for this configuration)
   DevBuf<int> tc_alpha;              // column scales of the tensor-core updates, zero between them
   DevBuf<uint8_t> tc64_images;       // their operand images; a refined workspace lends its tc_images instead
   int residual_pref = 1;             // refinement residual on the tensor cores (baked into graphs)
@@ -938,6 +939,7 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
   RF_CUDA(ctx, ws.info.alloc(size_t(B)));
   ws.use_tc = ws.fp32 && ctx->use_tensor_cores != 0;
   ws.digits = ws.use_tc64 = ctx->use_tensor_cores != 0;
+  ws.tc64_want = 0;
   if (ws.use_tc) {
     ws.tc_image_size = std::max(tc_image_bytes(n, m, B), tc64_image_bytes(n, m, 1));
     RF_CUDA(ctx, ws.alloc_alpha(size_t(B) * kTcKMax));
@@ -958,21 +960,28 @@ int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int b
                      const TunePrefs* tune = nullptr, bool lu64 = true) {
   int rc = ensure_workspace_impl(ctx, ws, n, m, batch, fp32, tune);
   if (!rc && lu64 && ws.use_tc64) {
-    // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); without room
-    // for them the updates stay on the CUDA cores
+    // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); smaller slices
+    // where there is no room for them, and without room for one system the updates stay on the CUDA cores
     const size_t room = ws.use_tc ? ws.tc_image_size : size_t(1) << 30;
-    ws.tc64_batch = 1;
-    for (int hi = ws.batch; ws.tc64_batch < hi;) {  // the most systems that fit
-      const int mid = ws.tc64_batch + (hi - ws.tc64_batch + 1) / 2;
-      if (tc64_image_bytes(n, m, mid) <= room) ws.tc64_batch = mid;
+    int want = 1;
+    for (int hi = ws.batch; want < hi;) {  // the most systems that fit
+      const int mid = want + (hi - want + 1) / 2;
+      if (tc64_image_bytes(n, m, mid) <= room) want = mid;
       else hi = mid - 1;
     }
-    const size_t bytes = ws.use_tc ? 0 : tc64_image_bytes(n, m, ws.tc64_batch), na = size_t(ws.tc64_batch) * 32;
-    if (ws.tc64_images.n < bytes || ws.tc_alpha.n < na) {
+    if (want != ws.tc64_want) {
       ws.drop_graphs();
-      if ((bytes && ws.tc64_images.alloc(bytes) != cudaSuccess) || ws.alloc_alpha(na) != cudaSuccess) {
+      ws.tc64_want = want;
+      for (ws.tc64_batch = want;; ws.tc64_batch /= 2) {
+        const size_t bytes = ws.use_tc ? 0 : tc64_image_bytes(n, m, ws.tc64_batch), na = size_t(ws.tc64_batch) * 32;
+        if ((ws.tc64_images.n >= bytes || ws.tc64_images.alloc(bytes) == cudaSuccess) &&
+            (ws.tc_alpha.n >= na || ws.alloc_alpha(na) == cudaSuccess))
+          break;
         cudaGetLastError();
-        ws.use_tc64 = false;
+        if (ws.tc64_batch == 1) {
+          ws.use_tc64 = false;
+          break;
+        }
       }
     }
   }

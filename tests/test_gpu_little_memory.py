@@ -1,0 +1,31 @@
+"""A batch of dense systems with room on the device for its matrices but not for the operand images of all of its FP64
+updates: the updates run in smaller slices of the batch and give the same bits as with room."""
+import numpy as np
+import pytest
+
+from refeff_gb300 import fms
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def test_operand_images_for_a_part_of_the_batch():
+    n, m, batch = 300, 4, 600  # matrices 0.94 GB, images 0.7 GB, staging 0.1 GB
+    rng = np.random.default_rng(2)
+    A = rng.normal(size=(batch, n, n)) + 3 * np.sqrt(n) * np.eye(n) + 0j
+    b = rng.normal(size=(batch, n, m)) + 0j
+    ctx = fms.Context(0)
+    want = fms.complex_lu_solve_batched(ctx, A, b)
+    ctx.close()
+    ctx = fms.Context(0)
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    hold = torch.empty(free - (1500 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = fms.complex_lu_solve_batched(ctx, A, b)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+        ctx.close()
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
