@@ -174,6 +174,7 @@ int fail(refeff_fms_context* ctx, int code, const std::string& msg) {
 
 int cuda_fail(refeff_fms_context* ctx, cudaError_t err, const char* where) {
   const int code = (err == cudaErrorMemoryAllocation) ? REFEFF_FMS_ERR_OUT_OF_MEMORY : REFEFF_FMS_ERR_CUDA;
+  cudaGetLastError();  // reported here: it must not come back as the next call's
   return fail(ctx, code, std::string(where) + ": " + cudaGetErrorString(err));
 }
 

@@ -29,3 +29,22 @@ def test_operand_images_for_a_part_of_the_batch():
         ctx.close()
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+def test_a_call_without_room_leaves_the_next_one_alone():
+    rng = np.random.default_rng(6)
+    A, b = rng.normal(size=(40, 300, 300)) + 60 * np.eye(300) + 0j, rng.normal(size=(40, 300, 4)) + 0j
+    ctx = fms.Context(0)
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    hold = torch.empty(free - (40 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        with pytest.raises(fms.FmsError) as e:
+            fms.complex_lu_solve_batched(ctx, A, b)
+        assert e.value.name == "OutOfMemory"
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    X, st, _ = fms.complex_lu_solve_batched(ctx, A, b)
+    ctx.close()
+    assert (st == 0).all() and np.isfinite(X).all()
