@@ -95,7 +95,8 @@ extern "C" unsigned long long refeff_fms_kernel_launches(void) { return g_launch
 // ---------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------
-struct DenseCache;  // the kept workspace of the context's dense solves (below)
+struct DenseCache;  // the kept workspace of the context's dense solves (below), at most kDenseKeep bytes
+constexpr size_t kDenseKeep = size_t(512) << 20;
 
 struct refeff_fms_context {
   refeff_fms_context();
@@ -952,6 +953,9 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
   return REFEFF_FMS_OK;
 }
 
+// Gives back the kept workspace of the context's dense solves (unless it is `ws`); true if there was one.
+bool dense_release(refeff_fms_context* ctx, const Workspace& ws);
+
 // A workspace whose (re)configuration failed part-way (an allocation) is left
 // unconfigured, so that the next call configures it again instead of running
 // on buffers sized for another shape.
@@ -960,6 +964,12 @@ int ensure_workspace_impl(refeff_fms_context* ctx, Workspace& ws, int n, int m, 
 int ensure_workspace(refeff_fms_context* ctx, Workspace& ws, int n, int m, int batch, bool fp32,
                      const TunePrefs* tune = nullptr, bool lu64 = true) {
   int rc = ensure_workspace_impl(ctx, ws, n, m, batch, fp32, tune);
+  if (rc == REFEFF_FMS_ERR_OUT_OF_MEMORY && dense_release(ctx, ws)) {
+    cudaGetLastError();
+    ws.lay.n = -1;  // configured only in part
+    ws.batch = 0;
+    rc = ensure_workspace_impl(ctx, ws, n, m, batch, fp32, tune);
+  }
   if (!rc && lu64 && ws.use_tc64) {
     // images of the whole batch, or of what 1 GiB holds (the updates then run in slices of the batch); smaller slices
     // where there is no room for them, and without room for one system the updates stay on the CUDA cores
@@ -1384,6 +1394,7 @@ int pick_batch(refeff_fms_plan& p, int E, bool fp32) {
   if (p.max_batch > 0) return std::min(E, p.max_batch);
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
+  if (free_b < kDenseKeep * 64 && dense_release(p.ctx, p.ws)) cudaMemGetInfo(&free_b, &total_b);
   const BatchLayout lay = make_layout(p.n, p.m);
   size_t per = bytes_per_system(lay, fp32);
   if (p.full) per += (size_t(lay.lda) * p.m + size_t(p.full_per)) * sizeof(double2);
@@ -2297,7 +2308,6 @@ struct DenseCache {
            ws.Xsplit.n * sizeof(float4) + ws.tc_images.n + ws.tc64_images.n;
   }
 };
-constexpr size_t kDenseKeep = size_t(512) << 20;
 refeff_fms_context::refeff_fms_context() = default;
 refeff_fms_context::~refeff_fms_context() = default;
 
@@ -2318,6 +2328,11 @@ int dense_workspace(refeff_fms_context* ctx, int n, int m, int batch, bool fp32,
     if (rc != REFEFF_FMS_ERR_OUT_OF_MEMORY || fresh) return rc;
     cudaGetLastError();  // buffers kept from other shapes may be in the way: once more from nothing
   }
+}
+bool dense_release(refeff_fms_context* ctx, const Workspace& ws) {
+  if (!ctx->dense || &ctx->dense->ws == &ws) return false;
+  ctx->dense.reset();
+  return true;
 }
 // Gives a large workspace back at the end of a call.
 struct DenseTrim {
