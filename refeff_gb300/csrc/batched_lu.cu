@@ -207,28 +207,26 @@ __global__ void __launch_bounds__(kPanelThreads) panel_kernel(BatchLayout lay, i
 
 template <typename T, int NB, bool kSolve>
 __device__ __forceinline__ void rhs_lower_column(const BatchLayout& lay, int k, int kb, cplx<T>* colp, const LuWork& w,
-                                                 int b, const cplx<T> (*L11)[NB + 1], int lane, int moves) {
+                                                 int b, const cplx<T> (*L11)[NB + 1], int lane) {
   using C = cplx<T>;
   const int panel = k / NB;
-  for (int q = 0; q < moves; ++q) {
-    const size_t pidx = size_t(b) * w.npanels + panel + q;
-    const int np = w.nperm[pidx];
-    const int2* pm = w.perm + pidx * (2 * NB);
-    constexpr int kMoves = (2 * NB + 31) / 32;
-    C v[kMoves];
-    int dst[kMoves];
+  const size_t pidx = size_t(b) * w.npanels + panel;
+  const int np = w.nperm[pidx];
+  const int2* pm = w.perm + pidx * (2 * NB);
+  constexpr int kMoves = (2 * NB + 31) / 32;
+  C v[kMoves];
+  int dst[kMoves];
 #pragma unroll
-    for (int t = 0; t < kMoves; ++t) {
-      const int i = lane + 32 * t;
-      dst[t] = -1;
-      if (i < np) { const int2 mv = pm[i]; dst[t] = mv.x; v[t] = colp[mv.y]; }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kMoves; ++t)
-      if (dst[t] >= 0) colp[dst[t]] = v[t];
-    __syncwarp();
+  for (int t = 0; t < kMoves; ++t) {
+    const int i = lane + 32 * t;
+    dst[t] = -1;
+    if (i < np) { const int2 mv = pm[i]; dst[t] = mv.x; v[t] = colp[mv.y]; }
   }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < kMoves; ++t)
+    if (dst[t] >= 0) colp[dst[t]] = v[t];
+  __syncwarp();
   if constexpr (!kSolve) return;
   constexpr int kRows = (NB + 31) / 32;
   C x[kRows];
@@ -261,13 +259,12 @@ __device__ __forceinline__ void rhs_lower_column(const BatchLayout& lay, int k, 
 
 // Columns [c_begin, c_end), kRhsColsPerWarp per warp (one after another, so
 // that each CTA reads L11 once for 8 * kRhsColsPerWarp columns): apply the
-// row moves of `moves` panels from this one on, then solve the panel rows with
-// the unit lower L11.
+// panel's row moves, then solve the panel rows with the unit lower L11.
 constexpr int kRhsColsPerWarp = 4;
 
 template <typename T, int NB, bool kSolve = true>
 __global__ void __launch_bounds__(256) rhs_lower_kernel(BatchLayout lay, int k, int c_begin, int c_end,
-                                                        cplx<T>* __restrict__ M, LuWork w, const int* skip, int moves) {
+                                                        cplx<T>* __restrict__ M, LuWork w, const int* skip) {
   using C = cplx<T>;
   const int b = blockIdx.y;
   if (skip && skip[b]) return;
@@ -287,7 +284,7 @@ __global__ void __launch_bounds__(256) rhs_lower_kernel(BatchLayout lay, int k, 
   for (int cw = 0; cw < kRhsColsPerWarp; ++cw) {
     const int col = first + cw * (blockDim.x / 32);
     if (col >= c_end) return;
-    rhs_lower_column<T, NB, kSolve>(lay, k, kb, Mb + size_t(lay.lda) * col, w, b, L11, lane, moves);
+    rhs_lower_column<T, NB, kSolve>(lay, k, kb, Mb + size_t(lay.lda) * col, w, b, L11, lane);
   }
 }
 // The outer block row of the two-level FP32 elimination as a product:
@@ -863,8 +860,11 @@ PanelConfig choose_panel(int n, int inner_pref) {
     // two-level: 64-column blocks of 16- or 32-column cluster panels.  A 32-column panel of the register kernel takes a
     // row a thread, so it serves 512 rows a CTA, and halves the launches between the panels (their row solves, moves and
     // in-block updates); 16 columns serve 1024 rows a CTA.  Measured, 16 against 32 columns: n = 688 x 60 5.83 / 5.37 ms,
-    // n = 1392 x 60 14.1 / 13.2 ms, n = 2256 x 10 18.0 / 16.7 ms, n = 2256 x 100 58.7 / 58.6 ms, n = 4112 x 24
-    // 64.6 / 62.2 ms (whole calls).  Where more than the first rows of 32 columns do not fit, 16.
+    // n = 1392 x 60 14.1 / 13.2 ms, n = 2256 x 10 18.0 / 16.7 ms, n = 2256 x 100 58.7 / 58.6 ms (whole calls).  From n =
+    // 4097 on the first panels of 32 columns have more rows than its CTAs hold and take panel_kernel; the line lies where
+    // they cost what the others save: 4 (24) systems of n = 4100 31.1 / 28.9 (76.4 / 73.2) ms, 4425 38.3 / 33.0 (90.3 /
+    // 84.5), 4625 40.7 / 35.6 (99.0 / 93.6), 4800 38.8 / 41.8 (101.8 / 104.0), 5000 43.7 / 43.2 (110.8 / 109.7), 5300 47.5
+    // / 45.2 (123.1 / 123.2).
     const bool wide = inner_pref ? inner_pref == 32 : n <= 4608;
     const int order[2] = {wide ? 32 : 16, wide ? 16 : 32};
     for (int iw : order)
@@ -921,13 +921,13 @@ static cudaError_t launch_panel(const PanelConfig& pc, const BatchLayout& lay, i
 
 template <typename T, int NB, bool kSolve = true>
 static void launch_rhs_lower(const BatchLayout& lay, int batch, int k, int c_begin, int c_end, cplx<T>* M,
-                             const LuWork& w, const int* skip, cudaStream_t s, int moves = 1) {
+                             const LuWork& w, const int* skip, cudaStream_t s) {
   const int ncols = c_end - c_begin;
   if (ncols <= 0) return;
   const int per_cta = 8 * kRhsColsPerWarp;
   dim3 grid(unsigned((ncols + per_cta - 1) / per_cta), unsigned(batch));
   count_launch();
-  rhs_lower_kernel<T, NB, kSolve><<<grid, 256, 0, s>>>(lay, k, c_begin, c_end, M, w, skip, moves);
+  rhs_lower_kernel<T, NB, kSolve><<<grid, 256, 0, s>>>(lay, k, c_begin, c_end, M, w, skip);
 }
 
 // Composes the row moves of the P inner panels of an outer block into one
@@ -1011,15 +1011,15 @@ static void gemm_any(int nb, const BatchLayout& lay, int batch, int r_begin, int
 
 template <typename T, bool kSolve = true>
 static void rhs_lower_any(int nb, const BatchLayout& lay, int batch, int k, int c_begin, int c_end, cplx<T>* M,
-                          const LuWork& w, const int* skip, cudaStream_t s, int moves = 1) {
+                          const LuWork& w, const int* skip, cudaStream_t s) {
   if constexpr (sizeof(T) == 8) {
     static_assert(kSolve, "the FP64 panels have no inner panels whose moves go to earlier columns");
     launch_trsm64(false, lay, batch, k, min(nb, lay.n - k), c_begin, c_end, M, w, skip, s);
   } else {
     switch (nb) {
-      case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
-      case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
-      default: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s, moves); break;
+      case 64: launch_rhs_lower<T, 64, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+      case 32: launch_rhs_lower<T, 32, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
+      default: launch_rhs_lower<T, 16, kSolve>(lay, batch, k, c_begin, c_end, M, w, skip, s); break;
     }
   }
 }
@@ -1181,10 +1181,7 @@ void lu_forward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cp
   const int n = lay.n, col_end = lay.n + lay.m;
   for (int k = 0; k < n; k += pc.nb) {
     const int kb = min(pc.nb, n - k);
-    // paired blocks: the second block's moves were also applied to the first one's L, so both come before the first
-    // solve (they only touch rows below the first block)
-    const int moves = !w.pair128 ? 1 : k / pc.nb % 2 ? 0 : k + pc.nb < n ? 2 : 1;
-    rhs_lower_any<T>(pc.nb, lay, batch, k, n, col_end, M, w, skip, s, moves);
+    rhs_lower_any<T>(pc.nb, lay, batch, k, n, col_end, M, w, skip, s);
     gemm_any<T>(pc.nb, lay, batch, k + kb, n, n, col_end, k, kb, M, skip, s);
   }
 }

@@ -121,7 +121,10 @@ cudaError_t lu_eliminate(const PanelConfig& pc, const BatchLayout& lay, int batc
                          cudaStream_t s);
 
 // Forward sweep (FP32) on the right-hand-side columns [n, n+m) only (new RHS):
-// Y = L^-1 P R with the stored per-panel row moves.
+// Y = L^-1 P R with the stored per-panel row moves.  Not for paired blocks,
+// whose second block's moves also went over the first one's L: they have 64
+// columns, and fused_forward_sweep takes those up to n about 45,000 (systems
+// beyond 24,800 states are refused).
 // `skip` (nullable, per matrix): matrices with skip[b] != 0 are left untouched.
 template <typename T>
 void lu_forward_rhs(const PanelConfig& pc, const BatchLayout& lay, int batch, cplx<T>* M, const LuWork& w,

@@ -1076,7 +1076,7 @@ cudaError_t refine_fp32(Workspace& ws, int batch, int iters, double tol, cudaStr
     }
   };
   const size_t nb8 = size_t(batch) * sizeof(unsigned long long);
-  // fused one-CTA-per-(matrix, column group) sweeps when the right-hand sides fit in shared memory
+  // fused sweeps, a thread-block cluster per (matrix, column group), where its CTAs' shared memory holds the right-hand sides
   auto forward = [&](const int* skip) {
     if (!fused_forward_sweep(ws.pc32.nb, lay, batch, ws.M32.p, w32, skip, s))
       lu_forward_rhs<float>(ws.pc32, lay, batch, ws.M32.p, w32, skip, s);
