@@ -18,7 +18,7 @@
 // 22 bits, some 2^-35 of the largest product of row and column in a sum of 128.
 // Where neither the sum nor C reaches 2^-11 of that product (2^28 in the scaled
 // operands) the epilogue looks the entry's largest product up and, below 2^-9 of
-// it, forms the sum again in FP32 multiply-adds (recheck_column).  Most such entries
+// it, forms the sum again in FP32 multiply-adds (recheck_columns).  Most such entries
 // are sums of large products that cancel (2% of a symmetric cluster's), and a
 // bit mask of the row's and the column's large entries tells it at once.
 // The operands are first written by tc_split_kernel into tile images that are
@@ -124,50 +124,115 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
 
 constexpr float kWeakSum = 131072.f;  // 2^(28 - 11)
 constexpr int kLost = 9, kLostRow = 4, kLostCol = kLost - kLostRow;
-// How many powers of two a scaled value lies below 2^14 (127: 127 or more, or zero).
+// How many powers of two a scaled value lies below 2^14 (63: 63 or more), kZero for a zero: a sum of two from kZero on means
+// a product that is zero.
+constexpr uint32_t kZero = 127;
 __device__ __forceinline__ uint32_t deficit(float2 v) {
   const int f = field_of(v);
-  return f == 0 ? 127u : uint32_t(min(max(140 - f, 0), 127));
+  return f == 0 ? kZero : uint32_t(min(max(140 - f, 0), 63));
 }
-// One column of a warp's 32 rows, in the lanes marked `mine`, whose sums (pr, pi) and C are small: C -= the sum where the
-// entry's largest product reaches 2^(28 - kLost) or C is not small, else C -= the sum in FP32 multiply-adds, the rows one
-// after another, 32 terms at a time (a lane a row takes 128 loads one after another, 13 us, however few lanes have one).
-// rdef, cdef: the deficits of this lane's row and of the column; a0: A's first row of the warp, bcol: B's column.
-__device__ __forceinline__ void recheck_column(bool mine, float2* c, float rs, float cf, float pr, float pi, const uint8_t* rdef,
-                                            const uint8_t* cdef, const float2* a0, const float2* bcol, int lda, int kb) {
+// Eight columns of a warp's 32 rows, a row a lane, in the columns marked in `mine` (any: in some lane of the warp), whose
+// sums are small: C -= the sum (in tensor memory at tr and ti) where the entry's largest product reaches 2^(28 - kLost),
+// all are zero or C is not small, else C -= the sum in FP32 multiply-adds: an entry at a time by the whole warp while
+// they are few (a lane alone would wait for 128 loads one after another), else the eight columns beside each other, a row
+// a lane.  c: the lane's C in the first column; cs: the columns' scales; rdef, cdef: the deficits of the lane's row and of
+// the first column; a0: A's first row of the warp; bcol: B's first column.  13 atoms with two spin channels (n = 416, up
+// to half of the entries couplings of 1e-8 and less), 116 systems: updates 4.6 ms entry by entry, 1.6 ms so (0.37 where
+// nothing is formed again).
+__device__ __forceinline__ void recheck_columns(uint32_t any, uint32_t mine, uint32_t tr, uint32_t ti, float2* c, float rs,
+                                                const float2* cs, const uint8_t* rdef, const uint8_t* cdef, const float2* a0,
+                                                const float2* bcol, int lda, int kb) {
   const int lane = threadIdx.x & 31;
-  bool again = false;
-  float2 v = make_float2(0.f, 0.f);
-  if (mine) {
-    v = *c;
-    const uint4 *ra = reinterpret_cast<const uint4*>(rdef), *cb = reinterpret_cast<const uint4*>(cdef);
-    uint32_t d = 0xfefefefeu;  // the smallest sum of two bytes (at most 254 each)
-#pragma unroll 4
-    for (int q = 0; q < (kb + 15) / 16; ++q) {
-      const uint4 x = ra[q], y = cb[q];
-      d = __vminu4(__vminu4(d, x.x + y.x), __vminu4(x.y + y.y, __vminu4(x.z + y.z, x.w + y.w)));
-    }
-    d = __vminu4(d, d >> 16);
-    again = min(d & 255u, d >> 8 & 255u) > uint32_t(kLost) && fmaxf(fabsf(v.x), fabsf(v.y)) < (kWeakSum * rs) * cf;
-  }
-  float2 p = make_float2(0.f, 0.f);
-  for (uint32_t rows = __ballot_sync(0xffffffffu, again); rows; rows &= rows - 1) {
-    const int r = __ffs(rows) - 1;
-    float2 acc = make_float2(0.f, 0.f);
+  uint32_t ur[8], ui[8], d[8];  // d: the smallest sums of two bytes (at most 254 each)
 #pragma unroll
-    for (int j = 0; j < kTcKMax / 32; ++j) {
-      const int k = 32 * j + lane;
-      if (k < kb) cfma(acc, a0[size_t(lda) * k + r], bcol[k]);
+  for (int j = 0; j < 8; ++j) {
+    ur[j] = ui[j] = 0;
+    d[j] = 0xfefefefeu;
+    if (any >> j & 1u) {
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ur[j]) : "r"(tr + uint32_t(j)));
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ui[j]) : "r"(ti + uint32_t(j)));
     }
-#pragma unroll
-    for (int w = 16; w > 0; w /= 2) {
-      acc.x += __shfl_xor_sync(0xffffffffu, acc.x, w);
-      acc.y += __shfl_xor_sync(0xffffffffu, acc.y, w);
-    }
-    if (lane == r) p = acc;
   }
-  if (mine) *c = again ? csub(v, p) : make_float2(fmaf(-(pr * rs), cf, v.x), fmaf(-(pi * rs), cf, v.y));
+  float2 v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = mine >> j & 1u ? c[size_t(lda) * j] : make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int q = 0; q < (kb + 15) / 16; ++q) {
+    const uint4 x = reinterpret_cast<const uint4*>(rdef)[q];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (any >> j & 1u) {
+        const uint4 y = reinterpret_cast<const uint4*>(cdef + j * kTcKMax)[q];
+        d[j] = __vminu4(__vminu4(d[j], x.x + y.x), __vminu4(x.y + y.y, __vminu4(x.z + y.z, x.w + y.w)));
+      }
+  }
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(ur[0]), "+r"(ur[1]), "+r"(ur[2]), "+r"(ur[3]), "+r"(ur[4]), "+r"(ur[5]), "+r"(ur[6]), "+r"(ur[7]),
+                 "+r"(ui[0]), "+r"(ui[1]), "+r"(ui[2]), "+r"(ui[3]), "+r"(ui[4]), "+r"(ui[5]), "+r"(ui[6]), "+r"(ui[7])::"memory");
+  uint32_t again = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t pair = __vminu4(d[j], d[j] >> 16), least = min(pair & 255u, pair >> 8 & 255u);
+    if (!(mine >> j & 1u)) continue;
+    const float cf = cs[j].x;
+    if (least > uint32_t(kLost) && least < kZero && fmaxf(fabsf(v[j].x), fabsf(v[j].y)) < (kWeakSum * rs) * cf)
+      again |= 1u << j;
+    else
+      c[size_t(lda) * j] = make_float2(fmaf(-(__uint_as_float(ur[j]) * rs), cf, v[j].x),
+                                       fmaf(-(__uint_as_float(ui[j]) * rs), cf, v[j].y));
+  }
+  const uint32_t lanes = __ballot_sync(0xffffffffu, again != 0);
+  if (lanes == 0) return;
+  if (__popc(lanes) * 64 <= kb) {
+    for (uint32_t rows = lanes; rows; rows &= rows - 1) {
+      const int r = __ffs(rows) - 1;
+      for (uint32_t cols = __shfl_sync(0xffffffffu, again, r); cols; cols &= cols - 1) {
+        const int j = __ffs(cols) - 1;
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < kTcKMax / 32; ++i) {
+          const int k = 32 * i + lane;
+          if (k < kb) cfma(acc, a0[size_t(lda) * k + r], bcol[size_t(lda) * j + k]);
+        }
+#pragma unroll
+        for (int w = 16; w > 0; w /= 2) {
+          acc.x += __shfl_xor_sync(0xffffffffu, acc.x, w);
+          acc.y += __shfl_xor_sync(0xffffffffu, acc.y, w);
+        }
+        if (lane == r) c[size_t(lda) * j] = csub(c[size_t(lda) * j], acc);
+      }
+    }
+    return;
+  }
+  const uint32_t cols = __reduce_or_sync(0xffffffffu, again);
+  float2 acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int k0 = 0; k0 < kb; k0 += 32) {
+    // 32 terms of the columns, one a lane, handed round by shuffles: the loads of all are in flight at once
+    float2 bl[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      bl[j] = (cols >> j & 1u) && k0 + lane < kb ? bcol[size_t(lda) * j + k0 + lane] : make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int h = 0; h < 32 && k0 + h < kb; h += 8) {
+      float2 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = again && k0 + h + i < kb ? a0[size_t(lda) * (k0 + h + i) + lane] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (cols >> j & 1u)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            cfma(acc[j], a[i], make_float2(__shfl_sync(0xffffffffu, bl[j].x, h + i), __shfl_sync(0xffffffffu, bl[j].y, h + i)));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (again >> j & 1u) c[size_t(lda) * j] = csub(c[size_t(lda) * j], acc[j]);
 }
+
 // Bit j of a row's or column's mask stands for g consecutive k from g j on, g = 1, 2 or 4 for kb <= 32, 64 or 128: all of
 // the row's entries lie within 2^kLostRow of its largest, one of the column's within 2^kLostCol; a common bit means a
 // product above 2^(28 - kLost).
@@ -673,19 +738,20 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_update_persistent_kernel(
         weak_cols |= static_cast<unsigned long long>(lost) << (16 * part);
       }
       // the columns in which a row of this warp has one (the accumulators are still there; C's registers are free)
-      unsigned long long any = (static_cast<unsigned long long>(__reduce_or_sync(0xffffffffu, uint32_t(weak_cols >> 32))) << 32) |
-                               __reduce_or_sync(0xffffffffu, uint32_t(weak_cols));
-      for (; any; any &= any - 1) {
-        const int off = __ffsll(static_cast<long long>(any)) - 1;
-        uint32_t ur, ui;
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ur) : "r"(tmem_r + uint32_t(off)));
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(ui) : "r"(tmem_i + uint32_t(off)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(ur), "+r"(ui)::"memory");
-        const float2* Mb = M + size_t(b) * lay.stride + size_t(k);
-        recheck_column(weak_cols >> off & 1u, crow + off * ld, rs, cs[off].x, __uint_as_float(ur), __uint_as_float(ui),
-                       rdef + ((size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane) * kTcKMax,
-                       cdef + ((size_t(b) * nbn_all + bn) * BN + off) * kTcKMax,
-                       Mb + size_t(ld) * k + size_t(r0 - k + quarter * 32), Mb + size_t(ld) * (c0 + off), ld, kb);
+      const uint32_t weak_lo = uint32_t(weak_cols), weak_hi = uint32_t(weak_cols >> 32);
+      const unsigned long long any = (static_cast<unsigned long long>(__reduce_or_sync(0xffffffffu, weak_hi)) << 32) |
+                                     __reduce_or_sync(0xffffffffu, weak_lo);
+      if (any) {
+#pragma unroll 1
+        for (int off = 0; off < BN; off += 8) {
+          const uint32_t any8 = uint32_t(any >> off) & 255u;
+          if (any8 == 0) continue;
+          const float2* Mb = M + size_t(b) * lay.stride + size_t(k);
+          recheck_columns(any8, uint32_t(weak_cols >> off) & 255u, tmem_r + uint32_t(off), tmem_i + uint32_t(off), crow + off * ld, rs,
+                          cs + off, rdef + ((size_t(b) * nbm_all + bm) * BM + quarter * 32 + lane) * kTcKMax,
+                          cdef + ((size_t(b) * nbn_all + bn) * BN + off) * kTcKMax,
+                          Mb + size_t(ld) * k + size_t(r0 - k + quarter * 32), Mb + size_t(ld) * (c0 + off), ld, kb);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       mbar_arrive(bar(kBarAccEmpty + g));  // the accumulator may be overwritten

@@ -173,6 +173,7 @@ __device__ __forceinline__ double2 direct_sum(const double2* arow, const double2
 // Most small sums are of large products that cancel: masks of the k at which a row's entries reach 2^-kLostPart of its
 // largest, and a column's of its, tell it by a common bit.
 constexpr int kLostPart = kLost / 2;
+constexpr int kZero = 127;  // a sum of two deficits from here on: a product that is zero
 // An entry whose sum the grid may have lost: C at (row, col) of matrix b is untouched yet; p the digit sum, of grid 2^e.
 struct alignas(16) Tc64Entry {
   double2 p;
@@ -216,8 +217,8 @@ __global__ void __launch_bounds__(kRows) tc64_scale_kernel(BatchLayout lay, int 
 // and the row exponents, two threads per row, 16 columns each.  The others: a column tile of B,
 // image[b][bn][K step][P, Q][digit 1..8][32 rows of 16 bf16] with P = [Br | Bi], Q = [-Bi | Br] (16 columns each) and the
 // column exponents, one warp per column, one lane per row, each exponent with its mask of large entries.  rdef and cdef:
-// 32 bytes a row of A and a column of B, how many powers of two each (balanced) entry lies below the grid (127: 127 or more,
-// or zero).
+// 32 bytes a row of A and a column of B, how many powers of two each (balanced) entry lies below the grid (63: 63 or more;
+// kZero: zero, or meeting only zeros).
 __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_begin, int r_end, int c_begin, int c_end,
                                                          int ka, int kb, const double2* __restrict__ M,
                                                          const int* __restrict__ alpha, uint8_t* __restrict__ aimg,
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
     uint32_t below_grid[4] = {}, large = 0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const int f = field_of(v[i]), d = f < 0 ? 127 : min(max(e - (max(f, 1) - 1022 + gk[16 * h + i]), 0), 127);
+      const int f = field_of(v[i]), d = f < 0 ? kZero : min(max(e - (max(f, 1) - 1022 + gk[16 * h + i]), 0), 63);
       below_grid[i / 4] |= uint32_t(d) << (8 * (i % 4));
       large |= d <= kLostPart ? 1u << i : 0u;
     }
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(256) tc64_split_kernel(BatchLayout lay, int r_
     const int f = field_of(v), g = gk[k];
     const int e = __reduce_max_sync(0xffffffffu, f == 0x7ff ? kNonfinite : f < 0 || g == kNoEntry ? kNoEntry : max(f, 1) - 1022 - g);
     const bool none = e == kNonfinite || e == kNoEntry || g == kNoEntry;
-    const int d = none || f < 0 ? 127 : min(e - (max(f, 1) - 1022 - g), 127);
+    const int d = none || f < 0 ? kZero : min(e - (max(f, 1) - 1022 - g), 63);
     const size_t at = (size_t(b) * nbn_all + bn) * kCols + c;
     cdef[at * 32 + k] = uint8_t(d);
     const uint32_t large = __ballot_sync(0xffffffffu, d <= kLostPart);
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// The listed entries: C -= p where a product reaches 2^(e - kLost), else C -= the sum in FP64 multiply-adds.  Four lanes
+// The listed entries: C -= p where a product reaches 2^(e - kLost) or all are zero, else C -= the sum in FP64 multiply-adds.  Four lanes
 // an entry, eight terms each.  A kernel of its own: these entries gather in few rows of few tiles (0.3 .. 0.6% of all on
 // symmetric clusters, whose structural zeros are rounding noise in C), where warps that summed their own ones would hold
 // their tiles up.  Most are sound, and the bytes of rdef and cdef tell it without A and B.
@@ -617,7 +618,8 @@ __global__ void __launch_bounds__(4 * kChunk, 2) tc64_recheck_kernel(BatchLayout
     d = __vminu4(d, __shfl_xor_sync(0xffffffffu, d, 1));
     d = __vminu4(d, __shfl_xor_sync(0xffffffffu, d, 2));
     d = __vminu4(d, d >> 16);
-    const bool again = min(d & 255u, (d >> 8) & 255u) > uint32_t(kLost);
+    const uint32_t least = min(d & 255u, (d >> 8) & 255u);
+    const bool again = least > uint32_t(kLost) && least < uint32_t(kZero);
     if (__any_sync(0xffffffffu, again)) {
       const double2* const a = Mb + size_t(q.row) + lda * size_t(ka);
       const double2* const b = Mb + size_t(ka) + lda * size_t(q.col);
