@@ -109,7 +109,9 @@ unsigned long long refeff_fms_kernel_launches(void);
  *   REFEFF_FMS_OPT_TENSOR_CORES: 1 (default) runs the block updates of the LU
  *     on the tcgen05 tensor cores: FP32 values as two FP16 terms with FP32
  *     accumulation, FP64 values as eight 8-bit digits whose products are summed
- *     exactly; 0 runs them on the CUDA cores.
+ *     exactly, and sums that those may have lost (entries far below their row's
+ *     and column's largest) as FP32 or FP64 multiply-adds; 0 runs them, and the
+ *     inner updates of the FP64 panels and block solves, on the CUDA cores.
  *   REFEFF_FMS_OPT_DENSE_REFINEMENT: corrections allowed in
  *     refeff_complex_lu_solve_batched with REFEFF_FMS_FORM_FP32_REFINED
  *     (default 10; 0 returns the plain FP32 LU solution, flagged NOT_CONVERGED).

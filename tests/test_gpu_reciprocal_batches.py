@@ -14,15 +14,26 @@ def _inputs(order, k_points, seed=1):
 
 
 def test_a_wait_that_runs_out_in_the_first_batch_is_reported():
-    """1025 k-points at a poll budget that 1024 systems at a time exceed and one alone does not (16 .. 24 and 64 .. 96
-    polls): the second batch's clean run must not hide the first one's."""
+    """1025 k-points at a poll budget that 1024 systems at a time exceed and one alone does not (between 24 and 64 polls
+    where this was written): the second batch's clean run must not hide the first one's."""
     ctx = fms.Context(0)
-    ctx.set_option(ctx.OPT_TC_WAIT_POLLS, 40)
-    _, st = fms.reciprocal_integrate(ctx, *_inputs(64, 1), fms.FORM_FP32_REFINED)
-    assert (st == 0).all()
-    with pytest.raises(fms.FmsError) as e:
-        fms.reciprocal_integrate(ctx, *_inputs(64, 1025), fms.FORM_FP32_REFINED)
-    assert "timed out" in str(e.value)
+    one, many, both = (_inputs(64, k) for k in (1, 1024, 1025))
+
+    def times_out(inputs):
+        try:
+            fms.reciprocal_integrate(ctx, *inputs, fms.FORM_FP32_REFINED)
+        except fms.FmsError as e:
+            assert "timed out" in str(e)
+            return True
+        return False
+
+    for polls in (40, 32, 48, 28, 56, 64, 80):
+        ctx.set_option(ctx.OPT_TC_WAIT_POLLS, polls)
+        if not any(times_out(one) for _ in range(4)) and all(times_out(many) for _ in range(4)):
+            assert times_out(both)
+            break
+    else:
+        pytest.skip("no poll budget tells the batches apart on this device")
     ctx.close()
 
 
