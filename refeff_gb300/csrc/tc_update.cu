@@ -16,11 +16,12 @@
 // entry in [2^13, 2^14), and the epilogue takes the scales out again.  Entries
 // more than 2^16 below their row's largest keep 2^-39 of that instead of their
 // 22 bits, some 2^-35 of the largest product of row and column in a sum of 128.
-// Where neither the sum nor C reaches 2^-11 of that product (2^28 in the scaled
-// operands) the epilogue looks the entry's largest product up and, below 2^-9 of
-// it, forms the sum again in FP32 multiply-adds (recheck_columns).  Most such entries
-// are sums of large products that cancel (2% of a symmetric cluster's), and a
-// bit mask of the row's and the column's large entries tells it at once.
+// Where neither the sum nor C reaches 2^-13 of that product (2^28 in the scaled
+// operands: the error stays below 2^-22 of the sum or C, what two terms keep of a
+// value) the epilogue looks the entry's largest product up and, below 2^-11 of it,
+// forms the sum again in FP32 multiply-adds (recheck_columns).  Most such entries
+// are sums of large products that cancel (2% of a symmetric cluster's), and a bit
+// mask of the row's and the column's large entries tells it at once.
 // The operands are first written by tc_split_kernel into tile images that are
 // already in the UMMA shared-memory layout (K-major, 64-byte rows, 64-byte
 // swizzle), so the update kernel moves them with plain cp.async.bulk copies
@@ -122,8 +123,8 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-constexpr float kWeakSum = 131072.f;  // 2^(28 - 11)
-constexpr int kLost = 9, kLostRow = 4, kLostCol = kLost - kLostRow;
+constexpr float kWeakSum = 32768.f;  // 2^(28 - 13)
+constexpr int kLost = 11, kLostRow = 5, kLostCol = kLost - kLostRow;
 // How many powers of two a scaled value lies below 2^14 (63: 63 or more), kZero for a zero: a sum of two from kZero on means
 // a product that is zero.
 constexpr uint32_t kZero = 127;
@@ -183,7 +184,7 @@ __device__ __forceinline__ void recheck_columns(uint32_t any, uint32_t mine, uin
   }
   const uint32_t lanes = __ballot_sync(0xffffffffu, again != 0);
   if (lanes == 0) return;
-  if (__popc(lanes) * 64 <= kb) {
+  if (__reduce_add_sync(0xffffffffu, __popc(again)) * 12 <= kb) {
     for (uint32_t rows = lanes; rows; rows &= rows - 1) {
       const int r = __ffs(rows) - 1;
       for (uint32_t cols = __shfl_sync(0xffffffffu, again, r); cols; cols &= cols - 1) {
