@@ -236,7 +236,7 @@ __device__ __forceinline__ void recheck_columns(uint32_t any, uint32_t mine, uin
 
 // Bit j of a row's or column's mask stands for g consecutive k from g j on, g = 1, 2 or 4 for kb <= 32, 64 or 128: all of
 // the row's entries lie within 2^kLostRow of its largest, one of the column's within 2^kLostCol; a common bit means a
-// product above 2^(28 - kLost).
+// product above 2^(28 - kLost).  (A row or column of zeros has every bit: its sums are exact.)
 __device__ __forceinline__ uint32_t large_mask(const uint8_t* def, int kb, bool row) {
   const uint32_t limit = 0x01010101u * uint32_t(row ? kLostRow : kLostCol);
   const uint32_t* d = reinterpret_cast<const uint32_t*>(def);
@@ -378,7 +378,7 @@ __device__ __forceinline__ void split_a_tile(const BatchLayout& lay, int k, int 
   }
   if (threadIdx.x < BM) {
     const size_t at = (size_t(b) * nbm + bm) * BM + threadIdx.x;
-    rscale[at].y = __uint_as_float(large_mask(rdef + at * kTcKMax, kb, true));
+    rscale[at].y = __uint_as_float(rscale[at].x == 0.f ? ~0u : large_mask(rdef + at * kTcKMax, kb, true));
   }
 }
 
@@ -442,7 +442,7 @@ __device__ __forceinline__ void split_b_tile(const BatchLayout& lay, int bn, int
   __syncthreads();
   if (threadIdx.x < BN) {
     const size_t at = (size_t(b) * nbn + bn) * BN + threadIdx.x;
-    cscale[at].y = __uint_as_float(large_mask(cdef + at * kTcKMax, kb, false));
+    cscale[at].y = __uint_as_float(cscale[at].x == 0.f ? ~0u : large_mask(cdef + at * kTcKMax, kb, false));
   }
 }
 
