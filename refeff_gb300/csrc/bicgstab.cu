@@ -366,11 +366,13 @@ __global__ void __launch_bounds__(kMvThreads) bicg_matvec_kernel(View w, const f
 // and the CTA drains its copies and MMAs and frees its tensor memory before it
 // returns.
 // Bound by HBM (A is read once).  The form at n = 4112, 12 matrices, 16 columns
-// (576 products and the vector kernels): 73.4 ms; with A in bulk copies of 1 KB,
-// one a column of a slab, 81.5, bound by their issue (1.65 GB in 346 us under a
-// profiler; another ring stage, twice the row warps or 1024-column slices
-// changed nothing); FP16 terms with loads in registers and 256-column slices
-// 92.8; split by the row's thread into two TF32 terms, 12 MMAs a slab, 101.9.
+// (576 products and the vector kernels), on one set of inputs: 73.4 ms; with A
+// in bulk copies of 1 KB, one a column of a slab, 81.5, bound by their issue
+// (1.65 GB in 346 us under a profiler; another ring stage, twice the row warps
+// or 1024-column slices changed nothing); FP16 terms with loads in registers
+// and 256-column slices 92.8; split by the row's thread into two TF32 terms, 12
+// MMAs a slab, 101.9.  Other inputs take other numbers of iterations (164 and
+// 117.6 ms in another run); the quotient to the last form stays 1.38 to 1.40.
 constexpr int kTcRows = 128, kTcK = 16, kTcThreads = 192, kTcStages = 2, kTcSub = 256;
 constexpr long long kTcBicgPolls = 1LL << 26;  // poll budget of each wait (about 1 s is the other bound)
 constexpr int kTcAPlane = kTcRows * 32;             // 4 KB: 128 rows of 16 FP16 values
